@@ -167,6 +167,26 @@ inline cudaError_t launch_kernel(dlb_ctx *ctx, void (*kernel)(P...), dim3 grid, 
   cfg.numAttrs = ctx->use_pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+// The same with the blocks of `cluster` consecutive x forming a cluster.
+template <class... P, class... A>
+inline cudaError_t launch_kernel_cluster(dlb_ctx *ctx, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                                         unsigned cluster, A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ctx->use_pdl ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 #define DLB_LAUNCH_KERNEL(ctx, kernel, grid, block, smem, ...) \
   dlb::launch_kernel((ctx), (kernel), dim3(grid), dim3(block), (size_t)(smem), __VA_ARGS__)
 #endif
@@ -242,6 +262,11 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float 
                 long long ldc, int M, int N, int K, const GemmEpilogue &ep);
 dlb_status gemm_simt(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C,
                      long long ldc, int M, int N, int K, const GemmEpilogue &ep);
+// Tensor-core product from the fp32 tensors (gemm_direct.cu).
+dlb_status gemm_direct(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C, long long ldc, int M, int N,
+                       int K, const GemmEpilogue &ep);
+bool gemm_direct_supported(const GemmOperand &A, const GemmOperand &B);
+double gemm_direct_us(const dlb_ctx *ctx, int M, int N, int K);  // about how long it takes
 // Returns DLB_ERR_UNSUPPORTED (without touching C) when the shape or alignment
 // is outside what the TMA descriptors can express.
 dlb_status gemm_tcgen05(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C,

@@ -108,8 +108,28 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
   }
   // The tensor-core tile is 128 x 256; below that the CUDA-core kernel is
   // used, as it is for layouts TMA cannot address.
-  const bool big = (long long)M * N >= 128 * 64 && K >= 32;
+  const bool big = ((long long)M * N >= 128 * 64 && K >= 32) || ctx->gemm_kind == DLB_GEMM_F16X3;
   if (!(ctx->use_tensor_core && ctx->tensor_core_ok && big)) return gemm_simt(ctx, A, B, C, ldc, M, N, K, ep);
+
+  // The fp16 form either reads operands split beforehand (plane_product) or splits
+  // them in the product (gemm_direct).  Planes that the caller keeps are used
+  // wherever TMA can address them and the output fills a 256 x 256 tile.  Below
+  // that, and for every other pitch and width, the direct kernel runs.  Where
+  // planes would have to be made for this call the shorter of the two wins: the
+  // direct kernel takes about 8 us and 2.6 us per round of 64-deep chunks (one
+  // 128 x 128 tile per SM), the product on fresh planes about 55 us (absolute
+  // maxima, split and check of two operands; 45 us when one is transposed) and
+  // 450 TFLOP/s (1024^3: 30 us against 67, 2048^3: 188 against 95).
+  const bool direct_form = ctx->gemm_kind == DLB_GEMM_F16X3 && !ep.fused && gemm_direct_supported(A, B);
+  const double direct_us = direct_form ? gemm_direct_us(ctx, M, N, K) : 1e30;
+  const double planes_us = 2.0 * M * N * K / 4.5e8;
+  auto direct = [&]() -> dlb_status {
+    ProfileSpan span;
+    DLB_TRY(span.begin(ctx, 0, 2.0 * M * N * K));
+    DLB_TRY(gemm_direct(ctx, A_in, B_in, C, ldc, M, N, K, ep));
+    return span.end();
+  };
+  const bool plane_size = (long long)M * N >= 256 * 256 && K >= 32;
 
   // A weight-gradient product (both operands mn-contiguous) whose A TMA cannot
   // tile as it lies (output rows not a multiple of 64, e.g. 1000 classes), or
@@ -123,8 +143,8 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
   // each output row multiplied by its line's 1 / scale.  Nothing of A is left
   // for the range guard to flag.
   if (ctx->gemm_kind == DLB_GEMM_F16X3 && A.stride_mn == 1 && A.stride_k != 1 && B.stride_mn == 1 &&
-      B.stride_k != 1 && gemm_pair_enabled() && (long long)M * N >= 256 * 256 && !ep.fused &&
-      (A.rescale_lines || !gemm_f16_supported(A, B, C, ldc, M, N, K))) {
+      B.stride_k != 1 && gemm_pair_enabled() && plane_size && !ep.fused &&
+      (A.rescale_lines || !gemm_f16_supported(A, B, C, ldc, M, N, K)) && direct_us > planes_us + 45.0) {
     GemmOperand a = A, b = B;
     const bool have_b = b.h_hi || planes_lookup(ctx, b.lo, &b);
     const long long kp = (long long)align_up((size_t)K, 8);
@@ -150,6 +170,13 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
         B = b;
       }
     }
+  }
+
+  if (direct_form && A.h_hi == nullptr) {  // (A.h_hi: planes just made for this product)
+    if (!plane_size || !gemm_f16_supported(A, B, C, ldc, M, N, K) || A.rescale_lines) return direct();
+    GemmOperand a = A, b = B;
+    const bool have = planes_lookup(ctx, a.lo, &a) && planes_lookup(ctx, b.lo, &b);
+    if (!have && direct_us <= planes_us + 55.0) return direct();
   }
 
   if (ctx->gemm_kind == DLB_GEMM_F16X3 && gemm_f16_supported(A, B, C, ldc, M, N, K)) {

@@ -38,21 +38,33 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// The same, suspended by the hardware for up to 20 us: a polling warp otherwise
+// spends issue slots that the working warps of its scheduler need (half of all
+// instructions of gemm_direct_kernel were polls).
+__device__ __forceinline__ bool mbar_try_wait_suspended(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(20000u)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait.  Returns false if the budget ran out or another role aborted.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag,
                                           int *status) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
-  uint32_t spins = 0;
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((++spins & 255u) == 0) {
-      if (*abort_flag) return false;
-      if (clock64() - t0 > WAIT_BUDGET_CLOCKS) {
-        *abort_flag = 1;
-        atomicExch(status, DLB_ERR_TIMEOUT);
-        return false;
-      }
+    if (mbar_try_wait_suspended(bar, parity)) return true;
+    if (*abort_flag) return false;
+    if (clock64() - t0 > WAIT_BUDGET_CLOCKS) {
+      *abort_flag = 1;
+      atomicExch(status, DLB_ERR_TIMEOUT);
+      return false;
     }
   }
 }
