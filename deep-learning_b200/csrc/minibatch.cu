@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_copy.cuh"
 #include "model.cuh"
 
 using namespace dlb;
@@ -44,14 +45,16 @@ size_t rows_of(const dlb_minibatch *mb, size_t k) { return k + 1 != mb->n_batch 
 // Rows of batch k into staging slot `slot`, by the host threads the model keeps.
 void gather(dlb_minibatch *mb, size_t k, int slot) {
   const size_t first = k * mb->per_batch, rows = rows_of(mb, k);
+  const size_t bytes = rows * (mb->width_x + mb->width_y) * sizeof(float);
+  const bool streaming = bytes >= STREAM_COPY_BYTES;
   auto part = [&](size_t a, size_t b) {
     for (size_t r = a; r < b; ++r) {
       const size_t src = mb->order[first + r];
-      memcpy(mb->host_x[slot] + r * mb->width_x, mb->Xm[src], mb->width_x * sizeof(float));
-      memcpy(mb->host_y[slot] + r * mb->width_y, mb->Ym[src], mb->width_y * sizeof(float));
+      staging_copy(mb->host_x[slot] + r * mb->width_x, mb->Xm[src], mb->width_x * sizeof(float), streaming);
+      staging_copy(mb->host_y[slot] + r * mb->width_y, mb->Ym[src], mb->width_y * sizeof(float), false);
     }
+    staging_fence(streaming);
   };
-  const size_t bytes = rows * (mb->width_x + mb->width_y) * sizeof(float);
   if (bytes < (1u << 20)) {
     part(0, rows);
     return;
@@ -172,23 +175,36 @@ dlb_status dlb_minibatch_train(dlb_minibatch *mb, double *loss) {
   m->training_accuracy = true;  // train_mp adds up the accuracy of every batch beside its loss
   double sum = 0.0, sum_accuracy = 0.0;
   dlb_status st = DLB_OK;
+  // Step k is enqueued first; while the device works on it the host reads the loss
+  // of step k - 1, gathers batch k + 1 and starts its copy.  (The reference reads
+  // each loss before the next step; the sums are the same.)
+  int pending = -1;  // slot of the loss that has not been read yet
+  auto collect = [&]() -> dlb_status {
+    if (pending < 0) return DLB_OK;
+    double batch_loss = 0.0;
+    const dlb_status r = staged_step_loss(m, pending, &batch_loss);
+    pending = -1;
+    sum += batch_loss;
+    sum_accuracy += m->step_accuracy;
+    return r;
+  };
   gather(mb, 0, 0);
   st = dlb_model_stage_batch(m, rows_of(mb, 0), mb->host_x[0], mb->host_y[0]);
   for (size_t k = 0; k < mb->n_batch && st == DLB_OK; ++k) {
-    if (k + 1 < mb->n_batch) {
-      // The step that read staging slot (k + 1) % 2 last was step k - 1, whose
-      // loss the host has waited for.
-      const int slot = (int)((k + 1) & 1);
-      gather(mb, k + 1, slot);
-      st = dlb_model_stage_batch(m, rows_of(mb, k + 1), mb->host_x[slot], mb->host_y[slot]);
-      if (st != DLB_OK) break;
-    }
     if (world > 1) st = dlb_model_set_global_batch(m, rows_of(mb, k) * world);
-    double batch_loss = 0.0;
-    if (st == DLB_OK) st = dlb_model_train_step_staged(m, &batch_loss);
-    sum += batch_loss;
-    sum_accuracy += m->step_accuracy;
+    int slot = -1;
+    if (st == DLB_OK) st = staged_step_enqueue(m, true, &slot);
+    if (st == DLB_OK) st = collect();
+    if (st != DLB_OK) break;
+    pending = slot;
+    if (k + 1 < mb->n_batch) {
+      // Step k - 1, whose loss has arrived, was the last to read this staging slot.
+      const int at = (int)((k + 1) & 1);
+      gather(mb, k + 1, at);
+      st = dlb_model_stage_batch(m, rows_of(mb, k + 1), mb->host_x[at], mb->host_y[at]);
+    }
   }
+  if (st == DLB_OK) st = collect();
   m->training_size = saved_training;
   m->global_rows = saved_global;
   m->training_accuracy = saved_accuracy;

@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_copy.cuh"
 #include "model.cuh"
 
 using namespace dlb;
@@ -1072,7 +1073,8 @@ dlb_status stage_rows(dlb_model *m, int which, float **stage, size_t *stage_elem
       const size_t r0 = piece * piece_rows, r1 = std::min(rows, r0 + piece_rows);
       const size_t per = (r1 - r0 + split - 1) / split;
       const size_t a = std::min(r1, r0 + share * per), b = std::min(r1, a + per);
-      for (size_t r = a; r < b; ++r) memcpy(staging + r * width, row_ptrs[r], width * sizeof(float));
+      for (size_t r = a; r < b; ++r) staging_copy(staging + r * width, row_ptrs[r], width * sizeof(float), true);
+      staging_fence(true);
       if (left[piece].fetch_sub(1) == 1) {
         if (cudaSetDevice(device) != cudaSuccess ||
             cudaMemcpyAsync(dev + r0 * width, staging + r0 * width, (r1 - r0) * width * sizeof(float),
@@ -1111,7 +1113,9 @@ dlb_status stage_block(dlb_model *m, float **stage, size_t *stage_elems, size_t 
     *stage_elems = elems;
   }
   DLB_CUDA(cudaStreamSynchronize(m->ctx->stream));
-  memcpy(*stage, host, elems * sizeof(float));
+  const bool streaming = elems * sizeof(float) >= STREAM_COPY_BYTES;
+  staging_copy(*stage, host, elems * sizeof(float), streaming);
+  staging_fence(streaming);
   return dlb_memcpy_h2d(m->ctx, dev, *stage, elems * sizeof(float));
 }
 
@@ -2715,27 +2719,12 @@ dlb_status dlb_model_stage_batch(dlb_model *m, size_t rows, const float *X_host,
 
 dlb_status dlb_model_train_step_staged(dlb_model *m, double *loss) {
   DLB_REQUIRE(m, "train_step_staged");
-  DLB_REQUIRE(m->ahead_head > m->ahead_tail, "train_step_staged: no batch has been staged");
-  dlb_model::Ahead &a = m->ahead[m->ahead_tail % 2];
-  ++m->ahead_tail;
-  const size_t rows = a.rows;
-  DLB_CUDA(cudaStreamWaitEvent(m->ctx->stream, a.ready, 0));
-  DLB_TRY(dlb_model_reset_loss(m));
-  DLB_TRY(dlb_model_forward_pass_device(m, rows, a.x));
-  DLB_TRY(dlb_model_compute_error_device(m, rows, a.y));
-  DLB_CUDA(cudaEventRecord(a.consumed, m->ctx->stream));
-  a.in_use = true;
-  DLB_TRY(backward_update_merge(m, rows));
-  // The loss starts its way to the host and the update is enqueued before the
-  // host waits for anything.  With a loss lag of one step the wait is for the
-  // loss of the step before, which has long arrived: the host then never waits
-  // for the step it has just enqueued and runs one step ahead of the device.
-  const int slot = (int)(m->loss_steps++ & 1);
-  if (loss) DLB_TRY(loss_capture(m, slot));
-  const size_t g = m->global_rows ? m->global_rows : rows;
-  DLB_TRY(dlb_model_update_weights(m, g, m->training_size ? m->training_size : g));
-  if (loss) DLB_TRY(loss_collect(m, m->loss_lag ? slot ^ 1 : slot, loss));
-  return DLB_OK;
+  // With a loss lag of one step the wait is for the loss of the step before,
+  // which has long arrived: the host then never waits for the step it has just
+  // enqueued and runs one step ahead of the device.
+  int slot = 0;
+  DLB_TRY(staged_step_enqueue(m, loss != nullptr, &slot));
+  return loss ? staged_step_loss(m, m->loss_lag ? slot ^ 1 : slot, loss) : DLB_OK;
 }
 
 dlb_status dlb_model_set_training_accuracy(dlb_model *m, int on) {
@@ -2776,3 +2765,24 @@ dlb_status dlb_model_get_layer_errors(dlb_model *m, size_t layer, size_t rows, i
 }
 
 }  // extern "C"
+
+// The step on the oldest staged batch, its loss on the way to the host (slot) and
+// the update enqueued behind it; nothing is waited for.
+dlb_status dlb::staged_step_enqueue(dlb_model *m, bool want_loss, int *slot) {
+  DLB_REQUIRE(m->ahead_head > m->ahead_tail, "train_step_staged: no batch has been staged");
+  dlb_model::Ahead &a = m->ahead[m->ahead_tail % 2];
+  ++m->ahead_tail;
+  const size_t rows = a.rows;
+  DLB_CUDA(cudaStreamWaitEvent(m->ctx->stream, a.ready, 0));
+  DLB_TRY(dlb_model_reset_loss(m));
+  DLB_TRY(dlb_model_forward_pass_device(m, rows, a.x));
+  DLB_TRY(dlb_model_compute_error_device(m, rows, a.y));
+  DLB_CUDA(cudaEventRecord(a.consumed, m->ctx->stream));
+  a.in_use = true;
+  DLB_TRY(backward_update_merge(m, rows));
+  *slot = (int)(m->loss_steps++ & 1);
+  if (want_loss) DLB_TRY(loss_capture(m, *slot));
+  const size_t g = m->global_rows ? m->global_rows : rows;
+  return dlb_model_update_weights(m, g, m->training_size ? m->training_size : g);
+}
+dlb_status dlb::staged_step_loss(dlb_model *m, int slot, double *loss) { return loss_collect(m, slot, loss); }

@@ -197,3 +197,10 @@ struct dlb_model {
   bool update_prepared = false;
   dlb_optimizer_scalars update_k = {};
 };
+
+namespace dlb {
+// The two halves of dlb_model_train_step_staged, for loops that have host work to
+// do while the device works on the step.  At most two slots are open at a time.
+dlb_status staged_step_enqueue(dlb_model *m, bool want_loss, int *slot);
+dlb_status staged_step_loss(dlb_model *m, int slot, double *loss);
+}  // namespace dlb

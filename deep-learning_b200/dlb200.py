@@ -567,11 +567,13 @@ class Model:
 
     @staticmethod
     def _row_pointers(a):
+        """(array, address of its row pointers); the array of pointers lives as long
+        as the returned address object."""
         a = np.ascontiguousarray(a, dtype=np.float32)
-        base = a.ctypes.data
-        stride = a.strides[0]
-        rows = (C.c_void_p * a.shape[0])(*[base + i * stride for i in range(a.shape[0])])
-        return a, rows
+        rows = np.arange(a.shape[0], dtype=np.uintp)
+        rows *= np.uintp(a.strides[0])
+        rows += np.uintp(a.ctypes.data)
+        return a, rows.ctypes.data_as(_vp)
 
     def forward_pass(self, batch, X):
         self._x, rows = self._row_pointers(X)
