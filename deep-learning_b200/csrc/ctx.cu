@@ -86,7 +86,7 @@ static dlb_status gemm_tensor_core(dlb_ctx *ctx, const GemmOperand &A, const Gem
   return st;
 }
 
-// The fused epilogue exists in the 2-CTA fp16-plane kernel at its default
+// The fused epilogues exist in the fp16-plane kernels on CTA pairs at their default
 // chunk, for K-major A, with both operands' planes kept by the caller and a
 // dense output.
 bool gemm_fused_supported(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, const float *C, long long ldc,
@@ -649,7 +649,10 @@ dlb_status dlb_fc_forward_activation(dlb_ctx *ctx, const float *X, const float *
   fe.mode = EPI_ACTIVATION;
   fe.af = af;
   fe.out = A_out;
-  if (A_lo && epilogue_dropout(dropout, &fe) && gemm_fused_supported(ctx, A, B, Z, n_out, rows, n_out, n_in)) {
+  const uintptr_t all = reinterpret_cast<uintptr_t>(Z) | reinterpret_cast<uintptr_t>(A_out) |
+                        reinterpret_cast<uintptr_t>(dropout ? dropout->noise : nullptr);
+  // (the epilogue moves quads of a row)
+  if (A_lo && n_out % 4 == 0 && (all & 15) == 0 && epilogue_dropout(dropout, &fe) && gemm_fused_supported(ctx, A, B, Z, n_out, rows, n_out, n_in)) {
     PlaneJob job;
     DLB_TRY(planes_open(ctx, A_out, A_lo, (size_t)rows * n_out, rows, n_out, true, &job));
     if (job.fused) {
@@ -674,7 +677,9 @@ dlb_status dlb_fc_backward_input_derivative(dlb_ctx *ctx, const float *delta, co
               "dlb_fc_backward_input_derivative");
   GemmOperand A{delta, delta_lo, n_out, 1};
   GemmOperand B{W, W_lo, 1, n_in};
-  if (dX_lo && gemm_fused_supported(ctx, A, B, dX, n_in, rows, n_in, n_out)) {
+  const uintptr_t all = reinterpret_cast<uintptr_t>(dX) | reinterpret_cast<uintptr_t>(Z_below) |
+                        reinterpret_cast<uintptr_t>(A_below);
+  if (dX_lo && n_in % 4 == 0 && (all & 15) == 0 && gemm_fused_supported(ctx, A, B, dX, n_in, rows, n_in, n_out)) {
     PlaneJob job;
     DLB_TRY(planes_open(ctx, dX, dX_lo, (size_t)rows * n_in, rows, n_in, true, &job));
     if (job.fused) {

@@ -37,7 +37,7 @@
 // do not depend on timing.
 #include "common.cuh"
 #include "gemm_simt.cuh"
-#include "tc_ptx.cuh"
+#include "tc_pair.cuh"
 
 namespace dlb {
 
@@ -75,42 +75,6 @@ struct DirectArgs {
   int *status;
 };
 
-__device__ __forceinline__ uint32_t direct_map(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void direct_arrive_remote(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// Bounded wait for the other CTAs' partial sums.
-__device__ __forceinline__ bool direct_wait_cluster(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status) {
-  const long long t0 = clock64();
-  while (true) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(20000u)
-        : "memory");
-    if (ok) return true;
-    if (*abort_flag) return false;
-    if (clock64() - t0 > WAIT_BUDGET_CLOCKS) {
-      *abort_flag = 1;
-      atomicExch(status, DLB_ERR_TIMEOUT);
-      return false;
-    }
-  }
-}
-__device__ __forceinline__ void st_cluster4(uint32_t addr, float a, float b, float c, float d) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
-               : "memory");
-}
-__device__ __forceinline__ void st_cluster_int(uint32_t addr, int v) {
-  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
 __device__ __forceinline__ void sts128(uint32_t addr, const uint32_t (&v)[4]) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
                : "memory");
@@ -331,7 +295,7 @@ __global__ void __launch_bounds__(D_THREADS, 1) gemm_direct_kernel(const __grid_
   const uint32_t tmem = *tmem_holder;
   // The cluster's other CTAs may write here from now on; the wait for theirs comes
   // before the first remote access.
-  if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (splits > 1) cluster_arrive();
   // The set-up above touches no global memory: it runs under the kernel before.
   pdl_enter();
 
@@ -430,7 +394,7 @@ __global__ void __launch_bounds__(D_THREADS, 1) gemm_direct_kernel(const __grid_
   const int width_shift = 7 - a.split_shift, width = 1 << width_shift, row_words = width + 4;
   tcgen05_fence_before();
   __syncthreads();  // the range flag is final
-  if (splits > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (splits > 1) cluster_wait();
   if (warp >= D_CONV_WARPS) {
     if (g * D_COLS < n_mma) {
       const int row = q * 32 + lane;
@@ -438,21 +402,21 @@ __global__ void __launch_bounds__(D_THREADS, 1) gemm_direct_kernel(const __grid_
       for (int j = 0; j < D_COLS; j += 4) {
         const int col = g * D_COLS + j, owner = col >> width_shift;
         const uint32_t at = base + D_PARTS + (uint32_t)(((piece * DM + row) * row_words + col - (owner << width_shift)) * 4);
-        st_cluster4(splits > 1 ? direct_map(at, (uint32_t)owner) : at, acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+        st_cluster4(splits > 1 ? map_to_cta(at, (uint32_t)owner) : at, acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
       }
     }
     if (splits > 1) {
       const int bad = *reinterpret_cast<volatile int *>(range_flag);
-      if (bad && lane < splits) st_cluster_int(direct_map(smem_u32(range_flag), (uint32_t)lane), 1);
+      if (bad && lane < splits) st_cluster_int(map_to_cta(smem_u32(range_flag), (uint32_t)lane), 1);
       asm volatile("fence.acq_rel.cluster;" ::: "memory");
       __syncwarp();
-      if (lane < splits) direct_arrive_remote(direct_map(parts_bar, (uint32_t)lane));
+      if (lane < splits) mbar_arrive_cluster(map_to_cta(parts_bar, (uint32_t)lane));
     } else {
       __syncwarp();
       if (lane == 0) mbar_arrive(parts_bar);
     }
   }
-  const bool here = direct_wait_cluster(parts_bar, 0, abort_flag, a.status);
+  const bool here = mbar_wait_cluster(parts_bar, 0, abort_flag, a.status);
   if (*reinterpret_cast<volatile int *>(range_flag)) {
     direct_fp32_tile(&a, m0, n0, piece, reinterpret_cast<float *>(smem));
   } else if (here) {

@@ -22,7 +22,8 @@
 
 #include "common.cuh"
 #include "gemm_simt.cuh"
-#include "tc_ptx.cuh"
+#include "gemm_store.cuh"
+#include "tc_pair.cuh"
 
 namespace dlb {
 
@@ -35,60 +36,6 @@ constexpr int PN = 256;  // columns of a pair's tile
 constexpr int PBK = 32;  // halfs per k-block (64-byte rows)
 constexpr int HALF_N = PN / 2;
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Address of the same shared-memory location in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// TMA loads of a CTA pair: the completion may be counted on the peer's barrier.
-__device__ __forceinline__ void tma_pair_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0,
-                                            int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tma_pair_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0,
-                                            int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-__device__ __forceinline__ void umma_pair_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                              uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Arrives on the barrier at this offset in both CTAs of the pair when all MMAs
-// issued so far have completed.
-__device__ __forceinline__ void umma_pair_commit(uint32_t bar) {
-  const uint16_t both = 3;
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-      ::"r"(bar), "h"(both)
-      : "memory");
-}
-
 template <int STAGES>
 struct PairPlan {
   static constexpr int A_BYTES = BM * PBK * 2;       // this CTA's 128 rows of A, one plane
@@ -96,7 +43,7 @@ struct PairPlan {
   static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
   static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
   static constexpr int EPI_OFFSET = RING_BYTES;
-  static constexpr int EPI_BYTES = NUM_DRAIN_WARPS * 32 * 33 * 4;
+  static constexpr int EPI_BYTES = NUM_DRAIN_WARPS * 32 * 32 * 4;
   static constexpr int BAR_OFFSET = EPI_OFFSET + EPI_BYTES;
   static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;
   static_assert(TOTAL <= 232448, "shared memory of one CTA");
@@ -151,27 +98,13 @@ template <int STAGES, int CHUNK_KB, bool A_MN, bool B_MN, bool FUSED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     gemm_x3_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_a_lo,
                         const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_b_lo,
-                        float *__restrict__ C, long long ldc, int M, int N, int K,
-                        const float *__restrict__ bias, int accumulate, int tiles_n, int band, int whole_tiles,
+                        const QuadTarget target, int K, int tiles_n, int band, int whole_tiles,
                         int parts, int total_items, const float *__restrict__ scale_a,
                         const float *__restrict__ scale_b, int *status, const unsigned *guard_a,
                         const unsigned *guard_b, unsigned mask_a, unsigned mask_b,
                         const float *__restrict__ line_inv_a, SimtOperands fp32, unsigned long long *fallbacks,
                         const FusedEpilogue fe) {
-  pdl_enter();
   using P = PairPlan<STAGES>;
-  // Range guard: the planes of a flagged operand do not stand for its tensor.
-  // The product is then formed from the fp32 tensors on the CUDA cores, every
-  // CTA taking its share of the 64 x 64 tiles (a rare and slow path that keeps
-  // the result right; the counter tells the host that it was taken).  Both
-  // CTAs of a pair read the same words and take the same branch.
-  if ((guard_a && (*guard_a & mask_a)) || (guard_b && (*guard_b & mask_b))) {
-    extern __shared__ __align__(16) uint8_t guard_smem[];
-    if (fallbacks && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(fallbacks, 1ull);
-    gemm_simt_guard_path(fp32, C, ldc, M, N, K, bias, accumulate, reinterpret_cast<float *>(guard_smem),
-                         FUSED ? &fe : nullptr);
-    return;
-  }
   constexpr int MN_W = 64;  // halfs of one 128-byte column of an MN-major tile
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -186,7 +119,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
   const uint32_t rank = cluster_rank();  // 0: the CTA that issues the MMAs
   const int pair = blockIdx.x / 2, pairs = gridDim.x / 2;
   const int total_kb = (K + PBK - 1) / PBK;
-  const int tiles_m = (M + PM - 1) / PM;
+  const int tiles_m = (target.M + PM - 1) / PM;
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES),
                  acc_full0 = smem_u32(bars + 2 * STAGES), acc_empty0 = smem_u32(bars + 2 * STAGES + 2);
 
@@ -201,6 +134,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     }
     *abort_flag = 0;
     *issued_kb = 0;
+    prefetch_tmap(&tm_a);
+    prefetch_tmap(&tm_a_lo);
+    prefetch_tmap(&tm_b);
+    prefetch_tmap(&tm_b_lo);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -216,8 +153,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
   cluster_sync_all();  // both CTAs' barriers exist before anything arrives on them
   tcgen05_fence_after();
   const uint32_t tmem_acc = *tmem_holder;
+  // The set-up above touches no global memory: it runs under the kernel before.
+  pdl_enter();
 
-  if (warp == 0) {
+  // Range guard: the planes of a flagged operand do not stand for its tensor.
+  // The product is then formed from the fp32 tensors on the CUDA cores, every
+  // CTA taking its share of the 64 x 64 tiles (a rare and slow path that keeps
+  // the result right; the counter tells the host that it was taken).  Both
+  // CTAs of a pair read the same words and take the same branch.
+  const bool flagged = (guard_a && (*guard_a & mask_a)) || (guard_b && (*guard_b & mask_b));
+  if (flagged) {
+    if (fallbacks && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(fallbacks, 1ull);
+    gemm_simt_guard_path(fp32, target.C, target.ldc, target.M, target.N, K, target.bias, target.accumulate,
+                         reinterpret_cast<float *>(smem), FUSED ? &fe : nullptr);
+  } else if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
     if (lane == 0) {
       const uint32_t lead_full0 = map_to_cta(full0, 0);
@@ -259,13 +208,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
       // fp32 accumulate, F16 operands, majors, N = 256, M = 256 over the pair.
       const uint32_t idesc = (1u << 4) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) |
                              ((uint32_t)(PN >> 3) << 17) | ((uint32_t)(PM >> 4) << 24);
-      constexpr int KI = 16;
-      constexpr uint32_t K_ROW = PBK * 2;  // 64-byte rows, 64-byte swizzle
-      constexpr uint32_t A_LBO = A_MN ? PBK * 128 : 16, A_SBO = A_MN ? 1024 : 8 * K_ROW;
-      constexpr uint32_t B_LBO = B_MN ? PBK * 128 : 16, B_SBO = B_MN ? 1024 : 8 * K_ROW;
-      constexpr uint32_t A_LAYOUT = A_MN ? LAYOUT_SW128 : LAYOUT_SW64;
-      constexpr uint32_t B_LAYOUT = B_MN ? LAYOUT_SW128 : LAYOUT_SW64;
-      constexpr uint32_t A_KSTEP = A_MN ? KI * 128 : 32, B_KSTEP = B_MN ? KI * 128 : 32;
+      // k-major: 64-byte rows and swizzle; mn-major: 128-byte columns of 64 lines.  The
+      // descriptors are built once; steps in their address field are 16 bytes.
+      // (Three stages of 64 k measured the same for k-major operands and 8 - 15 %
+      // slower for weight gradients.)
+      constexpr uint32_t A_LBO = A_MN ? PBK * 128 : 16, A_SBO = A_MN ? 1024 : 8 * PBK * 2;
+      constexpr uint32_t B_LBO = B_MN ? PBK * 128 : 16, B_SBO = B_MN ? 1024 : 8 * PBK * 2;
+      constexpr uint32_t A_KSTEP = (A_MN ? 16 * 128 : 32) >> 4, B_KSTEP = (B_MN ? 16 * 128 : 32) >> 4;
+      const uint64_t desc_a = make_smem_desc(base, A_LBO, A_SBO, A_MN ? LAYOUT_SW128 : LAYOUT_SW64),
+                     desc_b = make_smem_desc(base + 2 * P::A_BYTES, B_LBO, B_SBO, B_MN ? LAYOUT_SW128 : LAYOUT_SW64);
       bool ok = true;
       unsigned it = 0, cc = 0;
       for (int item = pair; item < total_items && ok; item += pairs) {
@@ -278,26 +229,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
           tcgen05_fence_after();
           const uint32_t d_tmem = tmem_acc + (uint32_t)(buf * PN);
           const int kb_end = min(w.num_kb, kb + CHUNK_KB);
-          bool first = true;
+          uint32_t add = 0u;
           for (; kb < kb_end; ++kb, ++it) {
             const unsigned s = it % STAGES;
             const uint32_t ph = (it / STAGES) & 1;
             ok = mbar_wait(full0 + 8 * s, ph, abort_flag, status);
             if (!ok) break;
             tcgen05_fence_after();
-            const uint32_t st = base + s * P::STAGE_BYTES;
-            const uint32_t a_hi = st, a_lo = st + P::A_BYTES, b_hi = st + 2 * P::A_BYTES,
-                           b_lo = st + 2 * P::A_BYTES + P::B_BYTES;
+            const uint64_t a_hi = desc_a + (uint64_t)(s * (P::STAGE_BYTES >> 4)),
+                           b_hi = desc_b + (uint64_t)(s * (P::STAGE_BYTES >> 4));
 #pragma unroll
-            for (int k8 = 0; k8 < PBK / KI; ++k8) {
-              const uint64_t da_hi = make_smem_desc(a_hi + k8 * A_KSTEP, A_LBO, A_SBO, A_LAYOUT);
-              const uint64_t da_lo = make_smem_desc(a_lo + k8 * A_KSTEP, A_LBO, A_SBO, A_LAYOUT);
-              const uint64_t db_hi = make_smem_desc(b_hi + k8 * B_KSTEP, B_LBO, B_SBO, B_LAYOUT);
-              const uint64_t db_lo = make_smem_desc(b_lo + k8 * B_KSTEP, B_LBO, B_SBO, B_LAYOUT);
-              umma_pair_f16(d_tmem, da_lo, db_hi, idesc, first ? 0u : 1u);
-              umma_pair_f16(d_tmem, da_hi, db_lo, idesc, 1u);
-              umma_pair_f16(d_tmem, da_hi, db_hi, idesc, 1u);
-              first = false;
+            for (int k = 0; k < PBK / 16; ++k) {
+              umma_pair_f16(d_tmem, a_hi + (P::A_BYTES >> 4) + k * A_KSTEP, b_hi + k * B_KSTEP, idesc, add);
+              umma_pair_f16(d_tmem, a_hi + k * A_KSTEP, b_hi + (P::B_BYTES >> 4) + k * B_KSTEP, idesc, 1u);
+              umma_pair_f16(d_tmem, a_hi + k * A_KSTEP, b_hi + k * B_KSTEP, idesc, 1u);
+              add = 1u;
             }
             umma_pair_commit(empty0 + 8 * s);
           }
@@ -311,7 +257,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     const int q = warp & 3;
     const int h = (warp - 2) >> 2;
     constexpr int HALF = PN / 2;
-    float *tile = reinterpret_cast<float *>(smem + P::EPI_OFFSET) + (warp - 2) * 32 * 33;
+    float4 *tile = reinterpret_cast<float4 *>(smem + P::EPI_OFFSET) + (warp - 2) * 32 * 8;
     const float out_b = 1.f / __ldg(scale_b);
     const float tensor_out_a = line_inv_a ? 1.f : 1.f / __ldg(scale_a);
     const float plane_scale = FUSED && fe.sink.hi ? sink_scale(fe.sink) : 1.f;
@@ -345,61 +291,78 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
       if (!ok) break;
       const int row_base = w.m0 + (int)rank * BM + q * 32;
       // This thread holds row row_base + lane; planes with a scale per line bring 1 / scale per row.
-      const float out_a = line_inv_a ? __ldg(line_inv_a + min(row_base + lane, M - 1)) : tensor_out_a;
+      const float out_a = line_inv_a ? __ldg(line_inv_a + min(row_base + lane, target.M - 1)) : tensor_out_a;
+      QuadTarget t = target;
+      t.atomic = w.split;
+      if (w.piece != 0) t.bias = nullptr;
+      const bool plain = target.quads && !target.accumulate && !w.split;
+      // 32 x 32 pieces turn through shared memory: rows go in by thread, quads of a
+      // row come out, eight lanes to a row (16-byte slot c of row r lies at
+      // c ^ (r & 7), so both sides touch all banks).
+      const int r8 = lane >> 3, cs = lane & 7;
 #pragma unroll
       for (int j = 0; j < HALF / 32; ++j) {
-        const int col0 = w.n0 + h * HALF + j * 32;
-        if (col0 < N) {
+        const int col0 = w.n0 + h * HALF + j * 32, col = col0 + cs * 4;
+        if (col0 >= target.N) continue;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) tile[lane * 33 + i] = acc[j * 32 + i] * out_a * out_b;
-          __syncwarp();
-          const int col = col0 + lane;
-          if (col < N) {
-            const float b = (bias && w.piece == 0) ? __ldg(bias + col) : 0.f;
-            if (FUSED) {
-              // Launches with a fused epilogue have no split tiles and do not
-              // accumulate.  The lanes of the warp that are here hold 32
-              // consecutive columns of one row at a time.
-              const float keep = epilogue_keep(fe, col);
-              unsigned col_max = 0u;
-#pragma unroll 2
-              for (int r = 0; r < 32; ++r) {
-                const int row = row_base + r;
-                if (row < M) {
-                  const size_t at = (size_t)row * N + col;
-                  const float x = epilogue_store(fe, C + (long long)row * ldc + col, at, tile[r * 33 + lane] + b, keep);
-                  if (fe.sink.hi) epilogue_planes(fe, at, x, plane_scale);
-                  const unsigned bits = abs_bits(x);
-                  col_max = max(col_max, bits);
-                  if (fe.sink.rowmax) {
-                    const unsigned row_max = __reduce_max_sync(__activemask(), bits);
-                    if (lane == 0 && row_max) atomicMax(fe.sink.rowmax + row, row_max);
-                  }
-                }
-              }
-              if (fe.sink.colmax && col_max) atomicMax(fe.sink.colmax + col, col_max);
-              if (fe.sink.slot) amax_commit(reinterpret_cast<unsigned *>(fe.sink.slot) + SLOT_AMAX, col_max);
-            } else if (w.split) {
-#pragma unroll 4
-              for (int r = 0; r < 32; ++r) {
-                const int row = row_base + r;
-                if (row < M) atomicAdd(C + (long long)row * ldc + col, tile[r * 33 + lane] + b);
-              }
-            } else {
-#pragma unroll 4
-              for (int r = 0; r < 32; ++r) {
-                const int row = row_base + r;
-                if (row < M) {
-                  float *dst = C + (long long)row * ldc + col;
-                  float val = tile[r * 33 + lane] + b;
-                  if (accumulate) val += *dst;
-                  *dst = val;
-                }
-              }
+        for (int c = 0; c < 8; ++c)
+          tile[lane * 8 + (c ^ (lane & 7))] =
+              make_float4(acc[j * 32 + 4 * c] * out_a * out_b, acc[j * 32 + 4 * c + 1] * out_a * out_b,
+                          acc[j * 32 + 4 * c + 2] * out_a * out_b, acc[j * 32 + 4 * c + 3] * out_a * out_b);
+        __syncwarp();
+        const float4 b4 = quad_bias(t, col);
+        const bool live = col < target.N;
+        if (FUSED) {
+          // Launches with a fused epilogue have no split tiles and do not accumulate;
+          // N is a multiple of four.
+          const float4 keep =
+              live ? make_float4(epilogue_keep(fe, col), epilogue_keep(fe, col + 1), epilogue_keep(fe, col + 2),
+                                 epilogue_keep(fe, col + 3))
+                   : b4;
+          QuadTracker track;
+#pragma unroll 1
+          for (int i0 = 0; i0 < 8; i0 += 4) {
+            FusedLoads in[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int row = row_base + r8 + 4 * (i0 + i);
+              if (live && row < target.M) in[i] = fused_loads(fe, (size_t)row * target.N + col);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int r = r8 + 4 * (i0 + i), row = row_base + r;
+              const bool inside = live && row < target.M;
+              float4 x = tile[r * 8 + (cs ^ (r & 7))];
+              x.x += b4.x, x.y += b4.y, x.z += b4.z, x.w += b4.w;
+              const size_t at = (size_t)row * target.N + col;
+              if (inside) x = fused_quad(fe, target.C + at, at, x, keep, in[i], plane_scale);
+              track.row(fe.sink, row, inside, x, 8);
             }
           }
-          __syncwarp();
+          track.finish(fe.sink, col, target.N, 8);
+        } else if (live) {
+          float4 x[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int r = r8 + 4 * i;
+            x[i] = tile[r * 8 + (cs ^ (r & 7))];
+            x[i].x += b4.x, x[i].y += b4.y, x[i].z += b4.z, x[i].w += b4.w;
+          }
+          if (plain) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int row = row_base + r8 + 4 * i;
+              if (row < target.M) *reinterpret_cast<float4 *>(target.C + (long long)row * target.ldc + col) = x[i];
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int row = row_base + r8 + 4 * i;
+              if (row < target.M) store_quad(t, row, col, x[i]);
+            }
+          }
         }
+        __syncwarp();
       }
     }
   }
@@ -505,12 +468,22 @@ dlb_status launch_pair(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B,
                                (size_t)(N - first_col) * sizeof(float), (size_t)(M - first_row), ctx->stream));
   }
   const int items = whole_tiles + parts * split_tiles;
-  DLB_LAUNCH_KERNEL(ctx, kernel, 2 * min(items, lanes), NUM_THREADS, P::TOTAL, ta, tal, tb, tbl, C, ldc, M, N, K, ep.bias, ep.accumulate, tiles_n, band, whole_tiles, parts, items, A.scale, B.scale, ctx->d_status, A.guard, B.guard, A.guard_mask, B.guard_mask, A.line_inv, SimtOperands{A.ptr, A.fp32_stride_mn ? A.fp32_stride_mn : A.stride_mn, A.fp32_stride_k ? A.fp32_stride_k : A.stride_k, B.ptr, B.stride_mn, B.stride_k}, ctx->d_guard ? ctx->d_guard + 1 : nullptr, FUSED ? *ep.fused : FusedEpilogue{});
+  DLB_LAUNCH_KERNEL(ctx, kernel, 2 * min(items, lanes), NUM_THREADS, P::TOTAL, ta, tal, tb, tbl, quad_target(C, ldc, M, N, ep.bias, ep.accumulate), K, tiles_n, band, whole_tiles, parts, items, A.scale, B.scale, ctx->d_status, A.guard, B.guard, A.guard_mask, B.guard_mask, A.line_inv, SimtOperands{A.ptr, A.fp32_stride_mn ? A.fp32_stride_mn : A.stride_mn, A.fp32_stride_k ? A.fp32_stride_k : A.stride_k, B.ptr, B.stride_mn, B.stride_k}, ctx->d_guard ? ctx->d_guard + 1 : nullptr, FUSED ? *ep.fused : FusedEpilogue{});
   DLB_LAUNCHED(ctx);
   return DLB_OK;
 }
 
 }  // namespace
+
+// About how long the product takes here: rounds of one 256 x 256 tile per pair, the
+// last one cut in two where launch_pair would.
+double gemm_pair_us(const dlb_ctx *ctx, int M, int N, int K, bool whole_tiles) {
+  const int tiles = ceil_div(M, PM) * ceil_div(N, PN), lanes = ctx->sm_count / 2, kb = ceil_div(K, PBK);
+  double rounds = tiles / lanes;
+  const int rest = tiles % lanes;
+  if (rest) rounds += !whole_tiles && 2 * rest <= lanes && kb >= 64 ? 0.6 : 1.0;
+  return 9.0 + rounds * 0.42 * kb;
+}
 
 // On unless DLB_GEMM_PAIR=0.
 bool gemm_pair_enabled() {

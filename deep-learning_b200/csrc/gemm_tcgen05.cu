@@ -444,15 +444,24 @@ bool tmap_cached(dlb_ctx *ctx, CUtensorMap *out, bool mn_major, const void *ptr,
   return true;
 }
 
+bool tmap_plane(dlb_ctx *ctx, CUtensorMap *out, bool mn_major, const void *ptr, uint64_t mn, uint64_t k, uint64_t ld,
+                uint32_t box_k, uint32_t lines) {
+  if (!mn_major) return tmap_cached(ctx, out, false, ptr, 2, mn, k, ld, box_k, lines);
+  // In the cache's terms a k-major map of the transposed view: rows of mn, 64 of
+  // them (128 bytes, the plain 128-byte swizzle) x box_k per box.
+  return tmap_cached(ctx, out, false, ptr, 2, k, mn, ld, 64, box_k);
+}
+
 namespace {
 
 // What TMA can address: 16-byte aligned base and row pitch; an MN-major extent
 // that is a whole number of 128-byte columns.
-bool operand_ok(const void *ptr, int es, long long stride_mn, long long stride_k, int mn, int k) {
+bool operand_ok(const void *ptr, int es, long long stride_mn, long long stride_k, int mn, int k,
+                bool any_extent = false) {
   const int per16 = 16 / es, w = 128 / es;
   if (reinterpret_cast<uintptr_t>(ptr) & 15) return false;
   if (stride_k == 1) return stride_mn % per16 == 0 && stride_mn >= k;
-  if (stride_mn == 1) return stride_k % per16 == 0 && stride_k >= mn && mn % w == 0;
+  if (stride_mn == 1) return stride_k % per16 == 0 && stride_k >= mn && (any_extent || mn % w == 0);
   return false;
 }
 
@@ -582,11 +591,14 @@ bool gemm_tcgen05_supported(const GemmOperand &A, const GemmOperand &B, const fl
 }
 
 // The fp16-plane form: planes have the strides of their tensor, so the test is
-// on the strides alone (the planes' own base alignment is checked at launch).
+// on the strides alone (the planes' own base alignment is checked at launch).  An
+// MN-major B of any extent runs on gemm_mid_kernel; an MN-major A does not have to:
+// weight gradients whose output rows are no multiple of 64 get planes of their own
+// or none (gemm() in ctx.cu).
 bool gemm_f16_supported(const GemmOperand &A, const GemmOperand &B, const float *C, long long ldc,
                         int M, int N, int K) {
   return shape_ok(A, B, C, ldc, M, N, K) && operand_ok(nullptr, 2, A.stride_mn, A.stride_k, M, K) &&
-         operand_ok(nullptr, 2, B.stride_mn, B.stride_k, N, K);
+         operand_ok(nullptr, 2, B.stride_mn, B.stride_k, N, K, gemm_pair_enabled() && (long long)M * N >= 256 * 256);
 }
 
 dlb_status gemm_tcgen05(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C,
@@ -598,7 +610,15 @@ dlb_status gemm_tcgen05(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B
       set_error("gemm_tcgen05: fp16 planes outside the TMA path");
       return DLB_ERR_UNSUPPORTED;
     }
-    if (gemm_pair_enabled() && (long long)M * N >= 256 * 256) return gemm_pair(ctx, A, B, C, ldc, M, N, K, ep);
+    if (gemm_pair_enabled() && (long long)M * N >= 256 * 256) {
+      // 256 x 256 tiles, or 256 x 128 with the k range shared: whichever is done first.
+      int split_shift = 0;
+      const double mid_us = gemm_mid_us(ctx, M, N, K, &split_shift);
+      const bool ragged = B.stride_k != 1 && N % 64 != 0;  // the pair kernel's 3-d maps want whole columns of 64
+      if (ragged || mid_us < gemm_pair_us(ctx, M, N, K, ep.accumulate || ep.fused))
+        return gemm_mid(ctx, A, B, C, ldc, M, N, K, split_shift, ep);
+      return gemm_pair(ctx, A, B, C, ldc, M, N, K, ep);
+    }
     if (ep.fused) {
       set_error("gemm_tcgen05: a fused epilogue runs on the 2-CTA kernel only");
       return DLB_ERR_UNSUPPORTED;

@@ -175,9 +175,18 @@ bool tmap_mn_major(CUtensorMap *m, const void *ptr, int es, uint64_t mn, uint64_
                    uint32_t box_k, uint32_t box_mn);
 bool tmap_cached(dlb_ctx *ctx, CUtensorMap *out, bool mn_major, const void *ptr, int es, uint64_t mn,
                  uint64_t k, uint64_t ld, uint32_t box_k, uint32_t box_mn);
-// The 2-CTA form of the fp16-plane product (gemm_pair.cu).
+// fp16 planes of an operand of which a CTA loads `lines` lines per k-block: one box
+// of {box_k, lines} where k is contiguous, boxes of {64 lines, box_k} where mn is.
+bool tmap_plane(dlb_ctx *ctx, CUtensorMap *out, bool mn_major, const void *ptr, uint64_t mn, uint64_t k, uint64_t ld,
+                uint32_t box_k, uint32_t lines);
+// The 2-CTA form of the fp16-plane product (gemm_pair.cu), and the form with smaller
+// tiles and up to four pairs per tile (gemm_mid.cu).
+dlb_status gemm_mid(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C, long long ldc, int M, int N,
+                    int K, int split_shift, const GemmEpilogue &ep);
+double gemm_mid_us(const dlb_ctx *ctx, int M, int N, int K, int *split_shift);
 bool gemm_pair_enabled();
 int gemm_pair_chunk();
+double gemm_pair_us(const dlb_ctx *ctx, int M, int N, int K, bool whole_tiles);
 dlb_status gemm_pair(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C, long long ldc,
                      int M, int N, int K, const GemmEpilogue &ep);
 
