@@ -47,6 +47,7 @@ struct dlb_ctx {
   };
   std::map<uintptr_t, PlaneEntry> planes;
   bool guard_strict = false;        // no exemptions (dlb_ctx_set_guard_strict)
+  std::map<uintptr_t, size_t> planes_unused;  // plane buffers (address, bytes) no product reads at the sizes in use
   std::map<uintptr_t, size_t> rows_exempt;  // plane buffers (address, bytes) of tensors whose small rows are not guarded
   // Bumped by dlb_ctx_set_gemm_kind, which also drops every registration above:
   // a model compares it with the value it last split its weights under and
@@ -266,6 +267,9 @@ dlb_status gemm_simt(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, f
 dlb_status gemm_direct(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C, long long ldc, int M, int N,
                        int K, const GemmEpilogue &ep);
 bool gemm_direct_supported(const GemmOperand &A, const GemmOperand &B);
+// Whether a product on planes runs on gemm_mid_kernel, and into how many pieces
+// (1 << split_shift) its k range is cut there.
+bool gemm_mid_chosen(const dlb_ctx *ctx, const GemmOperand &B, int M, int N, int K, bool accumulate, int *split_shift);
 double gemm_direct_us(const dlb_ctx *ctx, int M, int N, int K);  // about how long it takes
 // Returns DLB_ERR_UNSUPPORTED (without touching C) when the shape or alignment
 // is outside what the TMA descriptors can express.
@@ -308,6 +312,16 @@ bool planes_lookup(dlb_ctx *ctx, const float *aux, GemmOperand *o);
 // the backward pass whose rows are the examples of a batch: the range guard
 // then leaves its small rows alone (planes.cuh), unless the context is strict.
 void planes_rows_exempt(dlb_ctx *ctx, const float *planes, size_t bytes, bool on);
+// Marks (or unmarks) the plane buffer [planes, planes + bytes) as one that no product
+// reads at the sizes in use: producers then leave it alone and products do not
+// look it up.
+void planes_unused(dlb_ctx *ctx, const float *planes, size_t bytes, bool on);
+bool planes_unused_at(const dlb_ctx *ctx, const float *planes);
+// Which operands' kept planes gemm() would read for a product with these strides.
+struct PlaneUse {
+  bool a, b;
+};
+PlaneUse gemm_plane_use(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K);
 // x [K, M] with row pitch `pitch` (mn contiguous) -> fp16 planes [M, kp] (k
 // contiguous), line m scaled by a power of two of its own taken from the
 // line's largest |x| (`cmax`, M words of scratch); line_inv[m] = 1 / scale.
@@ -372,6 +386,7 @@ bool gemm_fused_supported(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand 
 // max |x| (sink.slot) and planes_close runs the split pass.  planes_close then
 // launches the check that sets the slot's scale and guard flag for the
 // consumers and the prediction for the next split (planes_finalize_kernel).
+// A buffer marked unused leaves the job inactive: nothing to write or to track.
 struct PlaneJob {
   PlaneSink sink;
   const float *x = nullptr;

@@ -86,17 +86,39 @@ static dlb_status gemm_tensor_core(dlb_ctx *ctx, const GemmOperand &A, const Gem
   return st;
 }
 
-// The fused epilogues exist in the fp16-plane kernels on CTA pairs at their default
-// chunk, for K-major A, with both operands' planes kept by the caller and a
-// dense output.
+// The fused epilogues exist in the medium fp16-plane kernel, for K-major A, with both
+// operands' planes kept by the caller and a dense output.  Outputs large enough
+// for the persistent kernel on 256 x 256 tiles take the kernels one after the
+// other: a tile's epilogue there is longer than the next tile's products (2048^3
+// with UOut and planes: 104 us against 40 + 26; 4096^3: 527 against 277 + 85).
 bool gemm_fused_supported(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, const float *C, long long ldc,
                           int M, int N, int K) {
   const bool big = (long long)M * N >= 256 * 256 && K >= 32;
   if (!(ctx->use_tensor_core && ctx->tensor_core_ok && big && ctx->gemm_kind == DLB_GEMM_F16X3)) return false;
-  if (!gemm_pair_enabled() || gemm_pair_chunk() != 8 || A.stride_k != 1 || ldc != N) return false;
+  int split_shift;
+  if (!gemm_pair_enabled() || gemm_pair_chunk() != 8 || A.stride_k != 1 || ldc != N ||
+      !gemm_mid_chosen(ctx, B, M, N, K, false, &split_shift))
+    return false;
   if (!gemm_f16_supported(A, B, C, ldc, M, N, K)) return false;
   GemmOperand a = A, b = B;
   return (a.h_hi || planes_lookup(ctx, a.lo, &a)) && (b.h_hi || planes_lookup(ctx, b.lo, &b));
+}
+
+// A product with both operands' planes kept runs on them where the output fills a
+// 256 x 256 tile and TMA can address them.
+static bool plane_size(int M, int N, int K) { return (long long)M * N >= 256 * 256 && K >= 32; }
+// About how long a product on kept planes takes.
+static double planes_us(int M, int N, int K) { return 2.0 * M * N * K / 4.5e8; }
+// Planes of A made for the product, transposed, instead of splitting in the product.
+static bool transposed_better(const dlb_ctx *ctx, int M, int N, int K) {
+  return gemm_direct_us(ctx, M, N, K) > planes_us(M, N, K) + 45.0;
+}
+
+PlaneUse gemm_plane_use(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K) {
+  if (ctx->gemm_kind != DLB_GEMM_F16X3) return {true, true};
+  if (!plane_size(M, N, K)) return {false, false};
+  if (gemm_f16_supported(A, B, nullptr, N, M, N, K) && !A.rescale_lines) return {true, true};
+  return {false, A.stride_k != 1 && B.stride_k != 1 && gemm_pair_enabled() && transposed_better(ctx, M, N, K)};
 }
 
 dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, float *C,
@@ -121,15 +143,12 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
   // maxima, split and check of two operands; 45 us when one is transposed) and
   // 450 TFLOP/s (1024^3: 30 us against 67, 2048^3: 188 against 95).
   const bool direct_form = ctx->gemm_kind == DLB_GEMM_F16X3 && !ep.fused && gemm_direct_supported(A, B);
-  const double direct_us = direct_form ? gemm_direct_us(ctx, M, N, K) : 1e30;
-  const double planes_us = 2.0 * M * N * K / 4.5e8;
   auto direct = [&]() -> dlb_status {
     ProfileSpan span;
     DLB_TRY(span.begin(ctx, 0, 2.0 * M * N * K));
     DLB_TRY(gemm_direct(ctx, A_in, B_in, C, ldc, M, N, K, ep));
     return span.end();
   };
-  const bool plane_size = (long long)M * N >= 256 * 256 && K >= 32;
 
   // A weight-gradient product (both operands mn-contiguous) whose A TMA cannot
   // tile as it lies (output rows not a multiple of 64, e.g. 1000 classes), or
@@ -143,8 +162,9 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
   // each output row multiplied by its line's 1 / scale.  Nothing of A is left
   // for the range guard to flag.
   if (ctx->gemm_kind == DLB_GEMM_F16X3 && A.stride_mn == 1 && A.stride_k != 1 && B.stride_mn == 1 &&
-      B.stride_k != 1 && gemm_pair_enabled() && plane_size && !ep.fused &&
-      (A.rescale_lines || !gemm_f16_supported(A, B, C, ldc, M, N, K)) && direct_us > planes_us + 45.0) {
+      B.stride_k != 1 && gemm_pair_enabled() && plane_size(M, N, K) && !ep.fused &&
+      (A.rescale_lines || !gemm_f16_supported(A, B, C, ldc, M, N, K)) &&
+      (!direct_form || transposed_better(ctx, M, N, K))) {
     GemmOperand a = A, b = B;
     const bool have_b = b.h_hi || planes_lookup(ctx, b.lo, &b);
     const long long kp = (long long)align_up((size_t)K, 8);
@@ -173,10 +193,10 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
   }
 
   if (direct_form && A.h_hi == nullptr) {  // (A.h_hi: planes just made for this product)
-    if (!plane_size || !gemm_f16_supported(A, B, C, ldc, M, N, K) || A.rescale_lines) return direct();
+    if (!plane_size(M, N, K) || !gemm_f16_supported(A, B, C, ldc, M, N, K) || A.rescale_lines) return direct();
     GemmOperand a = A, b = B;
     const bool have = planes_lookup(ctx, a.lo, &a) && planes_lookup(ctx, b.lo, &b);
-    if (!have && direct_us <= planes_us + 55.0) return direct();
+    if (!have && gemm_direct_us(ctx, M, N, K) <= planes_us(M, N, K) + 55.0) return direct();
   }
 
   if (ctx->gemm_kind == DLB_GEMM_F16X3 && gemm_f16_supported(A, B, C, ldc, M, N, K)) {
@@ -544,6 +564,8 @@ dlb_status dlb_free(dlb_ctx *ctx, void *dev_ptr) {
   auto it = ctx->allocs.find(reinterpret_cast<uintptr_t>(dev_ptr));
   if (it != ctx->allocs.end()) {
     planes_forget(ctx, it->first, it->second);
+    auto mark = ctx->planes_unused.lower_bound(it->first);
+    while (mark != ctx->planes_unused.end() && mark->first < it->first + it->second) mark = ctx->planes_unused.erase(mark);
     ctx->allocs.erase(it);
   }
   DLB_CUDA(cudaFree(dev_ptr));
@@ -655,7 +677,7 @@ dlb_status dlb_fc_forward_activation(dlb_ctx *ctx, const float *X, const float *
   if (A_lo && n_out % 4 == 0 && (all & 15) == 0 && epilogue_dropout(dropout, &fe) && gemm_fused_supported(ctx, A, B, Z, n_out, rows, n_out, n_in)) {
     PlaneJob job;
     DLB_TRY(planes_open(ctx, A_out, A_lo, (size_t)rows * n_out, rows, n_out, true, &job));
-    if (job.fused) {
+    if (job.fused || !job.active) {  // (inactive: nobody reads A's planes, the epilogue writes none)
       fe.sink = job.sink;
       GemmEpilogue ep;
       ep.bias = bias;
@@ -682,7 +704,7 @@ dlb_status dlb_fc_backward_input_derivative(dlb_ctx *ctx, const float *delta, co
   if (dX_lo && n_in % 4 == 0 && (all & 15) == 0 && gemm_fused_supported(ctx, A, B, dX, n_in, rows, n_in, n_out)) {
     PlaneJob job;
     DLB_TRY(planes_open(ctx, dX, dX_lo, (size_t)rows * n_in, rows, n_in, true, &job));
-    if (job.fused) {
+    if (job.fused || !job.active) {
       FusedEpilogue fe;
       fe.mode = EPI_DERIVATIVE;
       fe.af = af_below;

@@ -94,16 +94,15 @@ __device__ __forceinline__ PairItem pair_item(int item, int tiles_m, int tiles_n
   return w;
 }
 
-template <int STAGES, int CHUNK_KB, bool A_MN, bool B_MN, bool FUSED>
+template <int STAGES, int CHUNK_KB, bool A_MN, bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     gemm_x3_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_a_lo,
                         const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_b_lo,
-                        const QuadTarget target, int K, int tiles_n, int band, int whole_tiles,
+                        const __grid_constant__ QuadTarget target, int K, int tiles_n, int band, int whole_tiles,
                         int parts, int total_items, const float *__restrict__ scale_a,
                         const float *__restrict__ scale_b, int *status, const unsigned *guard_a,
                         const unsigned *guard_b, unsigned mask_a, unsigned mask_b,
-                        const float *__restrict__ line_inv_a, SimtOperands fp32, unsigned long long *fallbacks,
-                        const FusedEpilogue fe) {
+                        const float *__restrict__ line_inv_a, SimtOperands fp32, unsigned long long *fallbacks) {
   using P = PairPlan<STAGES>;
   constexpr int MN_W = 64;  // halfs of one 128-byte column of an MN-major tile
   extern __shared__ uint8_t smem_raw[];
@@ -165,7 +164,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
   if (flagged) {
     if (fallbacks && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(fallbacks, 1ull);
     gemm_simt_guard_path(fp32, target.C, target.ldc, target.M, target.N, K, target.bias, target.accumulate,
-                         reinterpret_cast<float *>(smem), FUSED ? &fe : nullptr);
+                         reinterpret_cast<float *>(smem));
   } else if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
     if (lane == 0) {
@@ -260,7 +259,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     float4 *tile = reinterpret_cast<float4 *>(smem + P::EPI_OFFSET) + (warp - 2) * 32 * 8;
     const float out_b = 1.f / __ldg(scale_b);
     const float tensor_out_a = line_inv_a ? 1.f : 1.f / __ldg(scale_a);
-    const float plane_scale = FUSED && fe.sink.hi ? sink_scale(fe.sink) : 1.f;
     const uint32_t lead_acc_empty0 = map_to_cta(acc_empty0, 0);
     float acc[HALF];
     bool ok = true;
@@ -312,35 +310,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
         __syncwarp();
         const float4 b4 = quad_bias(t, col);
         const bool live = col < target.N;
-        if (FUSED) {
-          // Launches with a fused epilogue have no split tiles and do not accumulate;
-          // N is a multiple of four.
-          const float4 keep =
-              live ? make_float4(epilogue_keep(fe, col), epilogue_keep(fe, col + 1), epilogue_keep(fe, col + 2),
-                                 epilogue_keep(fe, col + 3))
-                   : b4;
-          QuadTracker track;
-#pragma unroll 1
-          for (int i0 = 0; i0 < 8; i0 += 4) {
-            FusedLoads in[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int row = row_base + r8 + 4 * (i0 + i);
-              if (live && row < target.M) in[i] = fused_loads(fe, (size_t)row * target.N + col);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int r = r8 + 4 * (i0 + i), row = row_base + r;
-              const bool inside = live && row < target.M;
-              float4 x = tile[r * 8 + (cs ^ (r & 7))];
-              x.x += b4.x, x.y += b4.y, x.z += b4.z, x.w += b4.w;
-              const size_t at = (size_t)row * target.N + col;
-              if (inside) x = fused_quad(fe, target.C + at, at, x, keep, in[i], plane_scale);
-              track.row(fe.sink, row, inside, x, 8);
-            }
-          }
-          track.finish(fe.sink, col, target.N, 8);
-        } else if (live) {
+        if (live) {
           float4 x[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -398,7 +368,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 // ---------------------------------------------------------------------------
 namespace {
 
-template <int STAGES, int CHUNK_KB, bool A_MN, bool B_MN, bool FUSED = false>
+template <int STAGES, int CHUNK_KB, bool A_MN, bool B_MN>
 dlb_status launch_pair(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C, long long ldc,
                        int M, int N, int K, const GemmEpilogue &ep) {
   using P = PairPlan<STAGES>;
@@ -412,7 +382,7 @@ dlb_status launch_pair(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B,
     set_error("gemm_pair: cuTensorMapEncodeTiled rejected an operand");
     return DLB_ERR_CUDA;
   }
-  auto kernel = gemm_x3_pair_kernel<STAGES, CHUNK_KB, A_MN, B_MN, FUSED>;
+  auto kernel = gemm_x3_pair_kernel<STAGES, CHUNK_KB, A_MN, B_MN>;
   static bool attr_set[MAX_DEVICES] = {};  // the attribute belongs to the (function, device) pair
   if (!attr_set[ctx->device]) {
     DLB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P::TOTAL));
@@ -433,7 +403,7 @@ dlb_status launch_pair(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B,
   const int total_kb = ceil_div(K, PBK);
   const int rest = tiles % lanes;
   int parts = 1;
-  if (!ep.accumulate && rest > 0 && !FUSED) {  // a fused epilogue needs the whole sum of an element in one place
+  if (!ep.accumulate && rest > 0) {
     // Twelfths of a round; a cut must save at least a twelfth per extra piece.
     int best = 12;
     constexpr int MAX_PARTS = 2;
@@ -468,7 +438,7 @@ dlb_status launch_pair(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B,
                                (size_t)(N - first_col) * sizeof(float), (size_t)(M - first_row), ctx->stream));
   }
   const int items = whole_tiles + parts * split_tiles;
-  DLB_LAUNCH_KERNEL(ctx, kernel, 2 * min(items, lanes), NUM_THREADS, P::TOTAL, ta, tal, tb, tbl, quad_target(C, ldc, M, N, ep.bias, ep.accumulate), K, tiles_n, band, whole_tiles, parts, items, A.scale, B.scale, ctx->d_status, A.guard, B.guard, A.guard_mask, B.guard_mask, A.line_inv, SimtOperands{A.ptr, A.fp32_stride_mn ? A.fp32_stride_mn : A.stride_mn, A.fp32_stride_k ? A.fp32_stride_k : A.stride_k, B.ptr, B.stride_mn, B.stride_k}, ctx->d_guard ? ctx->d_guard + 1 : nullptr, FUSED ? *ep.fused : FusedEpilogue{});
+  DLB_LAUNCH_KERNEL(ctx, kernel, 2 * min(items, lanes), NUM_THREADS, P::TOTAL, ta, tal, tb, tbl, quad_target(C, ldc, M, N, ep.bias, ep.accumulate), K, tiles_n, band, whole_tiles, parts, items, A.scale, B.scale, ctx->d_status, A.guard, B.guard, A.guard_mask, B.guard_mask, A.line_inv, SimtOperands{A.ptr, A.fp32_stride_mn ? A.fp32_stride_mn : A.stride_mn, A.fp32_stride_k ? A.fp32_stride_k : A.stride_k, B.ptr, B.stride_mn, B.stride_k}, ctx->d_guard ? ctx->d_guard + 1 : nullptr);
   DLB_LAUNCHED(ctx);
   return DLB_OK;
 }
@@ -508,13 +478,8 @@ dlb_status gemm_pair(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, f
   const bool a_mn = !(A.stride_k == 1);
   const bool b_mn = !(B.stride_k == 1);
   const int chunk = gemm_pair_chunk();
-  if (ep.fused && ep.fused->mode != EPI_PLAIN) {
-    // Instantiated for the two layouts that carry one (forward: both operands
-    // K-major; input gradient: weights MN-major) at the default chunk.
-    if (chunk == 8 && !ep.accumulate && !a_mn)
-      return b_mn ? launch_pair<6, 8, false, true, true>(ctx, A, B, C, ldc, M, N, K, ep)
-                  : launch_pair<6, 8, false, false, true>(ctx, A, B, C, ldc, M, N, K, ep);
-    set_error("gemm_pair: no fused epilogue for this layout");
+  if (ep.fused) {
+    set_error("gemm_pair: fused epilogues run on the medium kernel");
     return DLB_ERR_UNSUPPORTED;
   }
 #define DLB_PAIR(CH)                                                                                  \

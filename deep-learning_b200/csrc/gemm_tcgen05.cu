@@ -601,6 +601,13 @@ bool gemm_f16_supported(const GemmOperand &A, const GemmOperand &B, const float 
          operand_ok(nullptr, 2, B.stride_mn, B.stride_k, N, K, gemm_pair_enabled() && (long long)M * N >= 256 * 256);
 }
 
+// 256 x 256 tiles, or 256 x 128 with the k range shared: whichever is done first.
+bool gemm_mid_chosen(const dlb_ctx *ctx, const GemmOperand &B, int M, int N, int K, bool accumulate, int *split_shift) {
+  const double mid_us = gemm_mid_us(ctx, M, N, K, split_shift);
+  const bool ragged = B.stride_k != 1 && N % 64 != 0;  // the pair kernel's 3-d maps want whole columns of 64
+  return ragged || mid_us < gemm_pair_us(ctx, M, N, K, accumulate);
+}
+
 dlb_status gemm_tcgen05(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C,
                         long long ldc, int M, int N, int K, const GemmEpilogue &ep) {
   if (A.h_hi && A.h_lo && B.h_hi && B.h_lo) {
@@ -611,16 +618,13 @@ dlb_status gemm_tcgen05(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B
       return DLB_ERR_UNSUPPORTED;
     }
     if (gemm_pair_enabled() && (long long)M * N >= 256 * 256) {
-      // 256 x 256 tiles, or 256 x 128 with the k range shared: whichever is done first.
       int split_shift = 0;
-      const double mid_us = gemm_mid_us(ctx, M, N, K, &split_shift);
-      const bool ragged = B.stride_k != 1 && N % 64 != 0;  // the pair kernel's 3-d maps want whole columns of 64
-      if (ragged || mid_us < gemm_pair_us(ctx, M, N, K, ep.accumulate || ep.fused))
+      if (gemm_mid_chosen(ctx, B, M, N, K, ep.accumulate, &split_shift) || ep.fused)
         return gemm_mid(ctx, A, B, C, ldc, M, N, K, split_shift, ep);
       return gemm_pair(ctx, A, B, C, ldc, M, N, K, ep);
     }
     if (ep.fused) {
-      set_error("gemm_tcgen05: a fused epilogue runs on the 2-CTA kernel only");
+      set_error("gemm_tcgen05: a fused epilogue runs on the medium kernel only");
       return DLB_ERR_UNSUPPORTED;
     }
     return launch_majors<2>(ctx, A, B, C, ldc, M, N, K, ep);

@@ -16,6 +16,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <map>
 #include <random>
 #include <string>
 #include <thread>
@@ -284,11 +285,13 @@ dlb_status free_batch_buffers(dlb_model *m) {
     float **bufs[] = {&l.Z, &l.A, &l.A_lo, &l.delta, &l.delta_lo, &l.IN, &l.IN_lo, &l.lstm_gin, &l.lstm_grec,
                       &l.lstm_z, &l.lstm_c, &l.lstm_ca, &l.lstm_gi, &l.lstm_gf, &l.lstm_go, &l.lstm_d, &l.lstm_dc};
     planes_rows_exempt(m->ctx, l.delta_lo, 0, false);
+    for (const float *lo : {l.A_lo, l.delta_lo, l.IN_lo}) planes_unused(m->ctx, lo, 0, false);
     for (float **b : bufs) {
       if (*b) DLB_TRY(dlb_free(m->ctx, *b));
       *b = nullptr;
     }
   }
+  planes_unused(m->ctx, m->input_lo, 0, false);
   float **bufs[] = {&m->input, &m->input_lo, &m->target, &m->input_rows, &m->target_rows};
   for (float **b : bufs) {
     if (*b) DLB_TRY(dlb_free(m->ctx, *b));
@@ -391,7 +394,66 @@ dlb_status ensure_batch(dlb_model *m, size_t rows) {
     DLB_TRY(dlb_memset(m->ctx, m->accu_sum, 0, sizeof(double)));
   }
   m->alloc_rows = rows;
+  m->planes_rows = 0;  // new buffers: choose_planes decides again
   return DLB_OK;
+}
+
+// Which tensors of the step some product will read as kept planes at this number of
+// rows; the plane buffers of the others are marked unused, so that no kernel
+// fills them.  Small products and products of widths TMA cannot address split
+// their operands themselves (gemm_direct.cu): their planes cost a pass or two and a
+// check launch per tensor, 96 of the 613 operations of a small classifier's epoch
+// and half a millisecond of four steps of a 1203-wide one.
+void choose_planes(dlb_model *m, size_t rows) {
+  dlb_ctx *ctx = m->ctx;
+  if (m->planes_rows == rows && m->planes_generation == ctx->plane_generation) return;
+  m->planes_rows = rows;
+  m->planes_generation = ctx->plane_generation;
+  const int R = (int)(rows * m->seq_w);
+  std::map<const float *, bool> used;  // plane buffer -> read by a product
+  const float *top = m->input_lo;
+  for (size_t i = 1; i < m->layers.size(); ++i) {
+    LayerRT &l = m->layers[i];
+    if (l.type == DLB_LAYER_RESIDUAL) continue;
+    const float *x = l.group == 1 && !l.block_input ? l.IN_lo : top;
+    const int I = (int)l.fan_in, H = (int)l.units;
+    PlaneUse f{true, true}, d{true, true}, g{true, true};
+    if (!is_lstm(l)) {
+      GemmOperand gd{nullptr, nullptr, 1, H};
+      gd.rescale_lines = class_error(m, i) && m->seq_w == 1;
+      f = gemm_plane_use(ctx, {nullptr, nullptr, I, 1}, {nullptr, nullptr, I, 1}, R, H, I);
+      g = gemm_plane_use(ctx, gd, {nullptr, nullptr, 1, I}, H, I, R);
+      d = i == 1 ? PlaneUse{false, false}
+                 : gemm_plane_use(ctx, {nullptr, nullptr, H, 1}, {nullptr, nullptr, 1, I}, R, I, H);
+    } else {
+      // (its weights and errors have no kept planes; its inputs' and outputs' may be
+      // read by products of any size)
+      used[l.A_lo] = true;
+    }
+    used[x] |= f.a || g.b;
+    used[l.delta_lo] |= d.a || g.a;
+    const bool w = f.b || d.b;
+    if (w && !l.w_planes) m->params_lo_valid = false;
+    l.w_planes = w;
+    if (!is_lstm(l)) planes_unused(ctx, m->params_lo + l.first_conn, l.units * l.fan_in * sizeof(float), !w);
+    if (l.group == 0) {
+      top = l.A_lo;
+    } else if (i + 1 < m->layers.size() && m->layers[i + 1].group == 0) {
+      size_t r = i;
+      while (m->layers[r].type != DLB_LAYER_RESIDUAL) --r;
+      top = m->layers[r].A_lo;
+    }
+  }
+  auto mark = [&](const float *lo, size_t width) {
+    auto it = used.find(lo);
+    if (lo) planes_unused(ctx, lo, m->seq_w * m->alloc_rows * width * sizeof(float), it == used.end() || !it->second);
+  };
+  mark(m->input_lo, n_in(m));
+  for (LayerRT &l : m->layers) {
+    mark(l.A_lo, l.units);
+    mark(l.delta_lo, l.units);
+    mark(l.IN_lo, l.fan_in);
+  }
 }
 
 dlb_brn_unit_arrays unit_arrays(dlb_model *m, LayerRT &l, size_t t) {
@@ -513,7 +575,7 @@ dlb_status refresh_weight_residuals(dlb_model *m) {
   // One plane buffer per layer, so that every weight matrix gets a scale of its own.
   for (size_t i = 1; i < m->layers.size(); ++i) {
     const LayerRT &l = m->layers[i];
-    if (l.type == DLB_LAYER_RESIDUAL) continue;
+    if (l.type == DLB_LAYER_RESIDUAL || !l.w_planes) continue;
     DLB_TRY(dlb_split_planes_2d(m->ctx, m->params + l.first_conn, m->params_lo + l.first_conn, (int)l.units,
                                 (int)l.fan_in));
   }
@@ -1700,6 +1762,7 @@ dlb_status dlb_model_forward_pass_device(dlb_model *m, size_t rows, const float 
   DLB_REQUIRE(m && X_dev && rows > 0, "forward_pass_device");
   DLB_TRY(check_supported(m));
   DLB_TRY(ensure_batch(m, rows));
+  choose_planes(m, rows);
   const size_t n = rows * m->seq_w * n_in(m);
   if (time_stepped(m)) {
     // [rows, T * n_in] -> [T, rows, n_in] with the residual plane in the same pass.
@@ -2295,41 +2358,36 @@ dlb_status dlb_model_update_weights(dlb_model *m, size_t rows, size_t training_s
   // next forward pass then finds the planes ready.  Everything between and
   // after the matrices (recurrent weights, biases, scales, shifts) goes in
   // passes of its own.
-  bool fused = m->ctx->gemm_kind == DLB_GEMM_F16X3 && m->params_lo != nullptr;
-  for (size_t i = 1; fused && i < m->layers.size(); ++i) {
-    const LayerRT &l = m->layers[i];
-    if (l.type != DLB_LAYER_RESIDUAL && ((l.first_conn | (l.units * l.fan_in) | l.last_conn) & 3)) fused = false;
-  }
+  const bool planes_form = m->ctx->gemm_kind == DLB_GEMM_F16X3 && m->params_lo != nullptr;
+  bool all_split = planes_form;  // every matrix whose planes are read has them after this update
   auto segment = [&](size_t at, size_t n, unsigned *amax) -> dlb_status {
     if (n == 0) return DLB_OK;
     return optimizer_step_amax(m->ctx, m->optimizer, &k, m->params + at, m->grads + at, m->m1 + at, m->m2 + at,
                                m->m2hat ? m->m2hat + at : nullptr, wd != 0.f ? m->wd_mask + at : nullptr, n, amax);
   };
-  if (fused) {
-    size_t at = 0;
-    for (size_t i = 1; i < m->layers.size(); ++i) {
-      const LayerRT &l = m->layers[i];
-      if (l.type == DLB_LAYER_RESIDUAL) continue;
-      const size_t nw = l.units * l.fan_in;
-      DLB_TRY(segment(at, l.first_conn - at, nullptr));
-      PlaneJob job;
-      DLB_TRY(planes_open(m->ctx, m->params + l.first_conn, m->params_lo + l.first_conn, nw, (int)l.units,
-                          (int)l.fan_in, true, &job));
-      if (job.fused) {
-        const size_t o = l.first_conn;
-        DLB_TRY(optimizer_step_sink(m->ctx, m->optimizer, &k, m->params + o, m->grads + o, m->m1 + o, m->m2 + o,
-                                    m->m2hat ? m->m2hat + o : nullptr, wd != 0.f ? m->wd_mask + o : nullptr,
-                                    (int)l.units, (int)l.fan_in, job.sink));
-      } else {
-        DLB_TRY(segment(l.first_conn, nw, reinterpret_cast<unsigned *>(job.sink.slot) + 2));
-      }
-      DLB_TRY(planes_close(m->ctx, job));
-      at = l.first_conn + nw;
+  size_t at = 0;
+  for (size_t i = 1; planes_form && i < m->layers.size(); ++i) {
+    const LayerRT &l = m->layers[i];
+    const size_t o = l.first_conn, nw = l.units * l.fan_in;
+    if (l.type == DLB_LAYER_RESIDUAL || !l.w_planes) continue;  // goes with what follows
+    if ((o | nw | l.last_conn) & 3) {
+      all_split = false;  // the next forward pass splits it
+      continue;
     }
-    DLB_TRY(segment(at, m->total_parameters - at, nullptr));
-  } else {
-    DLB_TRY(segment(0, m->total_parameters, nullptr));
+    DLB_TRY(segment(at, o - at, nullptr));
+    PlaneJob job;
+    DLB_TRY(planes_open(m->ctx, m->params + o, m->params_lo + o, nw, (int)l.units, (int)l.fan_in, true, &job));
+    if (job.fused) {
+      DLB_TRY(optimizer_step_sink(m->ctx, m->optimizer, &k, m->params + o, m->grads + o, m->m1 + o, m->m2 + o,
+                                  m->m2hat ? m->m2hat + o : nullptr, wd != 0.f ? m->wd_mask + o : nullptr,
+                                  (int)l.units, (int)l.fan_in, job.sink));
+    } else {
+      DLB_TRY(segment(o, nw, job.active ? reinterpret_cast<unsigned *>(job.sink.slot) + 2 : nullptr));
+    }
+    DLB_TRY(planes_close(m->ctx, job));
+    at = o + nw;
   }
+  DLB_TRY(segment(at, m->total_parameters - at, nullptr));
   // Recurrent weights of every IndRNN layer back into the layer's bounds
   // (Update_Weight_Regularization__Constraint_Recurrent_Weight,
   // v1/ops/constraints/constraint.cpp L:245-289).
@@ -2341,7 +2399,7 @@ dlb_status dlb_model_update_weights(dlb_model *m, size_t rows, size_t training_s
       DLB_TRY(dlb_indrnn_clamp(m->ctx, m->params + l.first_recurrent, (int)l.units, lo, hi));
   }
   m->grads_clean = true;  // the update kernel clears every gradient it consumes
-  m->params_lo_valid = fused;
+  m->params_lo_valid = all_split;
   return DLB_OK;
 }
 

@@ -74,6 +74,7 @@ struct LayerRT {
   // Owner-computes update across ranks: the reduce-scatter of the layer's
   // weight gradient and the gather of its updated weights are behind these.
   cudaEvent_t ev_reduced = nullptr, ev_gathered = nullptr;
+  bool w_planes = true;     // products read the planes of W at the sizes in use
   bool error_final = false; // backward: delta already holds the error w.r.t. Z (the product above formed it)
   size_t norm_units = 0;    // normalised units: width, or fan-in for a block layer
   // Device buffers (allocated by ensure_batch).  Stand-alone FC layer: Z sums,
@@ -179,6 +180,9 @@ struct dlb_model {
   int loss_lag = 0;
   size_t loss_rows = 0;  // rows accumulated since reset_loss
   bool params_lo_valid = false;
+  // What choose_planes last decided for: rows of the batch, operand form, buffers.
+  size_t planes_rows = 0;
+  uint64_t planes_generation = ~(uint64_t)0;
   uint64_t plane_generation = 0;  // the context's value when the weights were last split
   // Inside train_step the step is known to be a single chunk, so each layer's
   // weight gradient is all-reduced as soon as its GEMM has been enqueued.

@@ -231,8 +231,24 @@ static bool rows_exempt_at(const dlb_ctx *ctx, uintptr_t key) {
   return key < it->first + it->second;
 }
 
+void planes_unused(dlb_ctx *ctx, const float *planes, size_t bytes, bool on) {
+  if (!planes) return;
+  const uintptr_t key = reinterpret_cast<uintptr_t>(planes);
+  if (on) ctx->planes_unused[key] = bytes;
+  else ctx->planes_unused.erase(key);
+}
+
+bool planes_unused_at(const dlb_ctx *ctx, const float *planes) {
+  if (ctx->planes_unused.empty()) return false;
+  const uintptr_t key = reinterpret_cast<uintptr_t>(planes);
+  auto it = ctx->planes_unused.upper_bound(key);
+  if (it == ctx->planes_unused.begin()) return false;
+  --it;
+  return key < it->first + it->second;
+}
+
 bool planes_lookup(dlb_ctx *ctx, const float *aux, GemmOperand *o) {
-  if (!aux || ctx->planes.empty()) return false;
+  if (!aux || ctx->planes.empty() || planes_unused_at(ctx, aux)) return false;
   const uintptr_t p = reinterpret_cast<uintptr_t>(aux);
   auto it = ctx->planes.upper_bound(p);
   if (it == ctx->planes.begin()) return false;
@@ -270,6 +286,10 @@ static void sink_lines(PlaneSink &k, unsigned *lines, int rows, int cols, bool e
 dlb_status planes_open(dlb_ctx *ctx, const float *x, float *planes, size_t n, int rows, int cols,
                        bool kernel_can_fuse, PlaneJob *job) {
   DLB_REQUIRE(x && planes && n > 0 && n < ((size_t)1 << 40), "plane buffer: tensor, buffer and size");
+  if (planes_unused_at(ctx, planes)) {
+    *job = PlaneJob{};
+    return DLB_OK;
+  }
   if ((size_t)rows * (size_t)cols != n) rows = cols = 0;
   const uintptr_t key = reinterpret_cast<uintptr_t>(planes);
   planes_forget(ctx, key + 1, n * sizeof(float) - 1);
@@ -414,6 +434,7 @@ dlb_status dlb_split_planes_2d(dlb_ctx *ctx, const float *x, float *planes, int 
   if (ctx->gemm_kind == DLB_GEMM_TF32X3) return dlb_split_tf32(ctx, x, planes, n);
   PlaneJob job;
   DLB_TRY(planes_open(ctx, x, planes, n, rows, cols, true, &job));
+  if (!job.active) return DLB_OK;
   // With a scale predicted from this buffer's previous split one pass does; the
   // first split takes the tensor's maximum first.
   if (job.fused) DLB_TRY(launch_split(ctx, x, n, rows, cols, job.sink));
@@ -427,6 +448,7 @@ dlb_status dlb_split_planes(dlb_ctx *ctx, const float *x, float *planes, size_t 
   if (ctx->gemm_kind == DLB_GEMM_TF32X3) return dlb_split_tf32(ctx, x, planes, n);
   PlaneJob job;
   DLB_TRY(planes_open(ctx, x, planes, n, 0, 0, false, &job));
+  if (!job.active) return DLB_OK;
   DLB_TRY(planes_absmax(ctx, x, n, job.sink.slot));
   return planes_close(ctx, job);
 }

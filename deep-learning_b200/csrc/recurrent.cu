@@ -938,7 +938,7 @@ struct TimePlanes {
     }
     if (rows == 0 || n <= 0 || rows > 0x7fffffffu) return DLB_OK;
     DLB_TRY(planes_open(ctx, x, planes, rows * (size_t)n, (int)rows, n, can_write, &job));
-    amax = reinterpret_cast<unsigned *>(job.sink.slot) + 2;
+    if (job.active) amax = reinterpret_cast<unsigned *>(job.sink.slot) + 2;
     return DLB_OK;
   }
   const PlaneSink *sink() const { return job.active && job.fused ? &job.sink : nullptr; }
