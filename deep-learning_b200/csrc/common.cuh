@@ -414,4 +414,14 @@ constexpr int SCALE_SLOTS = 8192;
 constexpr int SLOT_WORDS = 8;    // words of one scale slot (layout: planes.cuh)
 constexpr int MAX_DEVICES = 64;  // device indices a process may hold contexts on
 
+// All time steps of an LSTM layer in one launch (lstm_walk.cu).  done: whether this
+// was the faster way and has been enqueued; the step entry points otherwise.
+// Backward: dH [T, rows, C] gets the recurrent part added.
+dlb_status lstm_forward_walk(dlb_ctx *ctx, const float *g_in, const float *w_rec, const float *bias, const float *peep,
+                             float *z, float *c, float *ca, float *h, float *gi, float *gf, float *go, int rows, int T,
+                             int blocks, int cells, bool *done);
+dlb_status lstm_backward_walk(dlb_ctx *ctx, float *dH, const float *w_rec, const float *z, const float *ca,
+                              const float *c, const float *gi, const float *gf, const float *go, const float *peep,
+                              float *d, int rows, int T, int blocks, int cells, bool *done);
+
 }  // namespace dlb

@@ -17,12 +17,9 @@
 // gradient vector after the weight gradients.  The gates' sums of a time step
 // are one row of G values in that order; so are the gates' errors.
 #include "common.cuh"
+#include "lstm_cell.cuh"
 
 namespace dlb {
-
-__device__ __forceinline__ float sigmoid_ref(float x) { return 1.f / (1.f + expf(-x)); }
-// The reference's tanh: 2 / (1 + exp(-2 x)) - 1 (v1/ops/activations/functions.hpp L:44).
-__device__ __forceinline__ float tanh_ref(float x) { return 2.f / (1.f + expf(-2.f * x)) - 1.f; }
 
 // dst[r, :] = src[offset[r] ...], rows of `width` floats.
 __global__ void gather_rows_kernel(const float *__restrict__ src, const unsigned long long *__restrict__ offset,

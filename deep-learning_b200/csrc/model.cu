@@ -822,8 +822,8 @@ dlb_status forward_residual_time(dlb_model *m, size_t i, const float *X, const f
 
 // LSTM layer forward (Recurrent__Forward_Pass__LSTM__OpenMP,
 // v1/learner/fwp_rec_mp.cpp L:395-418, L:802-1526): the input sums of all time
-// steps are one product over T * B rows; per time step the recurrent sums are a
-// product over B rows and the cells one kernel.
+// steps are one product over T * B rows; then one launch walks over time, or per time
+// step the recurrent sums are a product over B rows and the cells one kernel.
 dlb_status forward_lstm(dlb_model *m, LayerRT &l, const float *X, const float *X_lo, int B, int T) {
   const int I = (int)l.fan_in, C = (int)l.units, G = (int)lstm_gates(l);
   DLB_TRY(dlb_gather_rows(m->ctx, m->params, l.lstm_map_ff, l.lstm_wff, (size_t)G, I));
@@ -832,7 +832,10 @@ dlb_status forward_lstm(dlb_model *m, LayerRT &l, const float *X, const float *X
   DLB_TRY(dlb_gather_rows(m->ctx, m->params, l.lstm_map_peep, l.lstm_peep, (size_t)3 * C, 1));
   DLB_TRY(dlb_fc_forward(m->ctx, X, X_lo, l.lstm_wff, nullptr, nullptr, l.lstm_gin, T * B, I, G));
   const size_t sc = (size_t)B * C, sb = (size_t)B * l.blocks, sg = (size_t)B * G;
-  for (int t = 0; t < T; ++t) {
+  bool walked = false;
+  DLB_TRY(lstm_forward_walk(m->ctx, l.lstm_gin, l.lstm_wrec, l.lstm_bias, l.lstm_peep, l.lstm_z, l.lstm_c, l.lstm_ca,
+                            l.A, l.lstm_gi, l.lstm_gf, l.lstm_go, B, T, (int)l.blocks, (int)l.cells, &walked));
+  for (int t = 0; t < T && !walked; ++t) {
     if (t > 0)
       DLB_TRY(dlb_fc_forward(m->ctx, l.A + (t - 1) * sc, nullptr, l.lstm_wrec, nullptr, nullptr, l.lstm_grec, B, C, G));
     DLB_TRY(dlb_lstm_forward_step(m->ctx, l.lstm_gin + t * sg, t ? l.lstm_grec : nullptr, l.lstm_bias, l.lstm_peep,
@@ -845,12 +848,16 @@ dlb_status forward_lstm(dlb_model *m, LayerRT &l, const float *X, const float *X
 
 // Backward through time: l.delta holds the error of the layer's outputs from
 // above; per time step, from the last, the recurrent part is added (the gates'
-// errors of t + 1 times R) and the cell kernel forms the gates' errors of t.
+// errors of t + 1 times R) and the cell kernel forms the gates' errors of t, all in
+// one launch where that is faster.
 // Then the error of the layer's inputs is one product over T * B rows.
 dlb_status backward_lstm(dlb_model *m, LayerRT &l, float *below_delta, int B, int T) {
   const int I = (int)l.fan_in, C = (int)l.units, G = (int)lstm_gates(l);
   const size_t sc = (size_t)B * C, sb = (size_t)B * l.blocks, sg = (size_t)B * G;
-  for (int t = T - 1; t >= 0; --t) {
+  bool walked = false;
+  DLB_TRY(lstm_backward_walk(m->ctx, l.delta, l.lstm_wrec, l.lstm_z, l.lstm_ca, l.lstm_c, l.lstm_gi, l.lstm_gf,
+                             l.lstm_go, l.lstm_peep, l.lstm_d, B, T, (int)l.blocks, (int)l.cells, &walked));
+  for (int t = T - 1; t >= 0 && !walked; --t) {
     const bool last = t == T - 1;
     float *dH = l.delta + t * sc;
     if (!last) {
