@@ -80,6 +80,9 @@ struct dlb_ctx {
   // [1] products that therefore ran on the fp32 CUDA-core kernel, [2] tensors
   // split again after outgrowing their predicted scale.
   unsigned long long *d_guard = nullptr;
+  // Two flag words of planes_split_lines, used in turn: a launch clears the next one's.
+  unsigned *line_flags = nullptr;
+  unsigned line_splits = 0;
   std::vector<int> scale_free;
   std::map<uintptr_t, size_t> allocs;  // dlb_malloc'd blocks, to retire plane entries on free
   // Exchange of small fp64 vectors through peer memory: every rank's buffer
@@ -231,15 +234,15 @@ struct GemmOperand {
   // Bits of that word this operand's use in the product cares about: overflow,
   // and the small lines along its free dimension.
   unsigned guard_mask = 7u;
-  // Strides of `ptr` where they differ from the planes' (planes transposed into
-  // scratch for the product); 0: the same.
+  // Strides of `ptr` where they differ from the planes' (planes made in scratch for
+  // the product); 0: the same.
   long long fp32_stride_mn = 0, fp32_stride_k = 0;
-  // Planes with a scale of their own per mn line (k-contiguous planes made for
-  // one product): 1 / scale of every line; `scale` is then not read.
+  // Planes with a scale of their own per mn line (made for one product): 1 / scale of
+  // every line; `scale` is then not read.
   const float *line_inv = nullptr;
   // Asked by the caller: make such planes for this product (A of a weight
   // gradient whose columns differ widely in size, e.g. the classes of a softmax
-  // error).  Also done where TMA cannot tile the operand as it lies.
+  // error).  Also done where the caller kept no planes that TMA can address.
   bool rescale_lines = false;
 };
 // Flag bits (planes.cuh) a product looks at for an operand with these strides
@@ -255,7 +258,7 @@ struct GemmEpilogue {
   float *colsum = nullptr;       // per-n sum over m of C (db), written/accumulated
   int accumulate = 0;            // C += result
   // Work of the kernel that would follow the product, done on the tile while the
-  // drain warps hold it (2-CTA fp16-plane kernel only: ask gemm_fused_supported).
+  // drain warps hold it (the medium fp16-plane kernel only: ask gemm_fused_supported).
   const FusedEpilogue *fused = nullptr;
 };
 
@@ -269,7 +272,11 @@ dlb_status gemm_direct(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B,
 bool gemm_direct_supported(const GemmOperand &A, const GemmOperand &B);
 // Whether a product on planes runs on gemm_mid_kernel, and into how many pieces
 // (1 << split_shift) its k range is cut there.
-bool gemm_mid_chosen(const dlb_ctx *ctx, const GemmOperand &B, int M, int N, int K, bool accumulate, int *split_shift);
+bool gemm_mid_chosen(const dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K,
+                     bool accumulate, int *split_shift);
+// About how long a product on planes takes.
+double gemm_planes_us(const dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K,
+                      bool accumulate);
 double gemm_direct_us(const dlb_ctx *ctx, int M, int N, int K);  // about how long it takes
 // Returns DLB_ERR_UNSUPPORTED (without touching C) when the shape or alignment
 // is outside what the TMA descriptors can express.
@@ -322,11 +329,10 @@ struct PlaneUse {
   bool a, b;
 };
 PlaneUse gemm_plane_use(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K);
-// x [K, M] with row pitch `pitch` (mn contiguous) -> fp16 planes [M, kp] (k
-// contiguous), line m scaled by a power of two of its own taken from the
-// line's largest |x| (`cmax`, M words of scratch); line_inv[m] = 1 / scale.
-dlb_status planes_transpose_scaled(dlb_ctx *ctx, const float *x, long long pitch, int K, int M, uint16_t *hi_t,
-                                   uint16_t *lo_t, long long kp, unsigned *cmax, float *line_inv);
+// Planes of one or both operands (the other null) made in scratch for this product,
+// with a scale per line along the free dimension; fills in the operand's plane fields
+// and strides.
+dlb_status planes_split_lines(dlb_ctx *ctx, GemmOperand *A, int M, GemmOperand *B, int N, int K);
 // Drops the plane buffers registered at addresses in [base, base + bytes).
 void planes_forget(dlb_ctx *ctx, uintptr_t base, size_t bytes);
 
@@ -400,10 +406,6 @@ dlb_status planes_open(dlb_ctx *ctx, const float *x, float *planes, size_t n, in
 dlb_status planes_close(dlb_ctx *ctx, const PlaneJob &job);
 // max |x| of a tensor no kernel of the library produced (inputs, fresh weights).
 dlb_status planes_absmax(dlb_ctx *ctx, const float *x, size_t n, float *slot);
-// Split into caller storage outside the registry (scratch): planes, slot of
-// SLOT_WORDS words and rows + cols words of line maxima, all zeroed here.
-dlb_status planes_split_adhoc(dlb_ctx *ctx, const float *x, size_t n, int rows, int cols, uint16_t *hi,
-                              uint16_t *lo, float *slot, unsigned *lines);
 dlb_status optimizer_step_amax(dlb_ctx *ctx, int rule, const dlb_optimizer_scalars *s, float *p, float *g,
                                float *first, float *second, float *second_hat, const float *wd_mask, size_t n,
                                unsigned *amax);

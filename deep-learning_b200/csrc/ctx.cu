@@ -97,28 +97,42 @@ bool gemm_fused_supported(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand 
   if (!(ctx->use_tensor_core && ctx->tensor_core_ok && big && ctx->gemm_kind == DLB_GEMM_F16X3)) return false;
   int split_shift;
   if (!gemm_pair_enabled() || gemm_pair_chunk() != 8 || A.stride_k != 1 || ldc != N ||
-      !gemm_mid_chosen(ctx, B, M, N, K, false, &split_shift))
+      !gemm_mid_chosen(ctx, A, B, M, N, K, false, &split_shift))
     return false;
   if (!gemm_f16_supported(A, B, C, ldc, M, N, K)) return false;
   GemmOperand a = A, b = B;
   return (a.h_hi || planes_lookup(ctx, a.lo, &a)) && (b.h_hi || planes_lookup(ctx, b.lo, &b));
 }
 
-// A product with both operands' planes kept runs on them where the output fills a
-// 256 x 256 tile and TMA can address them.
+// Outputs that fill a 256 x 256 tile can run on fp16 planes.
 static bool plane_size(int M, int N, int K) { return (long long)M * N >= 256 * 256 && K >= 32; }
-// About how long a product on kept planes takes.
-static double planes_us(int M, int N, int K) { return 2.0 * M * N * K / 4.5e8; }
-// Planes of A made for the product, transposed, instead of splitting in the product.
-static bool transposed_better(const dlb_ctx *ctx, int M, int N, int K) {
-  return gemm_direct_us(ctx, M, N, K) > planes_us(M, N, K) + 45.0;
+// About how long the making of planes for one product takes.
+static double split_us(long long elements) { return 3.0 + (double)elements / 0.7e6; }
+
+// Whether the product runs on planes, given which operands' are kept: by the shorter
+// of that, with the missing ones made for it, and the direct kernel.
+static bool planes_better(const dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K,
+                          bool accumulate, bool have_a, bool have_b) {
+  if (have_a && have_b) return true;
+  if (!gemm_pair_enabled() || (A.stride_k != 1 && B.stride_k == 1)) return false;
+  const long long fresh = (have_a ? 0 : (long long)M * K) + (have_b ? 0 : (long long)N * K);
+  return gemm_planes_us(ctx, A, B, M, N, K, accumulate) + split_us(fresh) < gemm_direct_us(ctx, M, N, K);
+}
+// Whether kept planes serve: TMA takes their pitch and the caller asks for no scale per
+// line.  An mn-contiguous A (the error of a weight gradient) whose rows are no whole
+// 128-byte columns of halves is taken for one over classes and gets those scales too.
+static bool planes_serve(const GemmOperand &o, int mn, int k, bool is_a) {
+  if (o.rescale_lines) return false;
+  if (o.stride_k == 1) return o.stride_mn % 8 == 0 && o.stride_mn >= k;
+  return o.stride_mn == 1 && o.stride_k % 8 == 0 && o.stride_k >= mn && !(is_a && mn % 64 != 0);
 }
 
 PlaneUse gemm_plane_use(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K) {
   if (ctx->gemm_kind != DLB_GEMM_F16X3) return {true, true};
   if (!plane_size(M, N, K)) return {false, false};
-  if (gemm_f16_supported(A, B, nullptr, N, M, N, K) && !A.rescale_lines) return {true, true};
-  return {false, A.stride_k != 1 && B.stride_k != 1 && gemm_pair_enabled() && transposed_better(ctx, M, N, K)};
+  const bool a = planes_serve(A, M, K, true), b = planes_serve(B, N, K, false);
+  const bool on = planes_better(ctx, A, B, M, N, K, false, a, b);
+  return {on && a, on && b};
 }
 
 dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, float *C,
@@ -133,117 +147,30 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
   const bool big = ((long long)M * N >= 128 * 64 && K >= 32) || ctx->gemm_kind == DLB_GEMM_F16X3;
   if (!(ctx->use_tensor_core && ctx->tensor_core_ok && big)) return gemm_simt(ctx, A, B, C, ldc, M, N, K, ep);
 
-  // The fp16 form either reads operands split beforehand (plane_product) or splits
-  // them in the product (gemm_direct).  Planes that the caller keeps are used
-  // wherever TMA can address them and the output fills a 256 x 256 tile.  Below
-  // that, and for every other pitch and width, the direct kernel runs.  Where
-  // planes would have to be made for this call the shorter of the two wins: the
-  // direct kernel takes about 8 us and 2.6 us per round of 64-deep chunks (one
-  // 128 x 128 tile per SM), the product on fresh planes about 55 us (absolute
-  // maxima, split and check of two operands; 45 us when one is transposed) and
-  // 450 TFLOP/s (1024^3: 30 us against 67, 2048^3: 188 against 95).
-  const bool direct_form = ctx->gemm_kind == DLB_GEMM_F16X3 && !ep.fused && gemm_direct_supported(A, B);
-  auto direct = [&]() -> dlb_status {
-    ProfileSpan span;
-    DLB_TRY(span.begin(ctx, 0, 2.0 * M * N * K));
-    DLB_TRY(gemm_direct(ctx, A_in, B_in, C, ldc, M, N, K, ep));
-    return span.end();
-  };
-
-  // A weight-gradient product (both operands mn-contiguous) whose A TMA cannot
-  // tile as it lies (output rows not a multiple of 64, e.g. 1000 classes), or
-  // whose caller asked for a scale per output row (the classes of a softmax
-  // error differ by many orders of magnitude: the ones nobody is wrong about
-  // have errors 2^-20 and less of the others', and one scale for the tensor
-  // would leave their gradient rows with few bits).  A's planes are made for
-  // this product in scratch: k contiguous, every line with the scale of its own
-  // maximum (two passes over the fp32 tensor, 12 bytes per element), and the
-  // product runs on the 2-CTA kernel in the k-contiguous x mn-contiguous form,
-  // each output row multiplied by its line's 1 / scale.  Nothing of A is left
-  // for the range guard to flag.
-  if (ctx->gemm_kind == DLB_GEMM_F16X3 && A.stride_mn == 1 && A.stride_k != 1 && B.stride_mn == 1 &&
-      B.stride_k != 1 && gemm_pair_enabled() && plane_size(M, N, K) && !ep.fused &&
-      (A.rescale_lines || !gemm_f16_supported(A, B, C, ldc, M, N, K)) &&
-      (!direct_form || transposed_better(ctx, M, N, K))) {
-    GemmOperand a = A, b = B;
-    const bool have_b = b.h_hi || planes_lookup(ctx, b.lo, &b);
-    const long long kp = (long long)align_up((size_t)K, 8);
-    if (have_b && a.stride_k >= M) {
-      const size_t plane = align_up((size_t)M * kp, 64);
-      void *scr = nullptr;
-      DLB_TRY(scratch(ctx, 2 * plane * sizeof(uint16_t) + 2 * (size_t)M * sizeof(float), &scr));
-      uint16_t *hi_t = static_cast<uint16_t *>(scr), *lo_t = hi_t + plane;
-      unsigned *cmax = reinterpret_cast<unsigned *>(lo_t + plane);
-      float *line_inv = reinterpret_cast<float *>(cmax + M);
-      a.fp32_stride_mn = a.stride_mn;
-      a.fp32_stride_k = a.stride_k;
-      a.h_hi = hi_t;
-      a.h_lo = lo_t;
-      a.stride_mn = kp;
-      a.stride_k = 1;
-      a.scale = line_inv;  // not read
-      a.line_inv = line_inv;
-      a.guard = nullptr;
-      if (gemm_f16_supported(a, b, C, ldc, M, N, K)) {
-        DLB_TRY(planes_transpose_scaled(ctx, A.ptr, A.stride_k, K, M, hi_t, lo_t, kp, cmax, line_inv));
-        A = a;
-        B = b;
-      }
+  // The fp16 form runs on planes or splits its operands in the product (gemm_direct).
+  // Planes that the caller keeps are used wherever TMA can address them and the output
+  // fills a 256 x 256 tile.  Missing ones are made for this product, with a scale per
+  // line, where that and the product on planes are estimated to be shorter than the
+  // direct kernel, which reads any pitch and width (1024 x 1000 x 2048: 54 us against 6 and
+  // 17; 333 x 1203 x 1203: 24.8 against 21; 333 x 617 x 1203: 18 the direct way).  An operand
+  // whose caller asks for a scale per line (the classes of a softmax error differ by
+  // many orders of magnitude: the ones nobody is wrong about have errors 2^-20 and
+  // less of the others', and one scale for the tensor would leave their gradient
+  // rows with few bits) always gets planes of its own.
+  if (ctx->gemm_kind == DLB_GEMM_F16X3 && gemm_direct_supported(A, B)) {
+    bool have_a = false, have_b = false;
+    if (plane_size(M, N, K)) {
+      have_a = A.h_hi || (planes_serve(A, M, K, true) && planes_lookup(ctx, A.lo, &A));
+      have_b = B.h_hi || (planes_serve(B, N, K, false) && planes_lookup(ctx, B.lo, &B));
     }
-  }
-
-  if (direct_form && A.h_hi == nullptr) {  // (A.h_hi: planes just made for this product)
-    if (!plane_size(M, N, K) || !gemm_f16_supported(A, B, C, ldc, M, N, K) || A.rescale_lines) return direct();
-    GemmOperand a = A, b = B;
-    const bool have = planes_lookup(ctx, a.lo, &a) && planes_lookup(ctx, b.lo, &b);
-    if (!have && gemm_direct_us(ctx, M, N, K) <= planes_us(M, N, K) + 55.0) return direct();
-  }
-
-  if (ctx->gemm_kind == DLB_GEMM_F16X3 && gemm_f16_supported(A, B, C, ldc, M, N, K)) {
-    // fp16 planes: the caller's registered plane buffers, or planes derived
-    // into scratch for this call.
-    const bool a_have = A.h_hi || planes_lookup(ctx, A.lo, &A);
-    const bool b_have = B.h_hi || planes_lookup(ctx, B.lo, &B);
-    const size_t a_n = a_have ? 0 : align_up(operand_elems(A, M, K), 64);
-    const size_t b_n = b_have ? 0 : align_up(operand_elems(B, N, K), 64);
-    if (a_n + b_n) {
-      // Behind the planes: two scale slots, then the line maxima of the dense
-      // operands ([M + K] and [N + K] words).
-      const size_t line_words = align_up((size_t)M + K, 4) + align_up((size_t)N + K, 4);
-      void *scr = nullptr;
-      DLB_TRY(scratch(ctx, (a_n + b_n) * 2 * sizeof(uint16_t) + (2 * SLOT_WORDS + line_words) * 4 + 64, &scr));
-      uint16_t *h = static_cast<uint16_t *>(scr);
-      float *slots = reinterpret_cast<float *>(h + 2 * (a_n + b_n));
-      unsigned *lines = reinterpret_cast<unsigned *>(slots + 2 * SLOT_WORDS);
-      // A dense operand is a [mn, k] (k contiguous) or [k, mn] (mn contiguous) matrix.
-      auto shape = [](const GemmOperand &o, int mn, int k, int *rows, int *cols) {
-        *rows = *cols = 0;
-        if (o.stride_k == 1 && o.stride_mn == k) { *rows = mn; *cols = k; }
-        else if (o.stride_mn == 1 && o.stride_k == mn) { *rows = k; *cols = mn; }
-      };
-      if (!a_have) {
-        int r, c;
-        shape(A, M, K, &r, &c);
-        DLB_TRY(planes_split_adhoc(ctx, A.ptr, operand_elems(A, M, K), r, c, h, h + a_n, slots, lines));
-        A.h_hi = h;
-        A.h_lo = h + a_n;
-        A.scale = slots;
-        A.guard = reinterpret_cast<const unsigned *>(slots) + 3;
-        A.guard_mask = guard_mask_of(A);
-      }
-      if (!b_have) {
-        uint16_t *hb = h + 2 * a_n;
-        int r, c;
-        shape(B, N, K, &r, &c);
-        DLB_TRY(planes_split_adhoc(ctx, B.ptr, operand_elems(B, N, K), r, c, hb, hb + b_n, slots + SLOT_WORDS,
-                                   lines + align_up((size_t)M + K, 4)));
-        B.h_hi = hb;
-        B.h_lo = hb + b_n;
-        B.scale = slots + SLOT_WORDS;
-        B.guard = reinterpret_cast<const unsigned *>(slots + SLOT_WORDS) + 3;
-        B.guard_mask = guard_mask_of(B);
-      }
+    if (!plane_size(M, N, K) || !planes_better(ctx, A, B, M, N, K, ep.accumulate, have_a, have_b)) {
+      ProfileSpan span;
+      DLB_TRY(span.begin(ctx, 0, 2.0 * M * N * K));
+      DLB_TRY(gemm_direct(ctx, A_in, B_in, C, ldc, M, N, K, ep));
+      return span.end();
     }
+    if (!have_a || !have_b)
+      DLB_TRY(planes_split_lines(ctx, have_a ? nullptr : &A, M, have_b ? nullptr : &B, N, K));
     // A product with an operand the range guard flagged is computed by the
     // same launch on the CUDA cores, from the fp32 tensors.
     return gemm_tensor_core(ctx, A, B, C, ldc, M, N, K, ep);
@@ -450,6 +377,7 @@ dlb_status dlb_ctx_destroy(dlb_ctx *ctx) {
   planes_forget(ctx, 0, ~(size_t)0);
   if (ctx->scale_pool) cudaFree(ctx->scale_pool);
   if (ctx->d_guard) cudaFree(ctx->d_guard);
+  if (ctx->line_flags) cudaFree(ctx->line_flags);
   if (ctx->timer_start) cudaEventDestroy(ctx->timer_start);
   if (ctx->timer_stop) cudaEventDestroy(ctx->timer_stop);
   for (auto &r : ctx->gemm_records) {

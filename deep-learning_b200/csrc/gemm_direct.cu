@@ -480,7 +480,7 @@ double gemm_direct_us(const dlb_ctx *ctx, int M, int N, int K) {
   const int shift = direct_split_shift(ctx, M, N, K);
   const long long ctas = (long long)ceil_div(M, DM) * ceil_div(N, DN) << shift;
   const long long rounds = (ctas + ctx->sm_count - 1) / ctx->sm_count;
-  return 8.0 + 2.6 * (double)rounds * ceil_div(ceil_div(K, DK), 1 << shift);
+  return 7.5 + 3.0 * (double)rounds * ceil_div(ceil_div(K, DK), 1 << shift);
 }
 
 bool gemm_direct_supported(const GemmOperand &A, const GemmOperand &B) {

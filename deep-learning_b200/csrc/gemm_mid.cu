@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   } else {
     // ---------------- drain: warps 2..9 of every CTA ----------------
     const int q = warp & 3, h = (warp - 2) >> 2;
-    const float out_b = 1.f / __ldg(a.scale_b);
+    const float out_b = a.t.col_factor ? 1.f : 1.f / __ldg(a.scale_b);
     const int row = q * 32 + lane;
     const float out_a = a.line_inv_a ? __ldg(a.line_inv_a + min(m0 + row, a.t.M - 1)) : 1.f / __ldg(a.scale_a);
     const uint32_t lead_acc_empty0 = map_to_cta(acc_empty0, lead);
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     // Warp w takes units w, w + 10, ... of 32 quads each; a lane keeps its columns.
     const int quad0 = (warp * 32 + lane) & ((1 << quads_shift) - 1);
     const int col = n0 + (piece << width_shift) + quad0 * 4;
-    const float4 b4 = quad_bias(a.t, col);
+    const float4 b4 = quad_bias(a.t, col), f4 = quad_factor(a.t, col);
     const bool live = col < a.t.N;
     const bool plain = !FUSED && a.t.quads && !a.t.accumulate;
     const float plane_scale = FUSED && fe.sink.hi ? sink_scale(fe.sink) : 1.f;
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                 v[i].x += w.x, v[i].y += w.y, v[i].z += w.z, v[i].w += w.w;
               }
             }
-            v[i].x += b4.x, v[i].y += b4.y, v[i].z += b4.z, v[i].w += b4.w;
+            v[i] = quad_scaled(v[i], f4, b4);
           }
         }
 #pragma unroll
@@ -388,10 +388,9 @@ dlb_status launch_mid_shift(dlb_ctx *ctx, const GemmOperand &A, const GemmOperan
     attr_set[ctx->device] = true;
   }
   const int tiles_n = ceil_div(N, QN), tiles = tiles_n * ceil_div(M, QM);
-  const MidArgs args{quad_target(C, ldc, M, N, ep.bias, ep.accumulate), K, tiles_n, A.scale, B.scale,
+  const MidArgs args{quad_target(C, ldc, M, N, ep.bias, ep.accumulate, B.line_inv), K, tiles_n, A.scale, B.scale,
                      A.line_inv, A.guard, B.guard, A.guard_mask, B.guard_mask,
-                     SimtOperands{A.ptr, A.fp32_stride_mn ? A.fp32_stride_mn : A.stride_mn,
-                                  A.fp32_stride_k ? A.fp32_stride_k : A.stride_k, B.ptr, B.stride_mn, B.stride_k},
+                     fp32_operands(A, B),
                      ctx->d_guard ? ctx->d_guard + 1 : nullptr, ctx->d_status};
   DLB_CUDA(launch_kernel_cluster(ctx, kernel, dim3((unsigned)(tiles << (SHIFT + 1))), dim3(NUM_THREADS), Q_SMEM,
                                  2u << SHIFT, ta, tal, tb, tbl, args, FUSED ? *ep.fused : FusedEpilogue{}));

@@ -257,7 +257,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     const int h = (warp - 2) >> 2;
     constexpr int HALF = PN / 2;
     float4 *tile = reinterpret_cast<float4 *>(smem + P::EPI_OFFSET) + (warp - 2) * 32 * 8;
-    const float out_b = 1.f / __ldg(scale_b);
+    const float out_b = target.col_factor ? 1.f : 1.f / __ldg(scale_b);
     const float tensor_out_a = line_inv_a ? 1.f : 1.f / __ldg(scale_a);
     const uint32_t lead_acc_empty0 = map_to_cta(acc_empty0, 0);
     float acc[HALF];
@@ -308,15 +308,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
               make_float4(acc[j * 32 + 4 * c] * out_a * out_b, acc[j * 32 + 4 * c + 1] * out_a * out_b,
                           acc[j * 32 + 4 * c + 2] * out_a * out_b, acc[j * 32 + 4 * c + 3] * out_a * out_b);
         __syncwarp();
-        const float4 b4 = quad_bias(t, col);
+        const float4 b4 = quad_bias(t, col), f4 = quad_factor(t, col);
         const bool live = col < target.N;
         if (live) {
           float4 x[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const int r = r8 + 4 * i;
-            x[i] = tile[r * 8 + (cs ^ (r & 7))];
-            x[i].x += b4.x, x[i].y += b4.y, x[i].z += b4.z, x[i].w += b4.w;
+            x[i] = quad_scaled(tile[r * 8 + (cs ^ (r & 7))], f4, b4);
           }
           if (plain) {
 #pragma unroll
@@ -438,7 +437,7 @@ dlb_status launch_pair(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B,
                                (size_t)(N - first_col) * sizeof(float), (size_t)(M - first_row), ctx->stream));
   }
   const int items = whole_tiles + parts * split_tiles;
-  DLB_LAUNCH_KERNEL(ctx, kernel, 2 * min(items, lanes), NUM_THREADS, P::TOTAL, ta, tal, tb, tbl, quad_target(C, ldc, M, N, ep.bias, ep.accumulate), K, tiles_n, band, whole_tiles, parts, items, A.scale, B.scale, ctx->d_status, A.guard, B.guard, A.guard_mask, B.guard_mask, A.line_inv, SimtOperands{A.ptr, A.fp32_stride_mn ? A.fp32_stride_mn : A.stride_mn, A.fp32_stride_k ? A.fp32_stride_k : A.stride_k, B.ptr, B.stride_mn, B.stride_k}, ctx->d_guard ? ctx->d_guard + 1 : nullptr);
+  DLB_LAUNCH_KERNEL(ctx, kernel, 2 * min(items, lanes), NUM_THREADS, P::TOTAL, ta, tal, tb, tbl, quad_target(C, ldc, M, N, ep.bias, ep.accumulate, B.line_inv), K, tiles_n, band, whole_tiles, parts, items, A.scale, B.scale, ctx->d_status, A.guard, B.guard, A.guard_mask, B.guard_mask, A.line_inv, fp32_operands(A, B), ctx->d_guard ? ctx->d_guard + 1 : nullptr);
   DLB_LAUNCHED(ctx);
   return DLB_OK;
 }

@@ -22,6 +22,13 @@ struct SimtOperands {
   const float *B;
   long long b_sn, b_sk;
 };
+// The fp32 tensors of a product that runs on planes, with their own strides.
+inline SimtOperands fp32_operands(const GemmOperand &A, const GemmOperand &B) {
+  return SimtOperands{A.ptr, A.fp32_stride_mn ? A.fp32_stride_mn : A.stride_mn,
+                      A.fp32_stride_k ? A.fp32_stride_k : A.stride_k,
+                      B.ptr, B.fp32_stride_mn ? B.fp32_stride_mn : B.stride_mn,
+                      B.fp32_stride_k ? B.fp32_stride_k : B.stride_k};
+}
 
 // `shared` holds SIMT_SMEM_FLOATS floats.  first_tile / tile_stride: the block's
 // share of the tiles.  fe: the fused epilogue of the launch, or null.

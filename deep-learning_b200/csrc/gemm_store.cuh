@@ -23,21 +23,32 @@ struct QuadTarget {
   int accumulate;     // C += value
   int atomic;         // C += value from more than one CTA
   int quads;          // rows of C and N allow 16-byte accesses
+  const float *col_factor;  // every column times this first (1 / scale of B's lines), or null
 };
 inline bool quad_aligned(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-inline QuadTarget quad_target(float *C, long long ldc, int M, int N, const float *bias, int accumulate) {
-  return QuadTarget{C, ldc, M, N, bias, accumulate, 0, (quad_aligned(C) && (ldc & 3) == 0 && (N & 3) == 0) ? 1 : 0};
+inline QuadTarget quad_target(float *C, long long ldc, int M, int N, const float *bias, int accumulate,
+                              const float *col_factor) {
+  return QuadTarget{C, ldc, M, N, bias, accumulate, 0, (quad_aligned(C) && (ldc & 3) == 0 && (N & 3) == 0) ? 1 : 0,
+                    col_factor};
 }
 
-__device__ __forceinline__ float4 quad_bias(const QuadTarget &t, int col) {
-  float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (t.bias) {
-    if (col < t.N) b.x = __ldg(t.bias + col);
-    if (col + 1 < t.N) b.y = __ldg(t.bias + col + 1);
-    if (col + 2 < t.N) b.z = __ldg(t.bias + col + 2);
-    if (col + 3 < t.N) b.w = __ldg(t.bias + col + 3);
+__device__ __forceinline__ float4 quad_of(const float *p, int N, int col, float otherwise) {
+  float4 b = make_float4(otherwise, otherwise, otherwise, otherwise);
+  if (p) {
+    if (col < N) b.x = __ldg(p + col);
+    if (col + 1 < N) b.y = __ldg(p + col + 1);
+    if (col + 2 < N) b.z = __ldg(p + col + 2);
+    if (col + 3 < N) b.w = __ldg(p + col + 3);
   }
   return b;
+}
+__device__ __forceinline__ float4 quad_bias(const QuadTarget &t, int col) { return quad_of(t.bias, t.N, col, 0.f); }
+__device__ __forceinline__ float4 quad_factor(const QuadTarget &t, int col) {
+  return quad_of(t.col_factor, t.N, col, 1.f);
+}
+// v f + b, f a power of two (so that the product is exact).
+__device__ __forceinline__ float4 quad_scaled(float4 v, float4 f, float4 b) {
+  return make_float4(fmaf(v.x, f.x, b.x), fmaf(v.y, f.y, b.y), fmaf(v.z, f.z, b.z), fmaf(v.w, f.w, b.w));
 }
 
 // One quad of a row inside the output, columns col .. col + 3 (col < N).

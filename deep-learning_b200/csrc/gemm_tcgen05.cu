@@ -537,7 +537,7 @@ dlb_status launch(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, floa
                                (size_t)N * sizeof(float), (size_t)(M - first_row), ctx->stream));
   }
   const int items = whole_tiles + 2 * split_tiles;
-  DLB_LAUNCH_KERNEL(ctx, kernel, min(items, lanes), NUM_THREADS, P::TOTAL, ta, tal, tb, tbl, C, ldc, M, N, K, ep.bias, ep.accumulate, tiles_n, whole_tiles, items, A.scale, B.scale, ctx->d_status, ES == 2 ? A.guard : nullptr, ES == 2 ? B.guard : nullptr, A.guard_mask, B.guard_mask, SimtOperands{A.ptr, A.fp32_stride_mn ? A.fp32_stride_mn : A.stride_mn, A.fp32_stride_k ? A.fp32_stride_k : A.stride_k, B.ptr, B.stride_mn, B.stride_k}, ctx->d_guard ? ctx->d_guard + 1 : nullptr);
+  DLB_LAUNCH_KERNEL(ctx, kernel, min(items, lanes), NUM_THREADS, P::TOTAL, ta, tal, tb, tbl, C, ldc, M, N, K, ep.bias, ep.accumulate, tiles_n, whole_tiles, items, A.scale, B.scale, ctx->d_status, ES == 2 ? A.guard : nullptr, ES == 2 ? B.guard : nullptr, A.guard_mask, B.guard_mask, fp32_operands(A, B), ctx->d_guard ? ctx->d_guard + 1 : nullptr);
   DLB_LAUNCHED(ctx);
   return DLB_OK;
 }
@@ -591,21 +591,29 @@ bool gemm_tcgen05_supported(const GemmOperand &A, const GemmOperand &B, const fl
 }
 
 // The fp16-plane form: planes have the strides of their tensor, so the test is
-// on the strides alone (the planes' own base alignment is checked at launch).  An
-// MN-major B of any extent runs on gemm_mid_kernel; an MN-major A does not have to:
-// weight gradients whose output rows are no multiple of 64 get planes of their own
-// or none (gemm() in ctx.cu).
+// on the strides alone (the planes' own base alignment is checked at launch).
+// MN-major operands of any extent run on gemm_mid_kernel.
 bool gemm_f16_supported(const GemmOperand &A, const GemmOperand &B, const float *C, long long ldc,
                         int M, int N, int K) {
-  return shape_ok(A, B, C, ldc, M, N, K) && operand_ok(nullptr, 2, A.stride_mn, A.stride_k, M, K) &&
-         operand_ok(nullptr, 2, B.stride_mn, B.stride_k, N, K, gemm_pair_enabled() && (long long)M * N >= 256 * 256);
+  const bool any = gemm_pair_enabled() && (long long)M * N >= 256 * 256;
+  return shape_ok(A, B, C, ldc, M, N, K) && operand_ok(nullptr, 2, A.stride_mn, A.stride_k, M, K, any) &&
+         operand_ok(nullptr, 2, B.stride_mn, B.stride_k, N, K, any);
 }
 
 // 256 x 256 tiles, or 256 x 128 with the k range shared: whichever is done first.
-bool gemm_mid_chosen(const dlb_ctx *ctx, const GemmOperand &B, int M, int N, int K, bool accumulate, int *split_shift) {
+bool gemm_mid_chosen(const dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K,
+                     bool accumulate, int *split_shift) {
   const double mid_us = gemm_mid_us(ctx, M, N, K, split_shift);
-  const bool ragged = B.stride_k != 1 && N % 64 != 0;  // the pair kernel's 3-d maps want whole columns of 64
+  // The pair kernel's 3-d maps want whole columns of 64.
+  const bool ragged = (A.stride_k != 1 && M % 64 != 0) || (B.stride_k != 1 && N % 64 != 0);
   return ragged || mid_us < gemm_pair_us(ctx, M, N, K, accumulate);
+}
+
+double gemm_planes_us(const dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K,
+                      bool accumulate) {
+  int shift;
+  return gemm_mid_chosen(ctx, A, B, M, N, K, accumulate, &shift) ? gemm_mid_us(ctx, M, N, K, &shift)
+                                                                 : gemm_pair_us(ctx, M, N, K, accumulate);
 }
 
 dlb_status gemm_tcgen05(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C,
@@ -619,7 +627,7 @@ dlb_status gemm_tcgen05(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B
     }
     if (gemm_pair_enabled() && (long long)M * N >= 256 * 256) {
       int split_shift = 0;
-      if (gemm_mid_chosen(ctx, B, M, N, K, ep.accumulate, &split_shift) || ep.fused)
+      if (gemm_mid_chosen(ctx, A, B, M, N, K, ep.accumulate, &split_shift) || ep.fused)
         return gemm_mid(ctx, A, B, C, ldc, M, N, K, split_shift, ep);
       return gemm_pair(ctx, A, B, C, ldc, M, N, K, ep);
     }

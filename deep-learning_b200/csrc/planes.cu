@@ -12,6 +12,7 @@
 
 #include "common.cuh"
 #include "planes.cuh"
+#include "tc_pair.cuh"
 
 namespace dlb {
 
@@ -95,50 +96,160 @@ __global__ void __launch_bounds__(32 * SPLIT_LANES_Y)
   track.finish(k, shared, tx, ty, SPLIT_LANES_Y, blockIdx.x * 128, cols, live);
 }
 
-// Largest |x| of every column of x [K, M]: blocks of 32 columns x 8 row lanes
-// over a slab of rows, one atomic per column and block.
-__global__ void column_absmax_kernel(const float *__restrict__ x, long long pitch, int K, int M, int rows_per_block,
-                                     unsigned *__restrict__ cmax) {
-  pdl_enter();
-  __shared__ unsigned fold[8][32];
-  const int m = blockIdx.x * 32 + threadIdx.x;
-  const int k0 = blockIdx.y * rows_per_block, k1 = min(K, k0 + rows_per_block);
-  unsigned v = 0u;
-  if (m < M)
-    for (int k = k0 + threadIdx.y; k < k1; k += 8) v = max(v, abs_bits(x[(long long)k * pitch + m]));
-  fold[threadIdx.y][threadIdx.x] = v;
-  __syncthreads();
-  if (threadIdx.y == 0 && m < M) {
+// Planes made for one product, of up to two operands in one launch, every line along
+// the free dimension with the scale of its own maximum (so no line is small for its
+// scale and the range guard has only infinities and NaN to flag).
+//
+// A line that is contiguous belongs to a warp: 1024 elements stay in its registers
+// between the maximum and the split, the rest is read again.  Lines across the
+// memory's rows (the mn-contiguous operands of the backward products) belong to a
+// cluster: 64 columns, each CTA an eighth of the rows, the column maxima folded over
+// the CTAs through their shared memory.  So every element comes from memory once
+// and the second reading from L1.  Bound by memory latency at the sizes of the
+// products that take it: 6 - 8 us for 3 M elements (24 MB, 3.5 TB/s) in L2, where a
+// maximum, a split and a check per operand took 40.
+constexpr int LS_THREADS = 256, LS_KEEP = 8, LS_COLS = 64, LS_CLUSTER = 8;
+// Bits of 2^100.  Larger lines, infinities and NaN go to the fp32 path: the sums times
+// such a line's 1 / scale would leave the range before the other factor brings them back.
+constexpr unsigned LS_HUGE = (127u + 100u) << 23;
+
+struct LineSplit {
+  const float *x;
+  long long pitch;      // of the rows in memory
+  int rows, cols;       // in memory
+  int by_columns;       // lines are columns
+  int vec;              // rows allow 16-byte loads
+  uint16_t *hi, *lo;
+  long long out_pitch;  // of the planes' rows, a multiple of 8
+  float *line_inv;      // 1 / scale of every line
+  int blocks;
+};
+
+__device__ __forceinline__ float4 line_load4(const LineSplit &o, int row, int col) {
+  const float *p = o.x + (long long)row * o.pitch + col;
+  if (o.vec && col + 3 < o.cols) return __ldg(reinterpret_cast<const float4 *>(p));
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (col < o.cols) v.x = __ldg(p);
+  if (col + 1 < o.cols) v.y = __ldg(p + 1);
+  if (col + 2 < o.cols) v.z = __ldg(p + 2);
+  if (col + 3 < o.cols) v.w = __ldg(p + 3);
+  return v;
+}
+__device__ __forceinline__ unsigned abs_bits4(float4 v) {
+  return max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w)));
+}
+__device__ __forceinline__ void line_store4(const LineSplit &o, int row, int col, float4 v, float4 s) {
+  PlaneSink k;
+  k.hi = o.hi, k.lo = o.lo;
+  const float t[4] = {v.x * s.x, v.y * s.y, v.z * s.z, v.w * s.w};  // exact
+  sink_store4(k, (size_t)row * o.out_pitch + col, t, 1.f);
+}
+
+__device__ __forceinline__ void split_contiguous_lines(const LineSplit &o, int block, unsigned *flag) {
+  const int row = block * (LS_THREADS / 32) + (int)threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (row >= o.rows) return;
+  float4 v[LS_KEEP];
+  unsigned m = 0u;
 #pragma unroll
-    for (int y = 1; y < 8; ++y) v = max(v, fold[y][threadIdx.x]);
-    if (v) atomicMax(cmax + m, v);
+  for (int i = 0; i < LS_KEEP; ++i) {
+    const int col = lane * 4 + i * 128;
+    v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (col < o.cols) v[i] = line_load4(o, row, col);
+  }
+#pragma unroll
+  for (int i = 0; i < LS_KEEP; ++i) m = max(m, abs_bits4(v[i]));
+#pragma unroll 4
+  for (int col = lane * 4 + LS_KEEP * 128; col < o.cols; col += 128) m = max(m, abs_bits4(line_load4(o, row, col)));
+  m = __reduce_max_sync(0xffffffffu, m);
+  const float s = plane_scale_from_bits(m, PLANE_EXP_OWN);
+  const float4 s4 = make_float4(s, s, s, s);
+#pragma unroll
+  for (int i = 0; i < LS_KEEP; ++i) {
+    const int col = lane * 4 + i * 128;
+    if (col < o.cols) line_store4(o, row, col, v[i], s4);
+  }
+#pragma unroll 4
+  for (int col = lane * 4 + LS_KEEP * 128; col < o.cols; col += 128) line_store4(o, row, col, line_load4(o, row, col), s4);
+  if (lane == 0) {
+    o.line_inv[row] = 1.f / s;
+    if (m >= LS_HUGE) atomicOr(flag, GUARD_WHOLE);
   }
 }
 
-// planes_t[m, k] = halves of s_m x[k, m], s_m from the column's maximum: 32 x 32
-// tiles through shared memory.
-__global__ void transpose_split_kernel(const float *__restrict__ x, long long pitch, int K, int M,
-                                       const unsigned *__restrict__ cmax, uint16_t *__restrict__ hi_t,
-                                       uint16_t *__restrict__ lo_t, long long kp, float *__restrict__ line_inv) {
-  pdl_enter();
-  __shared__ float tile[32][33];
-  const int m0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
-  for (int y = threadIdx.y; y < 32; y += 8) {
-    const int k = k0 + y, m = m0 + threadIdx.x;
-    tile[y][threadIdx.x] = (k < K && m < M) ? x[(long long)k * pitch + m] : 0.f;
+__device__ __forceinline__ void split_column_lines(const LineSplit &o, int block, unsigned *flag) {
+  __shared__ uint4 fold[LS_THREADS / 16][LS_COLS / 4];
+  __shared__ unsigned cmax[LS_COLS];
+  __shared__ float scale[LS_COLS];
+  const int rank = block % LS_CLUSTER, col0 = block / LS_CLUSTER * LS_COLS;
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16, col = col0 + tx * 4;
+  const int r0 = (int)((long long)o.rows * rank / LS_CLUSTER) + ty, r1 = (int)((long long)o.rows * (rank + 1) / LS_CLUSTER);
+  constexpr int STEP = LS_THREADS / 16;
+  float4 v[LS_KEEP];
+  uint4 m = make_uint4(0u, 0u, 0u, 0u);
+  auto take = [&](float4 x) {
+    m.x = max(m.x, abs_bits(x.x)), m.y = max(m.y, abs_bits(x.y));
+    m.z = max(m.z, abs_bits(x.z)), m.w = max(m.w, abs_bits(x.w));
+  };
+#pragma unroll
+  for (int i = 0; i < LS_KEEP; ++i) {
+    v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r0 + i * STEP < r1 && col < o.cols) v[i] = line_load4(o, r0 + i * STEP, col);
   }
+#pragma unroll
+  for (int i = 0; i < LS_KEEP; ++i) take(v[i]);
+  if (col < o.cols) {
+#pragma unroll 4
+    for (int r = r0 + LS_KEEP * STEP; r < r1; r += STEP) take(line_load4(o, r, col));
+  }
+  fold[ty][tx] = m;
   __syncthreads();
-  for (int y = threadIdx.y; y < 32; y += 8) {
-    const int m = m0 + y, k = k0 + threadIdx.x;
-    if (m < M && k < kp) {
-      const float s = plane_scale_from_bits(cmax[m], PLANE_EXP_OWN);
-      __half h, l;
-      plane_halves(tile[threadIdx.x][y], s, &h, &l);
-      hi_t[(long long)m * kp + k] = *reinterpret_cast<const uint16_t *>(&h);
-      lo_t[(long long)m * kp + k] = *reinterpret_cast<const uint16_t *>(&l);
-      if (k == 0) line_inv[m] = 1.f / s;
+  if (threadIdx.x < LS_COLS) {
+    const unsigned *f = reinterpret_cast<const unsigned *>(fold);
+    unsigned w = 0u;
+#pragma unroll
+    for (int y = 0; y < LS_THREADS / 16; ++y) w = max(w, f[y * LS_COLS + threadIdx.x]);
+    cmax[threadIdx.x] = w;
+  }
+  tc::cluster_sync_all();
+  if (threadIdx.x < LS_COLS) {
+    unsigned w = 0u;
+#pragma unroll
+    for (int r = 0; r < LS_CLUSTER; ++r) {
+      unsigned u;
+      asm volatile("ld.shared::cluster.u32 %0, [%1];"
+                   : "=r"(u)
+                   : "r"(tc::map_to_cta(tc::smem_u32(cmax + threadIdx.x), (uint32_t)r)));
+      w = max(w, u);
+    }
+    const float s = plane_scale_from_bits(w, PLANE_EXP_OWN);
+    scale[threadIdx.x] = s;
+    if (rank == 0 && col0 + (int)threadIdx.x < o.cols) {
+      o.line_inv[col0 + threadIdx.x] = 1.f / s;
+      if (w >= LS_HUGE) atomicOr(flag, GUARD_WHOLE);
     }
   }
+  tc::cluster_sync_all();  // scales are set; no CTA leaves while another reads its maxima
+  if (col >= o.out_pitch) return;
+  const float4 s4 = *reinterpret_cast<const float4 *>(scale + tx * 4);
+#pragma unroll
+  for (int i = 0; i < LS_KEEP; ++i)
+    if (r0 + i * STEP < r1) line_store4(o, r0 + i * STEP, col, v[i], s4);
+#pragma unroll 4
+  for (int r = r0 + LS_KEEP * STEP; r < r1; r += STEP) line_store4(o, r, col, line_load4(o, r, col), s4);
+}
+
+// Blocks [0, a.blocks) work on a, the rest on b.  flag: set where an operand holds a
+// value the halves cannot stand for; next_flag: the word of the launch after this one.
+__global__ void __launch_bounds__(LS_THREADS) split_lines_kernel(const __grid_constant__ LineSplit a,
+                                                                 const __grid_constant__ LineSplit b, unsigned *flag,
+                                                                 unsigned *next_flag) {
+  pdl_enter();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *next_flag = 0u;
+  const bool second = (int)blockIdx.x >= a.blocks;
+  const LineSplit &o = second ? b : a;
+  const int block = second ? (int)blockIdx.x - a.blocks : (int)blockIdx.x;
+  if (o.by_columns) split_column_lines(o, block, flag);
+  else split_contiguous_lines(o, block, flag);
 }
 
 __global__ void __launch_bounds__(1024) planes_finalize_kernel(PlaneSink k) {
@@ -204,14 +315,69 @@ dlb_status launch_split(dlb_ctx *ctx, const float *x, size_t n, int rows, int co
 
 }  // namespace
 
-dlb_status planes_transpose_scaled(dlb_ctx *ctx, const float *x, long long pitch, int K, int M, uint16_t *hi_t,
-                                   uint16_t *lo_t, long long kp, unsigned *cmax, float *line_inv) {
-  DLB_CUDA(cudaMemsetAsync(cmax, 0, (size_t)M * sizeof(unsigned), ctx->stream));
-  const int slabs = max(1, min(ceil_div(K, 64), ceil_div(ctx->sm_count * 8, ceil_div(M, 32))));
-  const int rows_per_block = ceil_div(K, slabs);
-  DLB_LAUNCH_KERNEL(ctx, column_absmax_kernel, dim3(ceil_div(M, 32), ceil_div(K, rows_per_block)), dim3(32, 8), 0, x, pitch, K, M, rows_per_block, cmax);
-  DLB_LAUNCHED(ctx);
-  DLB_LAUNCH_KERNEL(ctx, transpose_split_kernel, dim3(ceil_div(M, 32), ceil_div((int)kp, 32)), dim3(32, 8), 0, x, pitch, K, M, cmax, hi_t, lo_t, kp, line_inv);
+static size_t line_rows(const GemmOperand &o, int mn, int k) { return o.stride_k == 1 ? mn : k; }
+static long long line_pitch(const GemmOperand &o, int mn, int k) {
+  return (long long)align_up((size_t)(o.stride_k == 1 ? k : mn), 8);
+}
+
+dlb_status planes_split_lines(dlb_ctx *ctx, GemmOperand *A, int M, GemmOperand *B, int N, int K) {
+  GemmOperand *const o[2] = {A, B};
+  const int mn[2] = {M, N};
+  size_t plane[2] = {0, 0}, halves = 0, lines = 0;
+  for (int i = 0; i < 2; ++i)
+    if (o[i]) {
+      plane[i] = align_up(line_rows(*o[i], mn[i], K) * (size_t)line_pitch(*o[i], mn[i], K), 64);
+      halves += 2 * plane[i];
+      lines += align_up((size_t)mn[i], 4);
+    }
+  if (!ctx->line_flags) {
+    DLB_CUDA(cudaMalloc(&ctx->line_flags, 2 * sizeof(unsigned)));
+    DLB_CUDA(cudaMemsetAsync(ctx->line_flags, 0, 2 * sizeof(unsigned), ctx->stream));
+  }
+  void *scr = nullptr;
+  DLB_TRY(scratch(ctx, halves * sizeof(uint16_t) + lines * sizeof(float), &scr));
+  uint16_t *h = static_cast<uint16_t *>(scr);
+  float *inv = reinterpret_cast<float *>(h + halves);
+  unsigned *flag = ctx->line_flags + (ctx->line_splits & 1), *next = ctx->line_flags + (~ctx->line_splits & 1);
+  ctx->line_splits++;
+  LineSplit job[2] = {};
+  bool columns = false;
+  for (int i = 0; i < 2; ++i)
+    if (o[i]) {
+      LineSplit &j = job[i];
+      GemmOperand &op = *o[i];
+      const bool by_rows = op.stride_k == 1;
+      j.x = op.ptr;
+      j.pitch = by_rows ? op.stride_mn : op.stride_k;
+      j.rows = by_rows ? mn[i] : K;
+      j.cols = by_rows ? K : mn[i];
+      j.by_columns = by_rows ? 0 : 1;
+      j.vec = (reinterpret_cast<uintptr_t>(j.x) & 15) == 0 && (j.pitch & 3) == 0;
+      j.hi = h;
+      j.lo = h + plane[i];
+      j.out_pitch = line_pitch(op, mn[i], K);
+      j.line_inv = inv;
+      j.blocks = by_rows ? (int)align_up((size_t)ceil_div(j.rows, LS_THREADS / 32), LS_CLUSTER)
+                         : LS_CLUSTER * (int)((j.out_pitch + LS_COLS - 1) / LS_COLS);
+      columns |= !by_rows;
+      op.fp32_stride_mn = op.stride_mn;
+      op.fp32_stride_k = op.stride_k;
+      (by_rows ? op.stride_mn : op.stride_k) = j.out_pitch;
+      op.h_hi = j.hi;
+      op.h_lo = j.lo;
+      op.scale = op.line_inv = inv;
+      op.guard = flag;
+      op.guard_mask = GUARD_WHOLE;
+      h += 2 * plane[i];
+      inv += align_up((size_t)mn[i], 4);
+    }
+  const unsigned grid = (unsigned)(job[0].blocks + job[1].blocks);
+  if (columns) {
+    DLB_CUDA(launch_kernel_cluster(ctx, split_lines_kernel, dim3(grid), dim3(LS_THREADS), 0, LS_CLUSTER, job[0], job[1],
+                                   flag, next));
+  } else {
+    DLB_LAUNCH_KERNEL(ctx, split_lines_kernel, grid, LS_THREADS, 0, job[0], job[1], flag, next);
+  }
   DLB_LAUNCHED(ctx);
   return DLB_OK;
 }
@@ -374,25 +540,6 @@ dlb_status planes_close(dlb_ctx *ctx, const PlaneJob &job) {
 
 dlb_status planes_absmax(dlb_ctx *ctx, const float *x, size_t n, float *slot) {
   DLB_LAUNCH_KERNEL(ctx, absmax_kernel, stream_blocks(ctx, n / 4 + 1), 256, 0, x, n, reinterpret_cast<unsigned *>(slot) + SLOT_AMAX);
-  DLB_LAUNCHED(ctx);
-  return DLB_OK;
-}
-
-dlb_status planes_split_adhoc(dlb_ctx *ctx, const float *x, size_t n, int rows, int cols, uint16_t *hi,
-                              uint16_t *lo, float *slot, unsigned *lines) {
-  if ((size_t)rows * (size_t)cols != n) rows = cols = 0;
-  DLB_CUDA(cudaMemsetAsync(slot, 0, SLOT_WORDS * sizeof(float), ctx->stream));
-  if (rows > 0 && lines) DLB_CUDA(cudaMemsetAsync(lines, 0, (size_t)(rows + cols) * sizeof(unsigned), ctx->stream));
-  DLB_TRY(planes_absmax(ctx, x, n, slot));
-  DLB_TRY(guard_counters(ctx));
-  PlaneSink k;
-  k.hi = hi;
-  k.lo = lo;
-  k.slot = slot;
-  sink_lines(k, rows > 0 ? lines : nullptr, rows, cols, false);
-  k.guard = ctx->d_guard;
-  DLB_TRY(launch_split(ctx, x, n, rows, cols, k));
-  DLB_LAUNCH_KERNEL(ctx, planes_finalize_kernel, 1, 1024, 0, k);
   DLB_LAUNCHED(ctx);
   return DLB_OK;
 }
