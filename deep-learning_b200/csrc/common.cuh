@@ -191,6 +191,28 @@ inline cudaError_t launch_kernel_cluster(dlb_ctx *ctx, void (*kernel)(P...), dim
   cfg.numAttrs = ctx->use_pdl ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+// Clusters of `cluster` blocks of the kernel that the device runs at once (fewer than
+// its SMs would hold where its processing clusters are not a multiple of that size).
+template <class... P>
+inline int resident_clusters(const dlb_ctx *ctx, void (*kernel)(P...), int threads, size_t smem, int cluster) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cluster * 64u);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int got = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&got, kernel, &cfg) != cudaSuccess || got < 1) {
+    cudaGetLastError();
+    got = ctx->sm_count / cluster;
+  }
+  return got;
+}
 #define DLB_LAUNCH_KERNEL(ctx, kernel, grid, block, smem, ...) \
   dlb::launch_kernel((ctx), (kernel), dim3(grid), dim3(block), (size_t)(smem), __VA_ARGS__)
 #endif
@@ -266,6 +288,10 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float 
                 long long ldc, int M, int N, int K, const GemmEpilogue &ep);
 dlb_status gemm_simt(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C,
                      long long ldc, int M, int N, int K, const GemmEpilogue &ep);
+// Small products in fp32 on the CUDA cores (gemm_small.cu).
+dlb_status gemm_small(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C, long long ldc, int M, int N,
+                      int K, const GemmEpilogue &ep);
+double gemm_small_us(const dlb_ctx *ctx, int M, int N, int K);
 // Tensor-core product from the fp32 tensors (gemm_direct.cu).
 dlb_status gemm_direct(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C, long long ldc, int M, int N,
                        int K, const GemmEpilogue &ep);

@@ -86,6 +86,27 @@ static dlb_status gemm_tensor_core(dlb_ctx *ctx, const GemmOperand &A, const Gem
   return st;
 }
 
+// Outputs that fill a 256 x 256 tile can run on fp16 planes.
+static bool plane_size(int M, int N, int K) { return (long long)M * N >= 256 * 256 && K >= 32; }
+// About how long the making of planes for one product takes.
+static double split_us(long long elements) { return 3.0 + (double)elements / 0.7e6; }
+// The ways of the fp16 form: the shortest by the kernels' own estimates, with
+// `planes_cost` us on top of a product on planes for what its planes take.
+enum class Way { SMALL, DIRECT, PLANES };
+static Way gemm_way(const dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K,
+                    bool accumulate, double planes_cost) {
+  const double small = gemm_small_us(ctx, M, N, K), direct = gemm_direct_us(ctx, M, N, K);
+  if (plane_size(M, N, K) && gemm_pair_enabled() && !(A.stride_k != 1 && B.stride_k == 1)) {
+    const double planes = gemm_planes_us(ctx, A, B, M, N, K, accumulate) + planes_cost;
+    if (planes <= small && planes <= direct) return Way::PLANES;
+  }
+  return small < direct ? Way::SMALL : Way::DIRECT;
+}
+// Planes that are missing, made for the product.
+static double fresh_us(int M, int N, int K, bool have_a, bool have_b) {
+  return split_us((have_a ? 0 : (long long)M * K) + (have_b ? 0 : (long long)N * K));
+}
+
 // The fused epilogues exist in the medium fp16-plane kernel, for K-major A, with both
 // operands' planes kept by the caller and a dense output.  Outputs large enough
 // for the persistent kernel on 256 x 256 tiles take the kernels one after the
@@ -104,20 +125,6 @@ bool gemm_fused_supported(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand 
   return (a.h_hi || planes_lookup(ctx, a.lo, &a)) && (b.h_hi || planes_lookup(ctx, b.lo, &b));
 }
 
-// Outputs that fill a 256 x 256 tile can run on fp16 planes.
-static bool plane_size(int M, int N, int K) { return (long long)M * N >= 256 * 256 && K >= 32; }
-// About how long the making of planes for one product takes.
-static double split_us(long long elements) { return 3.0 + (double)elements / 0.7e6; }
-
-// Whether the product runs on planes, given which operands' are kept: by the shorter
-// of that, with the missing ones made for it, and the direct kernel.
-static bool planes_better(const dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K,
-                          bool accumulate, bool have_a, bool have_b) {
-  if (have_a && have_b) return true;
-  if (!gemm_pair_enabled() || (A.stride_k != 1 && B.stride_k == 1)) return false;
-  const long long fresh = (have_a ? 0 : (long long)M * K) + (have_b ? 0 : (long long)N * K);
-  return gemm_planes_us(ctx, A, B, M, N, K, accumulate) + split_us(fresh) < gemm_direct_us(ctx, M, N, K);
-}
 // Whether kept planes serve: TMA takes their pitch and the caller asks for no scale per
 // line.  An mn-contiguous A (the error of a weight gradient) whose rows are no whole
 // 128-byte columns of halves is taken for one over classes and gets those scales too.
@@ -129,9 +136,12 @@ static bool planes_serve(const GemmOperand &o, int mn, int k, bool is_a) {
 
 PlaneUse gemm_plane_use(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K) {
   if (ctx->gemm_kind != DLB_GEMM_F16X3) return {true, true};
-  if (!plane_size(M, N, K)) return {false, false};
+  // Kept planes are a few bytes more to write for the kernel that makes the tensor and
+  // a check launch each: 4 us a product (an epoch of 128-row batches of 784-256-10
+  // takes 1430 us where its largest weight gradient has planes, 1340 where not).
   const bool a = planes_serve(A, M, K, true), b = planes_serve(B, N, K, false);
-  const bool on = planes_better(ctx, A, B, M, N, K, false, a, b);
+  const double cost = a && b ? 4.0 : fresh_us(M, N, K, a, b);
+  const bool on = gemm_way(ctx, A, B, M, N, K, false, cost) == Way::PLANES;
   return {on && a, on && b};
 }
 
@@ -147,7 +157,8 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
   const bool big = ((long long)M * N >= 128 * 64 && K >= 32) || ctx->gemm_kind == DLB_GEMM_F16X3;
   if (!(ctx->use_tensor_core && ctx->tensor_core_ok && big)) return gemm_simt(ctx, A, B, C, ldc, M, N, K, ep);
 
-  // The fp16 form runs on planes or splits its operands in the product (gemm_direct).
+  // The fp16 form leaves the smallest products to the CUDA cores (gemm_small).  Others run
+  // on planes or split their operands in the product (gemm_direct).
   // Planes that the caller keeps are used wherever TMA can address them and the output
   // fills a 256 x 256 tile.  Missing ones are made for this product, with a scale per
   // line, where that and the product on planes are estimated to be shorter than the
@@ -163,7 +174,11 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
       have_a = A.h_hi || (planes_serve(A, M, K, true) && planes_lookup(ctx, A.lo, &A));
       have_b = B.h_hi || (planes_serve(B, N, K, false) && planes_lookup(ctx, B.lo, &B));
     }
-    if (!plane_size(M, N, K) || !planes_better(ctx, A, B, M, N, K, ep.accumulate, have_a, have_b)) {
+    const bool kept = have_a && have_b && gemm_f16_supported(A, B, C, ldc, M, N, K);
+    const Way way = kept ? Way::PLANES
+                         : gemm_way(ctx, A, B, M, N, K, ep.accumulate, fresh_us(M, N, K, have_a, have_b));
+    if (way == Way::SMALL) return gemm_small(ctx, A_in, B_in, C, ldc, M, N, K, ep);
+    if (way == Way::DIRECT) {
       ProfileSpan span;
       DLB_TRY(span.begin(ctx, 0, 2.0 * M * N * K));
       DLB_TRY(gemm_direct(ctx, A_in, B_in, C, ldc, M, N, K, ep));

@@ -4,6 +4,7 @@
 // 128-bit accesses; per-unit (column) reductions go through partials in the
 // context scratch arena and are finished in double in a fixed order, so results
 // do not depend on block scheduling.
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -731,36 +732,57 @@ __global__ void sums_to_bias_grad_kernel(const double *__restrict__ sums, int n,
   else dbias[h] = (float)sums[h];
 }
 
-// MSE (or any non-softmax output): delta = f'(x,q) * 2 (q - y) / (N * n_out).
-__global__ void loss_delta_mse_kernel(const float *__restrict__ pre, const float *__restrict__ q,
-                                      const float *__restrict__ y, float *__restrict__ delta,
-                                      float *__restrict__ delta_lo, int af, size_t total,
-                                      float denom, double *loss_sum, unsigned *amax) {
-  pdl_enter();
-  __shared__ double red[8];
-  double local = 0.0;
-  unsigned mx = 0;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const float qq = q[i], yy = y[i];
-    const float diff = qq - yy;
-    local += (double)(diff * diff);  // loss_fn: pow(q - y, 2) in float, summed in double
-    float dl = 2.f * diff;
-    dl /= denom;
-    const float e = af_derive(af, pre[i], qq) * dl;
-    delta[i] = e;
-    mx = max(mx, abs_bits(e));
-    if (delta_lo) delta_lo[i] = tf32_lo(e);
-  }
-  amax_commit(amax, mx);
-  for (int o = 16; o; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = local;
+// Adds the block's values into *sum with one atomic: the double atomics of a grid
+// queue on one address, and one per block (or per warp) of a large grid took most of
+// the loss kernels' time (2048 x 1000 softmax 33 us, 10000 x 10 evaluation 24).
+__device__ __forceinline__ void block_add(double v, double *sum) {
+  __shared__ double red[32];
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = v;
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int w = 0; w < (int)(blockDim.x / 32); ++w) t += red[w];
-    atomicAdd(loss_sum, t);
+    if (t != 0.0) atomicAdd(sum, t);
   }
+  __syncthreads();
+}
+
+// MSE (or any non-softmax output): delta = f'(x,q) * 2 (q - y) / (N * n_out).
+// `total4` quads by 16-byte accesses, the rest (all of it where a pointer is not
+// aligned) one by one.
+__global__ void loss_delta_mse_kernel(const float *__restrict__ pre, const float *__restrict__ q,
+                                      const float *__restrict__ y, float *__restrict__ delta,
+                                      float *__restrict__ delta_lo, int af, size_t total, size_t total4,
+                                      float denom, double *loss_sum, unsigned *amax) {
+  pdl_enter();
+  double local = 0.0;
+  unsigned mx = 0;
+  const size_t stride = (size_t)gridDim.x * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  auto one = [&](float x, float qq, float yy) {
+    const float diff = qq - yy;
+    local += (double)(diff * diff);  // loss_fn: pow(q - y, 2) in float, summed in double
+    float dl = 2.f * diff;
+    dl /= denom;
+    const float e = af_derive(af, x, qq) * dl;
+    mx = max(mx, abs_bits(e));
+    return e;
+  };
+  for (size_t i = first; i < total4; i += stride) {
+    const float4 x = __ldg(reinterpret_cast<const float4 *>(pre) + i), v = __ldg(reinterpret_cast<const float4 *>(q) + i),
+                 t = __ldg(reinterpret_cast<const float4 *>(y) + i);
+    const float4 e = make_float4(one(x.x, v.x, t.x), one(x.y, v.y, t.y), one(x.z, v.z, t.z), one(x.w, v.w, t.w));
+    reinterpret_cast<float4 *>(delta)[i] = e;
+    if (delta_lo)
+      reinterpret_cast<float4 *>(delta_lo)[i] = make_float4(tf32_lo(e.x), tf32_lo(e.y), tf32_lo(e.z), tf32_lo(e.w));
+  }
+  for (size_t i = 4 * total4 + first; i < total; i += stride) {
+    const float e = one(pre[i], q[i], y[i]);
+    delta[i] = e;
+    if (delta_lo) delta_lo[i] = tf32_lo(e);
+  }
+  amax_commit(amax, mx);
+  block_add(local, loss_sum);
 }
 
 // Softmax + cross-entropy, one warp per row.
@@ -785,9 +807,20 @@ __global__ void loss_delta_softmax_ce_kernel(const float *__restrict__ q, const 
     const float *qr = q + (size_t)warp * n, *yr = y + (size_t)warp * n;
     const float EPS = 1e-7f;
     int count = 0;
+    // The targets of eight rounds at a time: one by one every round waited for its own
+    // (33 us at 2048 x 1000).
+    constexpr int AHEAD = 8;
+    float yk[AHEAD];
     for (int k0 = 0; k0 < n; k0 += 32) {
-      const int k = k0 + lane;
-      const bool hit = k < n && yr[k] == 1.f;
+      const int k = k0 + lane, at8 = (k0 / 32) % AHEAD;
+      if (at8 == 0) {
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) yk[i] = k + i * 32 < n ? yr[k + i * 32] : 0.f;
+      }
+      float yv = yk[0];
+#pragma unroll
+      for (int i = 1; i < AHEAD; ++i) yv = at8 == i ? yk[i] : yv;
+      const bool hit = k < n && yv == 1.f;
       const unsigned m = __ballot_sync(0xffffffffu, hit);
       if (hit) {
         const int at = count + __popc(m & ((1u << lane) - 1u));
@@ -803,6 +836,7 @@ __global__ void loss_delta_softmax_ce_kernel(const float *__restrict__ q, const 
       count += __popc(m);
     }
     __syncwarp();
+#pragma unroll 4
     for (int j = lane; j < n; j += 32) {
       const float qj = qr[j];
       float e = 0.f;
@@ -828,8 +862,7 @@ __global__ void loss_delta_softmax_ce_kernel(const float *__restrict__ q, const 
     }
   }
   amax_commit(amax, mx);
-  for (int o = 16; o; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-  if (lane == 0 && local != 0.0) atomicAdd(loss_sum, local);
+  block_add(local, loss_sum);
 }
 
 }  // namespace dlb
@@ -1013,7 +1046,11 @@ dlb_status loss_delta_impl(dlb_ctx *ctx, int loss, int af, const float *pre, con
     const size_t total = (size_t)rows * n_out;
     // loss_fn_derivative divides by static_cast<real>(bs * n_out).
     const float denom = (float)((size_t)global_rows * (size_t)n_out);
-    DLB_LAUNCH_KERNEL(ctx, loss_delta_mse_kernel, stream_grid(ctx, total, 256), 256, 0, pre, q, y, delta, delta_lo, af, total, denom, loss_sum, amax);
+    const bool vec = ((reinterpret_cast<uintptr_t>(pre) | reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(y) |
+                       reinterpret_cast<uintptr_t>(delta) | reinterpret_cast<uintptr_t>(delta_lo)) & 15) == 0;
+    const size_t total4 = vec ? total / 4 : 0, items = vec ? total / 4 + 3 : total;
+    const int grid = (int)std::max<size_t>(1, std::min<size_t>((items + 255) / 256, (size_t)ctx->sm_count * 4));
+    DLB_LAUNCH_KERNEL(ctx, loss_delta_mse_kernel, grid, 256, 0, pre, q, y, delta, delta_lo, af, total, total4, denom, loss_sum, amax);
     DLB_LAUNCHED(ctx);
     return DLB_OK;
   }
@@ -1388,9 +1425,9 @@ __global__ void loss_eval_kernel(int loss, int accu_fn, float accu_var, const fl
                                  const float *__restrict__ y, int rows, int n, double *loss_sum,
                                  double *accu_sum) {
   pdl_enter();
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x % 32;
+  const int lane = threadIdx.x % 32;
   double local = 0.0, hits = 0.0;
-  if (warp < rows) {
+  for (int warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32; warp < rows; warp += gridDim.x * (blockDim.x / 32)) {
     const float *qr = q + (size_t)warp * n, *yr = y + (size_t)warp * n;
     const float EPS = 1e-7f;
     // Largest output (the last of equal maxima, as `q >= q_max` keeps it) and
@@ -1421,17 +1458,11 @@ __global__ void loss_eval_kernel(int loss, int accu_fn, float accu_var, const fl
         // the last flagged index wins; n means none
         if (ot != n && (target == n || ot > target)) target = ot;
       }
-      if (lane == 0 && predict == target) hits = 1.0;
+      if (lane == 0 && predict == target) hits += 1.0;
     }
   }
-  for (int o = 16; o; o >>= 1) {
-    local += __shfl_xor_sync(0xffffffffu, local, o);
-    if (accu_fn == DLB_ACCU_DISTANCE) hits += __shfl_xor_sync(0xffffffffu, hits, o);
-  }
-  if (lane == 0) {
-    if (loss_sum && local != 0.0) atomicAdd(loss_sum, local);
-    if (hits != 0.0) atomicAdd(accu_sum, hits);
-  }
+  if (loss_sum) block_add(local, loss_sum);
+  block_add(hits, accu_sum);
 }
 }  // namespace dlb
 
@@ -1444,7 +1475,7 @@ extern "C" dlb_status dlb_loss_eval(dlb_ctx *ctx, int loss, int accu_fn, float a
     set_error("dlb_loss_eval: loss %d / accuracy function %d outside the supported set", loss, accu_fn);
     return DLB_ERR_UNSUPPORTED;
   }
-  DLB_LAUNCH_KERNEL(ctx, loss_eval_kernel, ceil_div(rows, 8), 256, 0, loss, accu_fn, accu_var, q, y, rows, n_out, loss_sum, accu_sum);
+  DLB_LAUNCH_KERNEL(ctx, loss_eval_kernel, std::min(ceil_div(rows, 8), ctx->sm_count), 256, 0, loss, accu_fn, accu_var, q, y, rows, n_out, loss_sum, accu_sum);
   DLB_LAUNCHED(ctx);
   return DLB_OK;
 }

@@ -2,10 +2,10 @@
 // operands of any size, pitch and alignment, without plane buffers.
 //
 // The plane kernels (gemm_pair.cu, gemm_tcgen05.cu) read operands that were
-// split into fp16 planes beforehand and that TMA can address; everything else
-// (widths that are no multiple of 8, weight gradients whose output rows are no
-// multiple of 64, outputs below a 256 x 256 tile) ran on the CUDA cores, one
-// 64 x 64 tile per block whatever K.  Here sixteen warps read fp32, split it in
+// split into fp16 planes beforehand and that TMA can address, and gemm_small.cu takes
+// a few million multiply-adds; what lies between (outputs below a 256 x 256 tile
+// with a long k, outputs for which making planes first takes longer) ran on the CUDA
+// cores, one 64 x 64 tile per block whatever K.  Here sixteen warps read fp32, split it in
 // registers and write the swizzled operand tiles the tensor core reads:
 //
 //   converters  warps 0-15   8 lines of A and 8 of B per chunk of 64 k each, the
@@ -23,15 +23,15 @@
 // guard here: nothing to flag.  A line with a value of 2^101 or more, infinity or
 // NaN sends its tile through the fp32 body at the end instead.
 //
-// Accumulation.  A chunk is 64 deep: four accumulator buffers of 128 columns in
+// Accumulation.  A chunk is 64 deep: two accumulator buffers of 128 columns in
 // tensor memory, each drained with round-to-nearest adds, so the tensor core's
 // truncating adder only sees sums of 64 products.
 //
-// What bounds it: the fp32 tiles come from L2 (64 KB per 64-deep chunk of a
-// 128 x 128 tile) and the conversion issues about 18 instructions per line of
-// 64 values, both about twice the 768 cycles of a chunk's MMAs.  That is why
-// outputs of 256 x 256 and more stay on the plane kernels, whose operands were
-// split once.  A small output has few tiles: up to eight CTAs of a cluster
+// What bounds it: the conversion.  A chunk of a 128 x 128 tile takes about 5000 cycles
+// where its MMAs take 768: 12000 instructions of loads, line maxima, splits and
+// stores, and their latencies.  That is why larger outputs go to the plane kernels,
+// whose operands are split once: 333 x 1203 x 1203 takes 25 us here (172 us on the CUDA
+// cores), 1024 x 1000 x 2048 54 (6 + 17 on planes).  A small output has few tiles: up to eight CTAs of a cluster
 // then share a tile's k range, and each adds the others' parts of its slice of
 // columns through distributed shared memory, in rank order, so that results
 // do not depend on timing.
@@ -59,6 +59,7 @@ constexpr int D_PARTS = D_STAGES * D_STAGE;      // partial sums of this CTA's c
 constexpr int D_PART_BYTES = DM * (DN + 8 * 4) * 4;
 constexpr int D_SCALES = D_PARTS + D_PART_BYTES; // [D_STAGES][DM + DN] floats
 constexpr int D_BARS = D_SCALES + D_STAGES * (DM + DN) * 4;
+constexpr int D_MAX_SHIFT = 3;
 constexpr int D_SMEM = D_BARS + 128 + 1024;
 static_assert(D_COLS == 32 && D_LINES == 8, "fragment sizes below");
 static_assert(D_SMEM <= 232448, "shared memory of one CTA");
@@ -442,11 +443,19 @@ __global__ void __launch_bounds__(D_THREADS, 1) gemm_direct_kernel(const __grid_
   }
 }
 
-// CTAs per tile: as many as the chip has room for, each with a chunk at least.
+int clusters_at_once(const dlb_ctx *ctx, int shift) {
+  static int known[MAX_DEVICES][D_MAX_SHIFT + 1] = {};
+  int &n = known[ctx->device][shift];
+  if (n == 0) n = resident_clusters(ctx, gemm_direct_kernel<false, false>, D_THREADS, D_SMEM, 1 << shift);
+  return n;
+}
+
+// CTAs per tile: as many as the chip runs at once (16 tiles by clusters of eight are
+// two rounds on 148 SMs: 512^3 22 us against 14), each with a chunk at least.
 int direct_split_shift(const dlb_ctx *ctx, int M, int N, int K) {
   const int tiles = ceil_div(M, DM) * ceil_div(N, DN), chunks = ceil_div(K, DK);
   int s = 0;
-  while (s < 3 && (tiles << (s + 1)) <= ctx->sm_count && (2 << s) <= chunks) ++s;
+  while (s < D_MAX_SHIFT && tiles <= clusters_at_once(ctx, s + 1) && (2 << s) <= chunks) ++s;
   return s;
 }
 

@@ -408,33 +408,15 @@ dlb_status launch_mid(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, 
   }
 }
 
-// Clusters of 2 << shift CTAs that the device runs at once (fewer than the SMs
-// would hold where its processing clusters are not a multiple of that size).
-int resident_clusters(const dlb_ctx *ctx, int shift) {
+int clusters_at_once(const dlb_ctx *ctx, int shift) {
   static int known[MAX_DEVICES][Q_MAX_SHIFT + 1] = {};
   int &n = known[ctx->device][shift];
-  if (n == 0) {
-    auto kernel = shift == 0   ? gemm_mid_kernel<false, false, false, 0>
-                  : shift == 1 ? gemm_mid_kernel<false, false, false, 1>
-                               : gemm_mid_kernel<false, false, false, 2>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(2 << shift) * 64u);
-    cfg.blockDim = dim3(NUM_THREADS);
-    cfg.dynamicSmemBytes = Q_SMEM;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2u << shift;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int got = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&got, kernel, &cfg) != cudaSuccess || got < 1) {
-      cudaGetLastError();
-      got = ctx->sm_count / (2 << shift);
-    }
-    n = got;
-  }
+  if (n == 0)
+    n = resident_clusters(ctx,
+                          shift == 0   ? gemm_mid_kernel<false, false, false, 0>
+                          : shift == 1 ? gemm_mid_kernel<false, false, false, 1>
+                                       : gemm_mid_kernel<false, false, false, 2>,
+                          NUM_THREADS, Q_SMEM, 2 << shift);
   return n;
 }
 
@@ -465,7 +447,7 @@ double gemm_mid_us(const dlb_ctx *ctx, int M, int N, int K, int *split_shift) {
   double best = 1e30;
   for (int s = 0; s <= Q_MAX_SHIFT; ++s) {
     if (s && kb < (Q_CHUNK << s)) break;  // a chunk at least per piece
-    const int at_once = resident_clusters(ctx, s);
+    const int at_once = clusters_at_once(ctx, s);
     const long long rounds = (tiles + at_once - 1) / at_once;
     const double us = 2.5 + (double)rounds * (4.5 + (s ? 0.8 : 0.0) + 0.55 * ceil_div(kb, 1 << s));
     if (us < best) {

@@ -530,26 +530,7 @@ int walk_clusters(const dlb_ctx *ctx, int cs) {
   if (cs == 1) return ctx->sm_count;
   static int known[MAX_DEVICES][W_MAX_CLUSTER + 1] = {};
   int &n = known[ctx->device][cs];
-  if (n == 0) {
-    auto kernel = lstm_forward_walk_kernel<4, 4, 0>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)cs * 64u);
-    cfg.blockDim = dim3(W_THREADS);
-    cfg.dynamicSmemBytes = W_SMEM_MAX;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)cs;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int got = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W_SMEM_MAX) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&got, kernel, &cfg) != cudaSuccess || got < 1) {
-      cudaGetLastError();
-      got = ctx->sm_count / cs;
-    }
-    n = got;
-  }
+  if (n == 0) n = resident_clusters(ctx, lstm_forward_walk_kernel<4, 4, 0>, W_THREADS, W_SMEM_MAX, cs);
   return n;
 }
 

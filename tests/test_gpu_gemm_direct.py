@@ -1,6 +1,7 @@
 """Products formed from the fp32 tensors by the tensor-core kernel that splits its
-operands itself (csrc/gemm_direct.cu): every size and pitch the plane kernels do
-not take, against the float64 product, line by line."""
+operands itself (csrc/gemm_direct.cu) and by the CUDA-core kernel for small ones
+(csrc/gemm_small.cu): every size and pitch the plane kernels do not take, against the
+float64 product, line by line."""
 import numpy as np
 import pytest
 
@@ -9,10 +10,12 @@ from dlb200 import check
 
 pytestmark = pytest.mark.gpu
 
-# rows, n_in, n_out: edges of the 128 x 128 tile and of the 64-deep chunk, one
-# chunk, several CTAs per tile, more tiles than SMs, lines of odd and even pitch.
+# rows, n_in, n_out: edges of the 32 x 32 and 128 x 128 tiles and of the 128- and 64-deep
+# chunks, one chunk, several CTAs per tile, more tiles than SMs, lines of odd and even
+# pitch; the second line by the direct kernel (shallow large outputs, long thin sums).
 SHAPES = [(1, 1, 1), (3, 65, 2), (127, 63, 129), (128, 64, 128), (129, 127, 130), (16, 784, 10), (1, 784, 256),
-          (333, 617, 203), (200, 513, 1027), (1000, 66, 1001), (77, 2050, 77), (1700, 129, 1601)]
+          (333, 617, 203), (200, 513, 1027), (1000, 66, 1001), (77, 2050, 77), (1700, 129, 1601), (31, 255, 33), (32, 256, 32), (1025, 127, 31),
+          (1305, 23, 2213), (1001, 5, 2825), (951, 7735, 65), (130, 9001, 127)]
 
 
 def _products(ctx, x, w, d, bias=None, start=None):
