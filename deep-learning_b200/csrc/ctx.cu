@@ -5,6 +5,8 @@
 #include <stdarg.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace dlb {
@@ -90,21 +92,27 @@ static dlb_status gemm_tensor_core(dlb_ctx *ctx, const GemmOperand &A, const Gem
 static bool plane_size(int M, int N, int K) { return (long long)M * N >= 256 * 256 && K >= 32; }
 // About how long the making of planes for one product takes.
 static double split_us(long long elements) { return 3.0 + (double)elements / 0.7e6; }
-// The ways of the fp16 form: the shortest by the kernels' own estimates, with
-// `planes_cost` us on top of a product on planes for what its planes take.
+// Whether planes_us, the time of a product on planes and of what its planes take, beats
+// the small kernel.  An output that gives most SMs two of that kernel's tiles, and no
+// side of which makes mostly padding of a plane kernel's tile, stays on planes: they
+// win from about 128 k on (512^3: 9 us against 16) and lose 2 us at most below, and the
+// range guard sees the errors of a wide layer whatever its depth.
+static bool planes_beat_small(const dlb_ctx *ctx, int M, int N, int K, double planes_us) {
+  const bool crowded = std::min(M, N) >= 64 && 2LL * ceil_div(M, 32) * ceil_div(N, 32) > 3LL * ctx->sm_count;
+  return crowded || planes_us <= gemm_small_us(ctx, M, N, K);
+}
+// The way of a product whose operands' planes are not both kept: the shortest by the
+// kernels' own estimates, missing planes made for it.
 enum class Way { SMALL, DIRECT, PLANES };
 static Way gemm_way(const dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K,
-                    bool accumulate, double planes_cost) {
-  const double small = gemm_small_us(ctx, M, N, K), direct = gemm_direct_us(ctx, M, N, K);
+                    bool accumulate, bool have_a, bool have_b) {
+  const double direct = gemm_direct_us(ctx, M, N, K);
   if (plane_size(M, N, K) && gemm_pair_enabled() && !(A.stride_k != 1 && B.stride_k == 1)) {
-    const double planes = gemm_planes_us(ctx, A, B, M, N, K, accumulate) + planes_cost;
-    if (planes <= small && planes <= direct) return Way::PLANES;
+    const double planes = gemm_planes_us(ctx, A, B, M, N, K, accumulate) +
+                          split_us((have_a ? 0 : (long long)M * K) + (have_b ? 0 : (long long)N * K));
+    if (planes <= direct && planes_beat_small(ctx, M, N, K, planes)) return Way::PLANES;
   }
-  return small < direct ? Way::SMALL : Way::DIRECT;
-}
-// Planes that are missing, made for the product.
-static double fresh_us(int M, int N, int K, bool have_a, bool have_b) {
-  return split_us((have_a ? 0 : (long long)M * K) + (have_b ? 0 : (long long)N * K));
+  return gemm_small_us(ctx, M, N, K) < direct ? Way::SMALL : Way::DIRECT;
 }
 
 // The fused epilogues exist in the medium fp16-plane kernel, for K-major A, with both
@@ -136,12 +144,13 @@ static bool planes_serve(const GemmOperand &o, int mn, int k, bool is_a) {
 
 PlaneUse gemm_plane_use(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K) {
   if (ctx->gemm_kind != DLB_GEMM_F16X3) return {true, true};
+  if (!plane_size(M, N, K)) return {false, false};
+  const bool a = planes_serve(A, M, K, true), b = planes_serve(B, N, K, false);
   // Kept planes are a few bytes more to write for the kernel that makes the tensor and
   // a check launch each: 4 us a product (an epoch of 128-row batches of 784-256-10
   // takes 1430 us where its largest weight gradient has planes, 1340 where not).
-  const bool a = planes_serve(A, M, K, true), b = planes_serve(B, N, K, false);
-  const double cost = a && b ? 4.0 : fresh_us(M, N, K, a, b);
-  const bool on = gemm_way(ctx, A, B, M, N, K, false, cost) == Way::PLANES;
+  const bool on = a && b ? planes_beat_small(ctx, M, N, K, gemm_planes_us(ctx, A, B, M, N, K, false) + 4.0)
+                         : gemm_way(ctx, A, B, M, N, K, false, a, b) == Way::PLANES;
   return {on && a, on && b};
 }
 
@@ -175,8 +184,7 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
       have_b = B.h_hi || (planes_serve(B, N, K, false) && planes_lookup(ctx, B.lo, &B));
     }
     const bool kept = have_a && have_b && gemm_f16_supported(A, B, C, ldc, M, N, K);
-    const Way way = kept ? Way::PLANES
-                         : gemm_way(ctx, A, B, M, N, K, ep.accumulate, fresh_us(M, N, K, have_a, have_b));
+    const Way way = kept ? Way::PLANES : gemm_way(ctx, A, B, M, N, K, ep.accumulate, have_a, have_b);
     if (way == Way::SMALL) return gemm_small(ctx, A_in, B_in, C, ldc, M, N, K, ep);
     if (way == Way::DIRECT) {
       ProfileSpan span;

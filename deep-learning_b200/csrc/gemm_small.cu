@@ -172,13 +172,14 @@ dlb_status launch_small(dlb_ctx *ctx, const SmallArgs &args, int tiles) {
 
 }  // namespace
 
-// About how long it takes: 1.5 us a chunk, and more where an SM has several CTAs.
+// About how long it takes: 1.6 us a chunk, and more where an SM has several CTAs (512^3,
+// two to an SM: 15.8 us; 300 x 1024 x 300, three: 15.6).
 double gemm_small_us(const dlb_ctx *ctx, int M, int N, int K) {
   const int shift = small_split_shift(ctx, M, N, K);
   const long long ctas = ((long long)ceil_div(M, ST) * ceil_div(N, ST)) << shift;
   const int chunks = ceil_div(ceil_div(K, 1 << shift), SK);
   const double per_sm = (double)((ctas + ctx->sm_count - 1) / ctx->sm_count);
-  return 3.2 + (shift ? 0.8 : 0.0) + chunks * std::max(1.5, 1.0 * per_sm);
+  return 3.2 + (shift ? 0.8 : 0.0) + chunks * std::max(1.6, 1.45 * per_sm);
 }
 
 dlb_status gemm_small(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C, long long ldc, int M, int N,
