@@ -442,6 +442,14 @@ constexpr int SCALE_SLOTS = 8192;
 constexpr int SLOT_WORDS = 8;    // words of one scale slot (layout: planes.cuh)
 constexpr int MAX_DEVICES = 64;  // device indices a process may hold contexts on
 
+// dlb_brn_forward_sums and _finalize of a single rank, and the backward sums with the
+// gradients of gamma and beta, each without the launch in between.
+dlb_status brn_forward_statistics(dlb_ctx *ctx, const float *Z, int rows, int global_rows, int n_units, float momentum,
+                                  float epsilon, float r_max, float d_max, const dlb_brn_unit_arrays *u);
+dlb_status brn_activation_backward(dlb_ctx *ctx, float *dA, const float *Z, const float *A,
+                                   const dlb_brn_unit_arrays *u, int af, int rows, int n_units, double *sums,
+                                   float *d_gamma, float *d_beta);
+
 // All time steps of an LSTM layer in one launch (lstm_walk.cu).  done: whether this
 // was the faster way and has been enqueued; the step entry points otherwise.
 // Backward: dH [T, rows, C] gets the recurrent part added.

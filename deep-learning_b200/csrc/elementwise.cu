@@ -44,9 +44,9 @@ constexpr size_t column_reduce_shared_bytes() {
   return ring > fold ? ring : fold;
 }
 
-template <int NSUM, class Op>
+template <int NSUM, class Op, class Fin>
 __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, Op::MIN_BLOCKS)
-    column_reduce_kernel(Op op, int rows, int n, int rows_per_chunk, double *partials) {
+    column_reduce_kernel(Op op, int rows, int n, int rows_per_chunk, double *partials, Fin fin) {
   pdl_enter();
   extern __shared__ float4 cr_shared[];
   const int tx = threadIdx.x % CR_LANES_X, ty = threadIdx.x / CR_LANES_X;
@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, Op::MIN_BLOCKS)
   for (int s = 0; s < NSUM; ++s)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[s][j] = 0.f;
+  double whole[NSUM][4] = {};
 
   if (col < n) {
     if ((n & 3) == 0) {
@@ -75,6 +76,16 @@ __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, Op::MIN_BLOCKS)
         // iteration by plain loads, all of them sent before the first is used.
         constexpr int U = Op::IN_FLIGHT;
         for (int r = r0 + ty; r < r1; r += U * CR_LANES_Y) {
+          if (gridDim.y == 1) {
+            // All rows in one chunk: fp32 sums of four rows, the rest in double.
+#pragma unroll
+            for (int s = 0; s < NSUM; ++s)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                whole[s][j] += (double)acc[s][j];
+                acc[s][j] = 0.f;
+              }
+          }
           float4 x[U][Op::NIN];
 #pragma unroll
           for (int k = 0; k < U; ++k)
@@ -106,7 +117,7 @@ __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, Op::MIN_BLOCKS)
 #pragma unroll
   for (int s = 0; s < NSUM; ++s)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) red[ty][s][tx * 4 + j] = (double)acc[s][j];
+    for (int j = 0; j < 4; ++j) red[ty][s][tx * 4 + j] = whole[s][j] + (double)acc[s][j];
   __syncthreads();
   // 256 threads fold NSUM*128 columns.
   for (int i = threadIdx.x; i < NSUM * CR_COLS; i += CR_LANES_X * CR_LANES_Y) {
@@ -116,25 +127,70 @@ __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, Op::MIN_BLOCKS)
       double t = 0.0;
 #pragma unroll
       for (int y = 0; y < CR_LANES_Y; ++y) t += red[y][s][c];
-      partials[((size_t)blockIdx.y * NSUM + s) * n + gc] = t;
+      // One chunk: the sums are whole.  They pass through shared memory, as a column's
+      // sums are finished together.
+      if (gridDim.y == 1) red[0][s][c] = t;
+      else partials[((size_t)blockIdx.y * NSUM + s) * n + gc] = t;
+    }
+  }
+  if (gridDim.y == 1) {
+    __syncthreads();
+    const int c = threadIdx.x, gc = blockIdx.x * CR_COLS + c;
+    if (c < CR_COLS && gc < n) {
+      double t[NSUM];
+#pragma unroll
+      for (int s = 0; s < NSUM; ++s) t[s] = red[0][s][c];
+      fin(gc, n, t);
     }
   }
 }
 
-__global__ void reduce_partials_kernel(const double *partials, int chunks, int total, double *out) {
+// Sums of the chunks and what follows from a column's sums.  Blocks of 32 columns: each
+// of the eight warps takes every eighth chunk (one thread per column waited for up
+// to 74 chunks one after the other), then the warps' sums are added in order.
+constexpr int RP_WARPS = 8;
+template <int NSUM, class Fin>
+__global__ void __launch_bounds__(32 * RP_WARPS)
+    reduce_partials_kernel(const double *__restrict__ partials, int chunks, int n, Fin fin) {
   pdl_enter();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  double t = 0.0;
-  for (int c = 0; c < chunks; ++c) t += partials[(size_t)c * total + i];
-  out[i] = t;
+  __shared__ double red[RP_WARPS][NSUM][32];
+  const int lane = threadIdx.x % 32, w = threadIdx.x / 32, c = blockIdx.x * 32 + lane;
+  double t[NSUM];
+#pragma unroll
+  for (int s = 0; s < NSUM; ++s) t[s] = 0.0;
+  if (c < n) {
+#pragma unroll 4
+    for (int i = w; i < chunks; i += RP_WARPS)
+#pragma unroll
+      for (int s = 0; s < NSUM; ++s) t[s] += partials[((size_t)i * NSUM + s) * n + c];
+  }
+#pragma unroll
+  for (int s = 0; s < NSUM; ++s) red[w][s][lane] = t[s];
+  __syncthreads();
+  if (w != 0 || c >= n) return;
+#pragma unroll
+  for (int s = 0; s < NSUM; ++s) {
+    t[s] = red[0][s][lane];
+#pragma unroll
+    for (int i = 1; i < RP_WARPS; ++i) t[s] += red[i][s][lane];
+  }
+  fin(c, n, t);
 }
 
 // Chunking of the rows: one wave of blocks over the SMs, CR_MAX_PER_SM blocks on
 // each or as many as `resident` (what an SM holds of the kernel) allows if that
 // is fewer; a grid larger than what is resident at once leaves a partial second
-// wave that costs a whole one.  Chunks of at least 64 rows.
-static void column_reduce_plan(int sm_count, int rows, int n, int resident, int *chunks, int *rows_per_chunk) {
+// wave that costs a whole one.  Chunks of at least 64 rows; where the kernel folds
+// into double as it goes (one_chunk), a single chunk up to CR_ONE_CHUNK rows: a second
+// launch for the chunks' sums takes longer than the rows.
+constexpr int CR_ONE_CHUNK = 256;
+static void column_reduce_plan(int sm_count, int rows, int n, int resident, bool one_chunk, int *chunks,
+                               int *rows_per_chunk) {
+  if (one_chunk && rows <= CR_ONE_CHUNK) {
+    *chunks = 1;
+    *rows_per_chunk = rows;
+    return;
+  }
   const int col_blocks = ceil_div(n, CR_COLS);
   const int target = max(1, min(resident, CR_MAX_PER_SM));
   int c = ceil_div(sm_count * target, col_blocks);
@@ -142,14 +198,6 @@ static void column_reduce_plan(int sm_count, int rows, int n, int resident, int 
   c = max(1, min(c, ceil_div(rows, 64)));
   *rows_per_chunk = ceil_div(ceil_div(rows, c), CR_LANES_Y) * CR_LANES_Y;
   *chunks = ceil_div(rows, *rows_per_chunk);
-}
-
-// Room for the partials of any kernel of the family (callers place their final
-// sums behind them in the same scratch request).
-static size_t column_reduce_partial_bytes(dlb_ctx *ctx, int nsum, int rows, int n) {
-  int chunks, rpc;
-  column_reduce_plan(ctx->sm_count, rows, n, 1 << 20, &chunks, &rpc);  // the most chunks any kernel's plan makes
-  return align_up((size_t)chunks * nsum * n * sizeof(double), 256);
 }
 
 // Lets `Kernel` take `bytes` of dynamic shared memory on the current device
@@ -167,11 +215,11 @@ static void kernel_shared_limit(size_t bytes) {
 
 // Blocks of one reduction kernel an SM of the current device holds.  The query
 // allocates nothing.
-template <int NSUM, class Op>
+template <int NSUM, class Op, class Fin>
 static int column_reduce_per_sm() {
   int blocks = CR_MAX_PER_SM;
-  kernel_shared_limit<column_reduce_kernel<NSUM, Op>>(column_reduce_shared_bytes<NSUM, Op>());
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, column_reduce_kernel<NSUM, Op>, CR_LANES_X * CR_LANES_Y,
+  kernel_shared_limit<column_reduce_kernel<NSUM, Op, Fin>>(column_reduce_shared_bytes<NSUM, Op>());
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, column_reduce_kernel<NSUM, Op, Fin>, CR_LANES_X * CR_LANES_Y,
                                                     column_reduce_shared_bytes<NSUM, Op>()) != cudaSuccess) {
     cudaGetLastError();
     blocks = CR_MAX_PER_SM;
@@ -179,24 +227,47 @@ static int column_reduce_per_sm() {
   return max(1, blocks);
 }
 
-template <int NSUM, class Op>
-static dlb_status column_reduce(dlb_ctx *ctx, Op op, int rows, int n, double *out) {
+// Whether the kernel folds into double as it goes when all rows are one chunk.
+template <class Op>
+static bool column_one_chunk(int n) {
+  return Op::DEPTH == 0 && (n & 3) == 0;
+}
+
+// fin(column, n, sums) runs once per column, in the last kernel of the reduction.  The
+// kernels that followed it (statistics, parameter gradients) were launches of 1.4 -
+// 2.4 us each for a few thousand values.
+template <int NSUM, class Op, class Fin>
+static dlb_status column_reduce(dlb_ctx *ctx, Op op, int rows, int n, Fin fin) {
   const int col_blocks = ceil_div(n, CR_COLS);
   static int per_sm_of[MAX_DEVICES] = {};  // 0: not asked yet on that device
   int &per_sm = per_sm_of[ctx->device];
-  if (per_sm == 0) per_sm = column_reduce_per_sm<NSUM, Op>();
+  if (per_sm == 0) per_sm = column_reduce_per_sm<NSUM, Op, Fin>();
   int chunks, rows_per_chunk;
-  column_reduce_plan(ctx->sm_count, rows, n, per_sm, &chunks, &rows_per_chunk);
-  void *scr = nullptr;
-  DLB_TRY(scratch(ctx, column_reduce_partial_bytes(ctx, NSUM, rows, n), &scr));
-  double *partials = static_cast<double *>(scr);
-  DLB_LAUNCH_KERNEL(ctx, (column_reduce_kernel<NSUM, Op>), dim3(col_blocks, chunks), CR_LANES_X * CR_LANES_Y, (column_reduce_shared_bytes<NSUM, Op>()), op, rows, n, rows_per_chunk, partials);
+  column_reduce_plan(ctx->sm_count, rows, n, per_sm, column_one_chunk<Op>(n), &chunks, &rows_per_chunk);
+  double *partials = nullptr;
+  if (chunks > 1) {
+    void *scr = nullptr;
+    DLB_TRY(scratch(ctx, (size_t)chunks * NSUM * n * sizeof(double), &scr));
+    partials = static_cast<double *>(scr);
+  }
+  DLB_LAUNCH_KERNEL(ctx, (column_reduce_kernel<NSUM, Op, Fin>), dim3(col_blocks, chunks), CR_LANES_X * CR_LANES_Y, (column_reduce_shared_bytes<NSUM, Op>()), op, rows, n, rows_per_chunk, partials, fin);
   DLB_LAUNCHED(ctx);
-  const int total = NSUM * n;
-  DLB_LAUNCH_KERNEL(ctx, reduce_partials_kernel, ceil_div(total, 256), 256, 0, partials, chunks, total, out);
-  DLB_LAUNCHED(ctx);
+  if (chunks > 1) {
+    DLB_LAUNCH_KERNEL(ctx, (reduce_partials_kernel<NSUM, Fin>), ceil_div(n, 32), 32 * RP_WARPS, 0, partials, chunks, n, fin);
+    DLB_LAUNCHED(ctx);
+  }
   return DLB_OK;
 }
+
+// Just the sums, [NSUM, n].
+template <int NSUM>
+struct StoreSums {
+  double *out;
+  __device__ void operator()(int c, int n, const double (&t)[NSUM]) const {
+#pragma unroll
+    for (int s = 0; s < NSUM; ++s) out[(size_t)s * n + c] = t[s];
+  }
+};
 
 // --- sum(z), sum(z^2) --------------------------------------------------------
 // The two read-only reductions use plain loads, four rows per thread in flight:
@@ -686,51 +757,64 @@ __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, ROWS_PER_SM)
   }
 }
 
-__global__ void brn_finalize_kernel(const double *__restrict__ sums, int n, float batch_scale,
-                                    float momentum, float eps, float r_max, float d_max,
-                                    dlb_brn_unit_arrays u) {
-  pdl_enter();
-  const int h = blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= n) return;
-  // fwp_mp.cpp L:4688-4717, in the reference's order: the running averages
-  // move first and r, d are taken from the moved averages.
-  const float mean = (float)sums[h] * batch_scale;
-  float mavg = u.mean_average[h];
-  mavg += momentum * (mean - mavg);
-  const float sigma = sqrtf((float)sums[n + h] * batch_scale - mean * mean + eps);
-  float savg = u.sigma_average[h];
-  savg += momentum * (sigma - savg);
-  u.mean[h] = mean;
-  u.sigma[h] = sigma;
-  u.mean_average[h] = mavg;
-  u.sigma_average[h] = savg;
-  u.r[h] = clipf(sigma / savg, 1.f / r_max, r_max);
-  u.d[h] = clipf((mean - mavg) / savg, -d_max, d_max);
-}
-
-__global__ void sums_to_grads_kernel(const double *__restrict__ sums, int n, float *d_gamma,
-                                     float *d_beta, int accumulate) {
-  pdl_enter();
-  const int h = blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= n) return;
-  const float g = (float)sums[h], b = (float)sums[n + h];
-  if (accumulate) {
-    d_gamma[h] += g;
-    d_beta[h] += b;
-  } else {
-    d_gamma[h] = g;
-    d_beta[h] = b;
+// Statistics of a unit from its sums.
+struct BrnFinalize {
+  float batch_scale, momentum, eps, r_max, d_max;
+  dlb_brn_unit_arrays u;
+  __device__ __forceinline__ void unit(int h, double sum, double sum_sq) const {
+    // fwp_mp.cpp L:4688-4717, in the reference's order: the running averages
+    // move first and r, d are taken from the moved averages.
+    const float mean = (float)sum * batch_scale;
+    float mavg = u.mean_average[h];
+    mavg += momentum * (mean - mavg);
+    const float sigma = sqrtf((float)sum_sq * batch_scale - mean * mean + eps);
+    float savg = u.sigma_average[h];
+    savg += momentum * (sigma - savg);
+    u.mean[h] = mean;
+    u.sigma[h] = sigma;
+    u.mean_average[h] = mavg;
+    u.sigma_average[h] = savg;
+    u.r[h] = clipf(sigma / savg, 1.f / r_max, r_max);
+    u.d[h] = clipf((mean - mavg) / savg, -d_max, d_max);
   }
-}
-
-__global__ void sums_to_bias_grad_kernel(const double *__restrict__ sums, int n, float *dbias,
-                                         int accumulate) {
+  __device__ void operator()(int h, int, const double (&t)[2]) const { unit(h, t[0], t[1]); }
+};
+__global__ void brn_finalize_kernel(const double *__restrict__ sums, int n, BrnFinalize f) {
   pdl_enter();
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= n) return;
-  if (accumulate) dbias[h] += (float)sums[h];
-  else dbias[h] = (float)sums[h];
+  if (h < n) f.unit(h, sums[h], sums[n + h]);
 }
+
+// Gradients of gamma and beta of a unit from the first two of its backward sums.
+struct BrnGrads {
+  float *d_gamma, *d_beta;
+  int accumulate;
+  __device__ __forceinline__ void unit(int h, double g, double b) const {
+    d_gamma[h] = accumulate ? d_gamma[h] + (float)g : (float)g;
+    d_beta[h] = accumulate ? d_beta[h] + (float)b : (float)b;
+  }
+};
+struct StoreSumsAndGrads {
+  StoreSums<4> store;
+  BrnGrads grads;
+  __device__ void operator()(int c, int n, const double (&t)[4]) const {
+    store(c, n, t);
+    grads.unit(c, t[0], t[1]);
+  }
+};
+__global__ void sums_to_grads_kernel(const double *__restrict__ sums, int n, BrnGrads grads) {
+  pdl_enter();
+  const int h = blockIdx.x * blockDim.x + threadIdx.x;
+  if (h < n) grads.unit(h, sums[h], sums[n + h]);
+}
+
+struct BiasGrad {
+  float *dbias;
+  int accumulate;
+  __device__ void operator()(int h, int, const double (&t)[1]) const {
+    dbias[h] = accumulate ? dbias[h] + (float)t[0] : (float)t[0];
+  }
+};
 
 // Adds the block's values into *sum with one atomic: the double atomics of a grid
 // queue on one address, and one per block (or per warp) of a large grid took most of
@@ -865,6 +949,30 @@ __global__ void loss_delta_softmax_ce_kernel(const float *__restrict__ q, const 
   block_add(local, loss_sum);
 }
 
+// dlb_brn_forward_sums and dlb_brn_forward_finalize of a single rank.
+dlb_status brn_forward_statistics(dlb_ctx *ctx, const float *Z, int rows, int global_rows, int n_units, float momentum,
+                                  float epsilon, float r_max, float d_max, const dlb_brn_unit_arrays *u) {
+  DLB_REQUIRE(ctx && Z && u && rows > 0 && n_units > 0, "brn_forward_statistics");
+  return column_reduce<2>(ctx, SumSqOp{Z, n_units}, rows, n_units,
+                          BrnFinalize{1.f / (float)global_rows, momentum, epsilon, r_max, d_max, *u});
+}
+
+// dlb_activation_backward of a normalised layer; with d_gamma, the parameter gradients
+// too (added to what is there).
+dlb_status brn_activation_backward(dlb_ctx *ctx, float *dA, const float *Z, const float *A,
+                                   const dlb_brn_unit_arrays *u, int af, int rows, int n_units, double *sums,
+                                   float *d_gamma, float *d_beta) {
+  DLB_REQUIRE(sums, "dlb_activation_backward: sums required with batch renormalization");
+  DLB_REQUIRE((n_units & 3) || ((reinterpret_cast<uintptr_t>(dA) | reinterpret_cast<uintptr_t>(Z) |
+                                 reinterpret_cast<uintptr_t>(A)) & 15) == 0,
+              "dlb_activation_backward: tensors must be 16-byte aligned");
+  return with_af(af, [&](auto AF) {
+    const ActBackwardOp<true, decltype(AF)::value> op{dA, Z, A, brn_ptrs(u), af, n_units};
+    if (!d_gamma) return column_reduce<4>(ctx, op, rows, n_units, StoreSums<4>{sums});
+    return column_reduce<4>(ctx, op, rows, n_units, StoreSumsAndGrads{{sums}, {d_gamma, d_beta, 1}});
+  });
+}
+
 }  // namespace dlb
 
 using namespace dlb;
@@ -887,7 +995,7 @@ dlb_status dlb_brn_forward_sums(dlb_ctx *ctx, const float *Z, int rows, int n_un
   DLB_REQUIRE(ctx && Z && sums && rows > 0 && n_units > 0, "dlb_brn_forward_sums");
   DLB_REQUIRE((n_units & 3) || (reinterpret_cast<uintptr_t>(Z) & 15) == 0,
               "dlb_brn_forward_sums: Z must be 16-byte aligned");
-  return column_reduce<2>(ctx, SumSqOp{Z, n_units}, rows, n_units, sums);
+  return column_reduce<2>(ctx, SumSqOp{Z, n_units}, rows, n_units, StoreSums<2>{sums});
 }
 
 dlb_status dlb_brn_forward_finalize(dlb_ctx *ctx, const double *sums, int global_rows,
@@ -896,7 +1004,7 @@ dlb_status dlb_brn_forward_finalize(dlb_ctx *ctx, const double *sums, int global
   DLB_REQUIRE(ctx && sums && u && global_rows > 0 && n_units > 0, "dlb_brn_forward_finalize");
   DLB_REQUIRE(u->mean && u->sigma && u->mean_average && u->sigma_average && u->r && u->d,
               "dlb_brn_forward_finalize: null unit array");
-  DLB_LAUNCH_KERNEL(ctx, brn_finalize_kernel, ceil_div(n_units, 256), 256, 0, sums, n_units, 1.f / (float)global_rows, momentum, epsilon, r_max, d_max, *u);
+  DLB_LAUNCH_KERNEL(ctx, brn_finalize_kernel, ceil_div(n_units, 256), 256, 0, sums, n_units, BrnFinalize{1.f / (float)global_rows, momentum, epsilon, r_max, d_max, *u});
   DLB_LAUNCHED(ctx);
   return DLB_OK;
 }
@@ -976,16 +1084,7 @@ dlb_status dlb_activation_backward(dlb_ctx *ctx, float *dA, const float *Z, cons
                                    const dlb_brn_unit_arrays *u, int af, int rows, int n_units,
                                    double *sums) {
   DLB_REQUIRE(ctx && dA && Z && A && rows > 0 && n_units > 0, "dlb_activation_backward");
-  if (u) {
-    DLB_REQUIRE(sums, "dlb_activation_backward: sums required with batch renormalization");
-    DLB_REQUIRE((n_units & 3) || ((reinterpret_cast<uintptr_t>(dA) | reinterpret_cast<uintptr_t>(Z) |
-                                   reinterpret_cast<uintptr_t>(A)) & 15) == 0,
-                "dlb_activation_backward: tensors must be 16-byte aligned");
-    return with_af(af, [&](auto AF) {
-      return column_reduce<4>(ctx, ActBackwardOp<true, decltype(AF)::value>{dA, Z, A, brn_ptrs(u), af, n_units}, rows,
-                              n_units, sums);
-    });
-  }
+  if (u) return brn_activation_backward(ctx, dA, Z, A, u, af, rows, n_units, sums, nullptr, nullptr);
   const size_t total = (size_t)rows * n_units;
   const bool vec4 = (total % 4 == 0) && ((reinterpret_cast<uintptr_t>(dA) & 15) == 0) &&
                     ((reinterpret_cast<uintptr_t>(Z) & 15) == 0) &&
@@ -1031,7 +1130,7 @@ dlb_status brn_backward_apply_impl(dlb_ctx *ctx, float *delta, float *delta_lo, 
 dlb_status dlb_brn_backward_param_grads(dlb_ctx *ctx, const double *sums, int n_units,
                                         float *d_gamma, float *d_beta, int accumulate) {
   DLB_REQUIRE(ctx && sums && d_gamma && d_beta && n_units > 0, "dlb_brn_backward_param_grads");
-  DLB_LAUNCH_KERNEL(ctx, sums_to_grads_kernel, ceil_div(n_units, 256), 256, 0, sums, n_units, d_gamma, d_beta, accumulate);
+  DLB_LAUNCH_KERNEL(ctx, sums_to_grads_kernel, ceil_div(n_units, 256), 256, 0, sums, n_units, BrnGrads{d_gamma, d_beta, accumulate});
   DLB_LAUNCHED(ctx);
   return DLB_OK;
 }
@@ -1069,14 +1168,7 @@ namespace dlb {
 // Column sum of delta into the bias gradient (used by dlb_fc_weight_gradient).
 dlb_status bias_gradient(dlb_ctx *ctx, const float *delta, int rows, int n, float *dbias,
                          int accumulate) {
-  void *scr = nullptr;
-  const size_t partial_bytes = column_reduce_partial_bytes(ctx, 1, rows, n);
-  DLB_TRY(scratch(ctx, partial_bytes + (size_t)n * sizeof(double), &scr));
-  double *out = reinterpret_cast<double *>(static_cast<char *>(scr) + partial_bytes);
-  DLB_TRY(column_reduce<1>(ctx, SumOp{delta, n}, rows, n, out));
-  DLB_LAUNCH_KERNEL(ctx, sums_to_bias_grad_kernel, ceil_div(n, 256), 256, 0, out, n, dbias, accumulate);
-  DLB_LAUNCHED(ctx);
-  return DLB_OK;
+  return column_reduce<1>(ctx, SumOp{delta, n}, rows, n, BiasGrad{dbias, accumulate});
 }
 }  // namespace dlb
 
@@ -1260,7 +1352,7 @@ static dlb_status noalloc_setup(NoallocDevice *d, int dev) {
   int sms = 0;
   DLB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   DLB_REQUIRE(ptr && sms > 0, "dlb_brn_forward_sums_noalloc: device set-up");
-  d->per_sm = column_reduce_per_sm<2, SumSqOp>();
+  d->per_sm = column_reduce_per_sm<2, SumSqOp, StoreSums<2>>();
   d->sm_count = sms;
   d->partials = ptr;
   return DLB_OK;
@@ -1300,7 +1392,7 @@ extern "C" dlb_status dlb_brn_forward_sums_noalloc(const float *Z, int rows, int
   // occupancy figure), so both add the same partial sums in the same order.
   const int col_blocks = ceil_div(n_units, CR_COLS);
   int chunks, rows_per_chunk;
-  column_reduce_plan(dev->sm_count, rows, n_units, dev->per_sm, &chunks, &rows_per_chunk);
+  column_reduce_plan(dev->sm_count, rows, n_units, dev->per_sm, column_one_chunk<SumSqOp>(n_units), &chunks, &rows_per_chunk);
   const size_t need = (size_t)chunks * 2 * (size_t)n_units;
   if (need > (size_t)DLB_NOALLOC_SCRATCH_DOUBLES) {
     set_error("dlb_brn_forward_sums_noalloc: %d rows x %d units need %zu partial sums, the built-in "
@@ -1309,13 +1401,15 @@ extern "C" dlb_status dlb_brn_forward_sums_noalloc(const float *Z, int rows, int
     return DLB_ERR_INVALID;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  column_reduce_kernel<2, SumSqOp><<<dim3(col_blocks, chunks), CR_LANES_X * CR_LANES_Y,
-                                     column_reduce_shared_bytes<2, SumSqOp>(), s>>>(
-      SumSqOp{Z, n_units}, rows, n_units, rows_per_chunk, dev->partials);
+  const StoreSums<2> store{sums};
+  column_reduce_kernel<2, SumSqOp, StoreSums<2>><<<dim3(col_blocks, chunks), CR_LANES_X * CR_LANES_Y,
+                                                   column_reduce_shared_bytes<2, SumSqOp>(), s>>>(
+      SumSqOp{Z, n_units}, rows, n_units, rows_per_chunk, dev->partials, store);
   DLB_CUDA(cudaGetLastError());
-  const int total = 2 * n_units;
-  reduce_partials_kernel<<<ceil_div(total, 256), 256, 0, s>>>(dev->partials, chunks, total, sums);
-  DLB_CUDA(cudaGetLastError());
+  if (chunks > 1) {
+    reduce_partials_kernel<2, StoreSums<2>><<<ceil_div(n_units, 32), 32 * RP_WARPS, 0, s>>>(dev->partials, chunks, n_units, store);
+    DLB_CUDA(cudaGetLastError());
+  }
   return DLB_OK;
 }
 

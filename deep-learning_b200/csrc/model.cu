@@ -388,10 +388,10 @@ dlb_status ensure_batch(dlb_model *m, size_t rows) {
     DLB_TRY(dev_alloc(m, &m->target_rows, T * rows * n_out(m), false));
   }
   if (!m->loss_sum) {
-    DLB_TRY(dlb_malloc(m->ctx, reinterpret_cast<void **>(&m->loss_sum), sizeof(double)));
-    DLB_TRY(dlb_memset(m->ctx, m->loss_sum, 0, sizeof(double)));
-    DLB_TRY(dlb_malloc(m->ctx, reinterpret_cast<void **>(&m->accu_sum), sizeof(double)));
-    DLB_TRY(dlb_memset(m->ctx, m->accu_sum, 0, sizeof(double)));
+    // One allocation: cleared and copied together.
+    DLB_TRY(dlb_malloc(m->ctx, reinterpret_cast<void **>(&m->loss_sum), 2 * sizeof(double)));
+    DLB_TRY(dlb_memset(m->ctx, m->loss_sum, 0, 2 * sizeof(double)));
+    m->accu_sum = m->loss_sum + 1;
   }
   m->alloc_rows = rows;
   m->planes_rows = 0;  // new buffers: choose_planes decides again
@@ -608,6 +608,9 @@ dlb_status norm_statistics(dlb_model *m, LayerRT &l, const float *in, int B, dlb
   const int Bg = (int)(m->global_rows ? m->global_rows : (size_t)B);
   const int n = (int)l.norm_units;
   *u = unit_arrays(m, l, 0);
+  if (dlb_comm_world(m->ctx) == 1)
+    return brn_forward_statistics(m->ctx, in, B, Bg, n, m->hp.normalization_momentum_average,
+                                  m->hp.normalization_epsilon, r_max_of(m, l), d_max_of(m, l), u);
   DLB_TRY(dlb_brn_forward_sums(m->ctx, in, B, n, l.fwd_sums));
   DLB_TRY(dlb_allreduce_f64(m->ctx, l.fwd_sums, 2 * (size_t)n));
   return dlb_brn_forward_finalize(m->ctx, l.fwd_sums, Bg, n, m->hp.normalization_momentum_average,
@@ -622,9 +625,8 @@ dlb_status norm_backward(dlb_model *m, LayerRT &l, float *e, float *e_lo, const 
   const int Bg = (int)(m->global_rows ? m->global_rows : (size_t)B);
   const int n = (int)l.norm_units;
   dlb_brn_unit_arrays u = unit_arrays(m, l, 0);
-  DLB_TRY(dlb_activation_backward(m->ctx, e, in, act, &u, af, B, n, l.bwd_sums));
-  DLB_TRY(dlb_brn_backward_param_grads(m->ctx, l.bwd_sums, n, m->grads + gamma_index(m, l),
-                                       m->grads + beta_index(m, l), 1));
+  DLB_TRY(brn_activation_backward(m->ctx, e, in, act, &u, af, B, n, l.bwd_sums, m->grads + gamma_index(m, l),
+                                  m->grads + beta_index(m, l)));
   DLB_TRY(dlb_allreduce_f64(m->ctx, l.bwd_sums + 2 * (size_t)n, 2 * (size_t)n));
   return dlb_brn_backward_apply(m->ctx, e, e_lo, in, &u, l.bwd_sums, Bg, B, n);
 }
@@ -1247,7 +1249,6 @@ dlb_status dlb_model_destroy(dlb_model *m) {
   if (m->loss_host) dlb_host_free(m->loss_host);
   for (cudaEvent_t e : m->loss_ready)
     if (e) cudaEventDestroy(e);
-  if (m->accu_sum) dlb_free(m->ctx, m->accu_sum);
   if (m->ones) dlb_free(m->ctx, m->ones);
   if (m->zeros) dlb_free(m->ctx, m->zeros);
   delete m->workers;
@@ -2463,8 +2464,7 @@ dlb_status dlb_model_get_constraint_recurrent_weight(dlb_model *m, size_t layer,
 dlb_status dlb_model_reset_loss(dlb_model *m) {
   DLB_REQUIRE(m, "null");
   m->loss_rows = 0;
-  if (m->loss_sum) DLB_TRY(dlb_memset(m->ctx, m->loss_sum, 0, sizeof(double)));
-  if (m->accu_sum) DLB_TRY(dlb_memset(m->ctx, m->accu_sum, 0, sizeof(double)));
+  if (m->loss_sum) DLB_TRY(dlb_memset(m->ctx, m->loss_sum, 0, 2 * sizeof(double)));
   return DLB_OK;
 }
 
@@ -2526,11 +2526,14 @@ dlb_status dlb_model_compute_loss(dlb_model *m, size_t rows, const float *const 
 // Driver::evalt sets it, drivers/driver.cpp L:95-99).
 dlb_status dlb_model_get_accuracy(dlb_model *m, double *accuracy) {
   DLB_REQUIRE(m && accuracy && m->accu_sum, "get_accuracy");
-  void *scr = nullptr;
-  DLB_TRY(scratch(m->ctx, sizeof(double), &scr));
-  double *tmp = static_cast<double *>(scr);
-  DLB_TRY(dlb_memcpy_d2d(m->ctx, tmp, m->accu_sum, sizeof(double)));
-  DLB_TRY(dlb_allreduce_f64(m->ctx, tmp, 1));
+  double *tmp = m->accu_sum;
+  if (dlb_comm_world(m->ctx) > 1) {
+    void *scr = nullptr;
+    DLB_TRY(scratch(m->ctx, sizeof(double), &scr));
+    tmp = static_cast<double *>(scr);
+    DLB_TRY(dlb_memcpy_d2d(m->ctx, tmp, m->accu_sum, sizeof(double)));
+    DLB_TRY(dlb_allreduce_f64(m->ctx, tmp, 1));
+  }
   double s = 0.0;
   DLB_TRY(dlb_memcpy_d2h(m->ctx, &s, tmp, sizeof(double)));
   const double trials = (double)m->loss_rows * (double)dlb_comm_world(m->ctx) *
@@ -2543,11 +2546,14 @@ dlb_status dlb_model_get_accuracy(dlb_model *m, double *accuracy) {
 // L:158-221), over every rank's rows.
 dlb_status dlb_model_get_loss(dlb_model *m, double *loss) {
   DLB_REQUIRE(m && loss && m->loss_sum, "get_loss");
-  void *scr = nullptr;
-  DLB_TRY(scratch(m->ctx, sizeof(double), &scr));
-  double *tmp = static_cast<double *>(scr);
-  DLB_TRY(dlb_memcpy_d2d(m->ctx, tmp, m->loss_sum, sizeof(double)));
-  DLB_TRY(dlb_allreduce_f64(m->ctx, tmp, 1));
+  double *tmp = m->loss_sum;
+  if (dlb_comm_world(m->ctx) > 1) {
+    void *scr = nullptr;
+    DLB_TRY(scratch(m->ctx, sizeof(double), &scr));
+    tmp = static_cast<double *>(scr);
+    DLB_TRY(dlb_memcpy_d2d(m->ctx, tmp, m->loss_sum, sizeof(double)));
+    DLB_TRY(dlb_allreduce_f64(m->ctx, tmp, 1));
+  }
   double s = 0.0;
   DLB_TRY(dlb_memcpy_d2h(m->ctx, &s, tmp, sizeof(double)));
   const double rows = (double)m->loss_rows * (double)dlb_comm_world(m->ctx);
@@ -2571,9 +2577,12 @@ static dlb_status loss_capture(dlb_model *m, int slot) {
   // pass keeps it.
   double *dev = m->loss_tmp + 2 * slot, *host = m->loss_host + 2 * slot;
   const size_t n = m->training_accuracy ? 2 : 1;
-  DLB_TRY(dlb_memcpy_d2d(m->ctx, dev, m->loss_sum, sizeof(double)));
-  if (n == 2) DLB_TRY(dlb_memcpy_d2d(m->ctx, dev + 1, m->accu_sum, sizeof(double)));
-  DLB_TRY(dlb_allreduce_f64(m->ctx, dev, n));
+  if (dlb_comm_world(m->ctx) == 1) {
+    dev = m->loss_sum;  // the counter lies behind it
+  } else {
+    DLB_TRY(dlb_memcpy_d2d(m->ctx, dev, m->loss_sum, n * sizeof(double)));
+    DLB_TRY(dlb_allreduce_f64(m->ctx, dev, n));
+  }
   DLB_CUDA(cudaMemcpyAsync(host, dev, n * sizeof(double), cudaMemcpyDeviceToHost, m->ctx->stream));
   DLB_CUDA(cudaEventRecord(m->loss_ready[slot], m->ctx->stream));
   m->loss_rows_at[slot] = m->loss_rows;

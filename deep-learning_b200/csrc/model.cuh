@@ -141,7 +141,7 @@ struct dlb_model {
   int propagation = DLB_PROPAGATION_TRAINING;
   int accu_fn = DLB_ACCU_DISTANCE;   // v1/learner/model.hpp L:157
   float accu_var = 0.49f;            // L:3019
-  double *accu_sum = nullptr;
+  double *accu_sum = nullptr;        // behind loss_sum
   bool training_accuracy = false;    // compute_error counts the accuracy too (one more pass over the outputs)
   float *ones = nullptr, *zeros = nullptr;
   size_t const_units = 0;
