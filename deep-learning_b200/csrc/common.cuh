@@ -450,6 +450,14 @@ dlb_status brn_activation_backward(dlb_ctx *ctx, float *dA, const float *Z, cons
                                    const dlb_brn_unit_arrays *u, int af, int rows, int n_units, double *sums,
                                    float *d_gamma, float *d_beta);
 
+// dlb_shakedrop_backward_window that also copies d to `shortcut` (if any; equal widths).
+dlb_status shakedrop_backward_shortcut(dlb_ctx *ctx, const float *d, int width_d, int first, const uint8_t *row_mask,
+                                       const float *noise, float *delta, float *delta_lo, float *shortcut, int rows,
+                                       int width);
+// dlb_activation_backward without normalization, and the planes of the result.
+dlb_status activation_backward_planes(dlb_ctx *ctx, float *dA, float *dA_lo, const float *Z, const float *A, int af,
+                                      int rows, int n_units);
+
 // All time steps of an LSTM layer in one launch (lstm_walk.cu).  done: whether this
 // was the faster way and has been enqueued; the step entry points otherwise.
 // Backward: dH [T, rows, C] gets the recurrent part added.

@@ -669,9 +669,7 @@ dlb_status dlb_fc_backward_input_derivative(dlb_ctx *ctx, const float *delta, co
     }
   }
   DLB_TRY(dlb_fc_backward_input(ctx, delta, delta_lo, W, W_lo, dX, rows, n_in, n_out));
-  DLB_TRY(dlb_activation_backward(ctx, dX, Z_below, A_below, nullptr, af_below, rows, n_in, nullptr));
-  if (dX_lo) DLB_TRY(dlb_split_planes_2d(ctx, dX, dX_lo, rows, n_in));
-  return DLB_OK;
+  return activation_backward_planes(ctx, dX, dX_lo, Z_below, A_below, af_below, rows, n_in);
 }
 
 dlb_status dlb_fc_weight_gradient(dlb_ctx *ctx, const float *delta, const float *delta_lo,

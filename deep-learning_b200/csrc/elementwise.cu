@@ -44,7 +44,8 @@ constexpr size_t column_reduce_shared_bytes() {
   return ring > fold ? ring : fold;
 }
 
-template <int NSUM, class Op, class Fin>
+// ONE: all rows in one chunk by plain loads, folded into double every Op::IN_FLIGHT rows.
+template <int NSUM, class Op, class Fin, bool ONE>
 __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, Op::MIN_BLOCKS)
     column_reduce_kernel(Op op, int rows, int n, int rows_per_chunk, double *partials, Fin fin) {
   pdl_enter();
@@ -58,7 +59,7 @@ __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, Op::MIN_BLOCKS)
   for (int s = 0; s < NSUM; ++s)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[s][j] = 0.f;
-  double whole[NSUM][4] = {};
+  double whole[ONE ? NSUM : 1][4] = {};
 
   if (col < n) {
     if ((n & 3) == 0) {
@@ -76,8 +77,7 @@ __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, Op::MIN_BLOCKS)
         // iteration by plain loads, all of them sent before the first is used.
         constexpr int U = Op::IN_FLIGHT;
         for (int r = r0 + ty; r < r1; r += U * CR_LANES_Y) {
-          if (gridDim.y == 1) {
-            // All rows in one chunk: fp32 sums of four rows, the rest in double.
+          if constexpr (ONE) {
 #pragma unroll
             for (int s = 0; s < NSUM; ++s)
 #pragma unroll
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, Op::MIN_BLOCKS)
 #pragma unroll
   for (int s = 0; s < NSUM; ++s)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) red[ty][s][tx * 4 + j] = whole[s][j] + (double)acc[s][j];
+    for (int j = 0; j < 4; ++j) red[ty][s][tx * 4 + j] = (ONE ? whole[ONE ? s : 0][j] : 0.0) + (double)acc[s][j];
   __syncthreads();
   // 256 threads fold NSUM*128 columns.
   for (int i = threadIdx.x; i < NSUM * CR_COLS; i += CR_LANES_X * CR_LANES_Y) {
@@ -218,8 +218,8 @@ static void kernel_shared_limit(size_t bytes) {
 template <int NSUM, class Op, class Fin>
 static int column_reduce_per_sm() {
   int blocks = CR_MAX_PER_SM;
-  kernel_shared_limit<column_reduce_kernel<NSUM, Op, Fin>>(column_reduce_shared_bytes<NSUM, Op>());
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, column_reduce_kernel<NSUM, Op, Fin>, CR_LANES_X * CR_LANES_Y,
+  kernel_shared_limit<column_reduce_kernel<NSUM, Op, Fin, false>>(column_reduce_shared_bytes<NSUM, Op>());
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, column_reduce_kernel<NSUM, Op, Fin, false>, CR_LANES_X * CR_LANES_Y,
                                                     column_reduce_shared_bytes<NSUM, Op>()) != cudaSuccess) {
     cudaGetLastError();
     blocks = CR_MAX_PER_SM;
@@ -250,7 +250,16 @@ static dlb_status column_reduce(dlb_ctx *ctx, Op op, int rows, int n, Fin fin) {
     DLB_TRY(scratch(ctx, (size_t)chunks * NSUM * n * sizeof(double), &scr));
     partials = static_cast<double *>(scr);
   }
-  DLB_LAUNCH_KERNEL(ctx, (column_reduce_kernel<NSUM, Op, Fin>), dim3(col_blocks, chunks), CR_LANES_X * CR_LANES_Y, (column_reduce_shared_bytes<NSUM, Op>()), op, rows, n, rows_per_chunk, partials, fin);
+  const dim3 grid(col_blocks, chunks);
+  constexpr size_t shared = column_reduce_shared_bytes<NSUM, Op>();
+  bool launched = false;
+  if constexpr (Op::DEPTH == 0)
+    if (chunks == 1 && column_one_chunk<Op>(n)) {
+      DLB_LAUNCH_KERNEL(ctx, (column_reduce_kernel<NSUM, Op, Fin, true>), grid, CR_LANES_X * CR_LANES_Y, shared, op, rows, n, rows_per_chunk, partials, fin);
+      launched = true;
+    }
+  if (!launched)
+    DLB_LAUNCH_KERNEL(ctx, (column_reduce_kernel<NSUM, Op, Fin, false>), grid, CR_LANES_X * CR_LANES_Y, shared, op, rows, n, rows_per_chunk, partials, fin);
   DLB_LAUNCHED(ctx);
   if (chunks > 1) {
     DLB_LAUNCH_KERNEL(ctx, (reduce_partials_kernel<NSUM, Fin>), ceil_div(n, 32), 32 * RP_WARPS, 0, partials, chunks, n, fin);
@@ -949,6 +958,213 @@ __global__ void loss_delta_softmax_ce_kernel(const float *__restrict__ q, const 
   block_add(local, loss_sum);
 }
 
+// ---------------------------------------------------------------------------
+// Element-wise producers of a [rows, n] operand (n % 4 == 0, 16-byte aligned) that
+// write the operand's planes and range statistics in the same pass.
+//
+// Grid (column blocks, row chunks); a thread owns four columns and has QR_AHEAD of its
+// rows in flight.  Op::load reads a quad's inputs, Op::use stores what belongs to it
+// and returns the operand's values.  The passes over the tensor are what such a
+// kernel costs (2048 x 2048: 10 us each in L2), so the split that followed it, one
+// read and one write more, is worth the statistics here.  2048 x 2048 activation with
+// UOut: 12.2 + 9.5 us with a split of its own, 12.9 here; 2048 x 1024 residual sum 14.2 +
+// 6.5 and 12.2, ShakeDrop error with the shortcut's copy 13.5 + 6.5 + 8.5 and 8.9.
+// ---------------------------------------------------------------------------
+
+constexpr int QR_AHEAD = 4;
+
+template <bool PLANES, class Op>
+__global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, 4)
+    quad_rows_kernel(const __grid_constant__ Op op, int rows, int n, int rows_per_chunk, PlaneSink sink) {
+  pdl_enter();
+  __shared__ unsigned fold[PLANES ? CR_LANES_Y * CR_COLS : 1];
+  const int tx = threadIdx.x % CR_LANES_X, ty = threadIdx.x / CR_LANES_X;
+  const int col = blockIdx.x * CR_COLS + tx * 4;
+  const bool live = col < n;
+  LineTracker track;
+  const float scale = PLANES ? sink_scale(sink) : 1.f;
+  if (live) {
+    const int r1 = min(rows, (int)(blockIdx.y + 1) * rows_per_chunk);
+    const typename Op::Cols cols = op.columns(col);
+    for (int r0 = blockIdx.y * rows_per_chunk + ty; r0 < r1; r0 += QR_AHEAD * CR_LANES_Y) {
+      typename Op::In in[QR_AHEAD];
+#pragma unroll
+      for (int i = 0; i < QR_AHEAD; ++i) {
+        const int r = r0 + i * CR_LANES_Y;
+        if (r < r1) in[i] = op.load(r, col, (size_t)r * n + col);
+      }
+#pragma unroll
+      for (int i = 0; i < QR_AHEAD; ++i) {
+        const int r = r0 + i * CR_LANES_Y;
+        if (r < r1) {
+          const size_t at = (size_t)r * n + col;
+          const float4 v = op.use(in[i], cols, at);
+          const float a[4] = {v.x, v.y, v.z, v.w};
+          if (PLANES) {
+            sink_store4(sink, at, a, scale);
+            track.row(sink, r, a);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) track.all = max(track.all, abs_bits(a[j]));
+          }
+        }
+      }
+    }
+  }
+  if (PLANES) track.finish(sink, fold, tx, ty, CR_LANES_Y, blockIdx.x * CR_COLS, n, live);
+  else if (sink.slot && live) amax_commit(reinterpret_cast<unsigned *>(sink.slot) + SLOT_AMAX, track.all);
+}
+
+__device__ __forceinline__ float4 load4(const float *p, size_t at) {
+  return __ldg(reinterpret_cast<const float4 *>(p + at));
+}
+__device__ __forceinline__ void store4(float *p, size_t at, float4 v) { *reinterpret_cast<float4 *>(p + at) = v; }
+
+// A = dropout(f(Z)) without normalization.
+template <int AF>
+struct ActivationRows {
+  const float *Z;
+  float *A;
+  DropoutDev dp;
+  struct In {
+    float4 z, noise;
+  };
+  struct Cols {
+    float4 keep;  // Bernoulli: 0 drops the unit (a select, not a product)
+  };
+  __device__ Cols columns(int col) const {
+    float k[4] = {1.f, 1.f, 1.f, 1.f};
+    if (dp.type == DLB_DROPOUT_BERNOULLI || dp.type == DLB_DROPOUT_BERNOULLI_INVERTED) {
+      const float kept = dp.type == DLB_DROPOUT_BERNOULLI_INVERTED ? dp.scale : 1.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) k[j] = dp.mask[col + j] ? kept : 0.f;
+    } else if (dp.type == DROPOUT_INFERENCE_SCALE) {
+      return {make_float4(dp.scale, dp.scale, dp.scale, dp.scale)};
+    }
+    return {make_float4(k[0], k[1], k[2], k[3])};
+  }
+  __device__ In load(int, int, size_t at) const {
+    In in;
+    in.z = load4(Z, at);
+    if (dp.type == DLB_DROPOUT_UOUT) in.noise = load4(dp.noise, at);
+    return in;
+  }
+  __device__ float one(float z, float noise, float keep) const {
+    const float a = af_fire(AF, z);
+    if (dp.type == DLB_DROPOUT_UOUT) return a + a * noise;
+    if (dp.type == DROPOUT_INFERENCE_SCALE) return a * keep;
+    return keep == 0.f ? 0.f : a * keep;
+  }
+  __device__ float4 use(const In &in, const Cols &c, size_t at) const {
+    const float4 a = make_float4(one(in.z.x, in.noise.x, c.keep.x), one(in.z.y, in.noise.y, c.keep.y),
+                                 one(in.z.z, in.noise.z, c.keep.z), one(in.z.w, in.noise.w, c.keep.w));
+    store4(A, at, a);
+    return a;
+  }
+};
+
+struct NoCols {};
+
+// dA *= f'(Z, A).
+template <int AF>
+struct DerivativeRows {
+  float *dA;
+  const float *Z, *A;
+  struct In {
+    float4 e, z, a;
+  };
+  using Cols = NoCols;
+  __device__ Cols columns(int) const { return {}; }
+  __device__ In load(int, int, size_t at) const {
+    return {*reinterpret_cast<const float4 *>(dA + at), load4(Z, at), load4(A, at)};
+  }
+  __device__ float4 use(const In &in, const Cols &, size_t at) const {
+    const float4 e = make_float4(in.e.x * af_derive(AF, in.z.x, in.a.x), in.e.y * af_derive(AF, in.z.y, in.a.y),
+                                 in.e.z * af_derive(AF, in.z.z, in.a.z), in.e.w * af_derive(AF, in.z.w, in.a.w));
+    store4(dA, at, e);
+    return e;
+  }
+};
+
+// out = x + block, the block's flagged rows times their draws first (and stored so).
+struct ResidualRows {
+  const float *x;
+  float *block;
+  const uint8_t *row_mask;
+  const float *noise;
+  float *out;
+  struct In {
+    float4 x, o, k;
+    bool flagged;
+  };
+  using Cols = NoCols;
+  __device__ Cols columns(int) const { return {}; }
+  __device__ In load(int r, int, size_t at) const {
+    In in;
+    in.x = load4(x, at);
+    in.o = *reinterpret_cast<const float4 *>(block + at);
+    in.flagged = row_mask && row_mask[r];
+    if (in.flagged) in.k = load4(noise, at);
+    return in;
+  }
+  __device__ float4 use(const In &in, const Cols &, size_t at) const {
+    float4 o = in.o;
+    if (in.flagged) {
+      o.x *= in.k.x; o.y *= in.k.y; o.z *= in.k.z; o.w *= in.k.w;
+      store4(block, at, o);
+    }
+    const float4 v = make_float4(in.x.x + o.x, in.x.y + o.y, in.x.z + o.z, in.x.w + o.w);
+    store4(out, at, v);
+    return v;
+  }
+};
+
+// delta = d, the flagged rows times their draws; shortcut = d where the widths agree.
+struct ShakeDropRows {
+  const float *d;
+  int ld_d, first;
+  const uint8_t *row_mask;
+  const float *noise;
+  float *delta, *shortcut;
+  struct In {
+    float4 d, k;
+    bool flagged;
+  };
+  using Cols = NoCols;
+  __device__ Cols columns(int) const { return {}; }
+  __device__ In load(int r, int col, size_t at) const {
+    In in;
+    in.d = load4(d, (size_t)r * ld_d + first + col);
+    in.flagged = row_mask && row_mask[r];
+    if (in.flagged) in.k = load4(noise, at);
+    return in;
+  }
+  __device__ float4 use(const In &in, const Cols &, size_t at) const {
+    float4 v = in.d;
+    if (shortcut) store4(shortcut, at, v);
+    if (in.flagged) v.x *= in.k.x, v.y *= in.k.y, v.z *= in.k.z, v.w *= in.k.w;
+    store4(delta, at, v);
+    return v;
+  }
+};
+
+static bool quads(int n, std::initializer_list<const void *> ptrs) {
+  uintptr_t all = 0;
+  for (const void *p : ptrs) all |= reinterpret_cast<uintptr_t>(p);
+  return n % 4 == 0 && (all & 15) == 0;
+}
+
+template <class Op>
+static dlb_status quad_rows(dlb_ctx *ctx, const Op &op, int rows, int n, const PlaneSink &sink) {
+  int chunks, rpc;
+  rows_plan(ctx, rows, n, &chunks, &rpc);
+  const dim3 grid(ceil_div(n, CR_COLS), chunks);
+  if (sink.hi) DLB_LAUNCH_KERNEL(ctx, (quad_rows_kernel<true, Op>), grid, CR_LANES_X * CR_LANES_Y, 0, op, rows, n, rpc, sink);
+  else DLB_LAUNCH_KERNEL(ctx, (quad_rows_kernel<false, Op>), grid, CR_LANES_X * CR_LANES_Y, 0, op, rows, n, rpc, sink);
+  DLB_LAUNCHED(ctx);
+  return DLB_OK;
+}
+
 // dlb_brn_forward_sums and dlb_brn_forward_finalize of a single rank.
 dlb_status brn_forward_statistics(dlb_ctx *ctx, const float *Z, int rows, int global_rows, int n_units, float momentum,
                                   float epsilon, float r_max, float d_max, const dlb_brn_unit_arrays *u) {
@@ -1061,6 +1277,10 @@ dlb_status activation_forward_impl(dlb_ctx *ctx, const float *Z, const dlb_brn_u
       return DLB_OK;
     });
   }
+  if (!u && !A_lo && quads(n_units, {Z, A, dp.noise}))
+    return with_af(af, [&](auto AF) {
+      return quad_rows(ctx, ActivationRows<decltype(AF)::value>{Z, A, dp}, rows, n_units, sink);
+    });
   DLB_REQUIRE(!sink.hi, "dlb_activation_forward: planes from a kernel that cannot write them");
   const size_t items = vec4 ? (size_t)rows * (n_units / 4) : (size_t)rows * n_units;
   const int grid = stream_grid(ctx, items, 256);
@@ -1287,13 +1507,14 @@ __global__ void residual_forward_padded_kernel(const float *__restrict__ x, int 
 
 static dlb_status residual_forward_impl(dlb_ctx *ctx, const float *x, float *block,
                                            const uint8_t *row_mask, const float *noise, float *out,
-                                           float *out_lo, int rows, int width, unsigned *amax) {
+                                           float *out_lo, int rows, int width, const PlaneSink &sink) {
   DLB_REQUIRE(ctx && x && block && out && rows > 0 && width > 0, "dlb_residual_forward");
   DLB_REQUIRE(!row_mask || noise, "dlb_residual_forward: row flags need the noise draws");
-  const uintptr_t al = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(block) |
-                       reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_lo) |
-                       reinterpret_cast<uintptr_t>(noise);
-  const int vec = (width % 4 == 0) && (al & 15) == 0;
+  if (!out_lo && quads(width, {x, block, out, row_mask ? noise : nullptr}))
+    return quad_rows(ctx, ResidualRows{x, block, row_mask, noise, out}, rows, width, sink);
+  DLB_REQUIRE(!sink.hi, "dlb_residual_forward: planes from a kernel that cannot write them");
+  unsigned *amax = sink.slot ? reinterpret_cast<unsigned *>(sink.slot) + SLOT_AMAX : nullptr;
+  const int vec = quads(width, {x, block, out, out_lo, noise});
   const size_t items = vec ? (size_t)rows * (width / 4) : (size_t)rows * width;
   DLB_LAUNCH_KERNEL(ctx, residual_forward_kernel, stream_grid(ctx, items, 256), 256, 0, x, block, row_mask, noise, out, out_lo, rows, width, vec, amax);
   DLB_LAUNCHED(ctx);
@@ -1314,10 +1535,16 @@ static dlb_status residual_forward_padded_impl(dlb_ctx *ctx, const float *x, int
 
 static dlb_status shakedrop_backward_impl(dlb_ctx *ctx, const float *d, int ld_d, int first,
                                           const uint8_t *row_mask, const float *noise, float *delta,
-                                          float *delta_lo, int rows, int width, unsigned *amax) {
+                                          float *delta_lo, float *shortcut, int rows, int width, const PlaneSink &sink) {
   DLB_REQUIRE(ctx && d && delta && rows > 0 && width > 0 && first >= 0 && first + width <= ld_d,
               "dlb_shakedrop_backward");
   DLB_REQUIRE(!row_mask || noise, "dlb_shakedrop_backward: row flags need the noise draws");
+  if (!delta_lo && quads(width, {d, delta, row_mask ? noise : nullptr, shortcut}) && ((ld_d | first) & 3) == 0)
+    return quad_rows(ctx, ShakeDropRows{d, ld_d, first, row_mask, noise, delta, shortcut}, rows, width, sink);
+  DLB_REQUIRE(!sink.hi, "dlb_shakedrop_backward: planes from a kernel that cannot write them");
+  unsigned *amax = sink.slot ? reinterpret_cast<unsigned *>(sink.slot) + SLOT_AMAX : nullptr;
+  if (shortcut)
+    DLB_CUDA(cudaMemcpyAsync(shortcut, d, (size_t)rows * width * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
   DLB_LAUNCH_KERNEL(ctx, shakedrop_backward_kernel, stream_grid(ctx, (size_t)rows * width, 256), 256, 0, d, ld_d, first, row_mask, noise, delta, delta_lo, rows, width, amax);
   DLB_LAUNCHED(ctx);
   return DLB_OK;
@@ -1402,8 +1629,10 @@ extern "C" dlb_status dlb_brn_forward_sums_noalloc(const float *Z, int rows, int
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const StoreSums<2> store{sums};
-  column_reduce_kernel<2, SumSqOp, StoreSums<2>><<<dim3(col_blocks, chunks), CR_LANES_X * CR_LANES_Y,
-                                                   column_reduce_shared_bytes<2, SumSqOp>(), s>>>(
+  const bool one = chunks == 1 && column_one_chunk<SumSqOp>(n_units);
+  const auto kernel = one ? column_reduce_kernel<2, SumSqOp, StoreSums<2>, true>
+                          : column_reduce_kernel<2, SumSqOp, StoreSums<2>, false>;
+  kernel<<<dim3(col_blocks, chunks), CR_LANES_X * CR_LANES_Y, column_reduce_shared_bytes<2, SumSqOp>(), s>>>(
       SumSqOp{Z, n_units}, rows, n_units, rows_per_chunk, dev->partials, store);
   DLB_CUDA(cudaGetLastError());
   if (chunks > 1) {
@@ -1445,13 +1674,42 @@ struct PlaneOutput {
 };
 }  // namespace
 
+namespace dlb {
+
+dlb_status shakedrop_backward_shortcut(dlb_ctx *ctx, const float *d, int width_d, int first, const uint8_t *row_mask,
+                                       const float *noise, float *delta, float *delta_lo, float *shortcut, int rows,
+                                       int width) {
+  DLB_REQUIRE(!shortcut || width == width_d, "shakedrop_backward_shortcut: widths");
+  PlaneOutput p;
+  const bool fuse = quads(width, {d, delta, row_mask ? noise : nullptr, shortcut}) && ((width_d | first) & 3) == 0;
+  DLB_TRY(p.begin(ctx, delta, delta_lo, rows, width, fuse));
+  return p.finish(ctx, shakedrop_backward_impl(ctx, d, width_d, first, row_mask, noise, delta, p.kernel_arg, shortcut,
+                                               rows, width, p.sink()));
+}
+
+dlb_status activation_backward_planes(dlb_ctx *ctx, float *dA, float *dA_lo, const float *Z, const float *A, int af,
+                                      int rows, int n_units) {
+  if (!dA_lo || ctx->gemm_kind != DLB_GEMM_F16X3 || !quads(n_units, {dA, Z, A})) {
+    DLB_TRY(dlb_activation_backward(ctx, dA, Z, A, nullptr, af, rows, n_units, nullptr));
+    return dA_lo ? dlb_split_planes_2d(ctx, dA, dA_lo, rows, n_units) : DLB_OK;
+  }
+  PlaneOutput p;
+  DLB_TRY(p.begin(ctx, dA, dA_lo, rows, n_units, true));
+  return p.finish(ctx, with_af(af, [&](auto AF) {
+    return quad_rows(ctx, DerivativeRows<decltype(AF)::value>{dA, Z, A}, rows, n_units, p.sink());
+  }));
+}
+
+}  // namespace dlb
+
 extern "C" {
 
 dlb_status dlb_activation_forward(dlb_ctx *ctx, const float *Z, const dlb_brn_unit_arrays *u, int af,
                                   const dlb_dropout_desc *dropout, float *A, float *A_lo, int rows,
                                   int n_units) {
   PlaneOutput p;
-  DLB_TRY(p.begin(ctx, A, A_lo, rows, n_units, u != nullptr && rows_kernel_applies(Z, A, nullptr, n_units)));
+  const float *draws = !u && dropout && dropout->type == DLB_DROPOUT_UOUT ? dropout->noise : nullptr;
+  DLB_TRY(p.begin(ctx, A, A_lo, rows, n_units, rows_kernel_applies(Z, A, draws, n_units)));
   return p.finish(ctx, activation_forward_impl(ctx, Z, u, af, dropout, A, p.kernel_arg, rows, n_units, p.sink()));
 }
 
@@ -1476,16 +1734,13 @@ dlb_status dlb_loss_delta(dlb_ctx *ctx, int loss, int af, const float *pre, cons
 dlb_status dlb_residual_forward(dlb_ctx *ctx, const float *x, float *block, const uint8_t *row_mask,
                                 const float *noise, float *out, float *out_lo, int rows, int width) {
   PlaneOutput p;
-  DLB_TRY(p.begin(ctx, out, out_lo, rows, width, false));
-  return p.finish(ctx, residual_forward_impl(ctx, x, block, row_mask, noise, out, p.kernel_arg, rows, width, p.amax()));
+  DLB_TRY(p.begin(ctx, out, out_lo, rows, width, quads(width, {x, block, out, row_mask ? noise : nullptr})));
+  return p.finish(ctx, residual_forward_impl(ctx, x, block, row_mask, noise, out, p.kernel_arg, rows, width, p.sink()));
 }
 
 dlb_status dlb_shakedrop_backward(dlb_ctx *ctx, const float *d, const uint8_t *row_mask, const float *noise,
                                   float *delta, float *delta_lo, int rows, int width) {
-  PlaneOutput p;
-  DLB_TRY(p.begin(ctx, delta, delta_lo, rows, width, false));
-  return p.finish(ctx, shakedrop_backward_impl(ctx, d, width, 0, row_mask, noise, delta, p.kernel_arg, rows, width,
-                                               p.amax()));
+  return shakedrop_backward_shortcut(ctx, d, width, 0, row_mask, noise, delta, delta_lo, nullptr, rows, width);
 }
 
 dlb_status dlb_residual_forward_padded(dlb_ctx *ctx, const float *x, int width_x, float *block, int width_block,
@@ -1500,10 +1755,7 @@ dlb_status dlb_residual_forward_padded(dlb_ctx *ctx, const float *x, int width_x
 dlb_status dlb_shakedrop_backward_window(dlb_ctx *ctx, const float *d, int width_d, int first,
                                          const uint8_t *row_mask, const float *noise, float *delta,
                                          float *delta_lo, int rows, int width) {
-  PlaneOutput p;
-  DLB_TRY(p.begin(ctx, delta, delta_lo, rows, width, false));
-  return p.finish(ctx, shakedrop_backward_impl(ctx, d, width_d, first, row_mask, noise, delta, p.kernel_arg, rows,
-                                               width, p.amax()));
+  return shakedrop_backward_shortcut(ctx, d, width_d, first, row_mask, noise, delta, delta_lo, nullptr, rows, width);
 }
 
 }  // extern "C"

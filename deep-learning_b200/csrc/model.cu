@@ -1899,16 +1899,16 @@ static std::vector<size_t> top_level(const dlb_model *m) {
 // L:310-406, L:658-874): the error of the residual output becomes the error of
 // the block output (ShakeDrop rows scaled by fresh U(0,1), then the residual
 // layer's normalization), then the block layers from last to first.
-static dlb_status backward_residual(dlb_model *m, size_t i, int B) {
+static dlb_status backward_residual(dlb_model *m, size_t i, float *shortcut, int B) {
   LayerRT &res = m->layers[i];
   LayerRT &last = m->layers[i + res.depth];
   const bool shake = res.dropout == DLB_DROPOUT_SHAKEDROP;
   const bool rnorm = res.norm != DLB_NORM_NONE;
   // The block reads its window of the residual layer's error.
   const int first = last.units < res.units ? (int)res.pad : 0;
-  DLB_TRY(dlb_shakedrop_backward_window(m->ctx, res.delta, (int)res.units, first, shake ? res.sd_mask : nullptr,
-                                        shake ? res.sd_bwd : nullptr, last.delta,
-                                        rnorm ? nullptr : last.delta_lo, B, (int)last.units));
+  DLB_TRY(shakedrop_backward_shortcut(m->ctx, res.delta, (int)res.units, first, shake ? res.sd_mask : nullptr,
+                                      shake ? res.sd_bwd : nullptr, last.delta, rnorm ? nullptr : last.delta_lo,
+                                      shortcut, B, (int)last.units));
   if (rnorm)
     DLB_TRY(norm_backward(m, res, last.delta, last.delta_lo, last.A, last.A, DLB_AF_LINEAR, B));
   for (size_t j = res.depth; j >= 2; --j) {
@@ -1920,9 +1920,7 @@ static dlb_status backward_residual(dlb_model *m, size_t i, int B) {
     if (b.norm != DLB_NORM_NONE) {
       DLB_TRY(norm_backward(m, b, prev.delta, prev.delta_lo, prev.A, b.IN, b.af, B));
     } else {
-      DLB_TRY(dlb_activation_backward(m->ctx, prev.delta, prev.A, b.IN, nullptr, b.af, B,
-                                      (int)b.fan_in, nullptr));
-      DLB_TRY(dlb_split_planes_2d(m->ctx, prev.delta, prev.delta_lo, B, (int)b.fan_in));
+      DLB_TRY(activation_backward_planes(m->ctx, prev.delta, prev.delta_lo, prev.A, b.IN, b.af, B, (int)b.fan_in));
     }
   }
   return DLB_OK;
@@ -1930,16 +1928,16 @@ static dlb_status backward_residual(dlb_model *m, size_t i, int B) {
 
 // Backward of a residual block inside a time-stepped model: backward_residual
 // over the T * B rows with the per-time-step normalization backward.
-static dlb_status backward_residual_time(dlb_model *m, size_t i, int B, int T) {
+static dlb_status backward_residual_time(dlb_model *m, size_t i, float *shortcut, int B, int T) {
   LayerRT &res = m->layers[i];
   LayerRT &last = m->layers[i + res.depth];
   const int TB = T * B;
   const bool shake = res.dropout == DLB_DROPOUT_SHAKEDROP;
   const bool rnorm = res.norm != DLB_NORM_NONE;
   const int first = last.units < res.units ? (int)res.pad : 0;
-  DLB_TRY(dlb_shakedrop_backward_window(m->ctx, res.delta, (int)res.units, first, shake ? res.sd_mask : nullptr,
-                                        shake ? res.sd_bwd : nullptr, last.delta,
-                                        rnorm ? nullptr : last.delta_lo, TB, (int)last.units));
+  DLB_TRY(shakedrop_backward_shortcut(m->ctx, res.delta, (int)res.units, first, shake ? res.sd_mask : nullptr,
+                                      shake ? res.sd_bwd : nullptr, last.delta, rnorm ? nullptr : last.delta_lo,
+                                      shortcut, TB, (int)last.units));
   if (rnorm) DLB_TRY(norm_backward_time(m, res, last.delta, last.delta_lo, last.A, last.A, DLB_AF_LINEAR, T, B));
   for (size_t j = res.depth; j >= 2; --j) {
     LayerRT &b = m->layers[i + j];
@@ -1949,8 +1947,7 @@ static dlb_status backward_residual_time(dlb_model *m, size_t i, int B, int T) {
     if (b.norm != DLB_NORM_NONE) {
       DLB_TRY(norm_backward_time(m, b, prev.delta, prev.delta_lo, prev.A, b.IN, b.af, T, B));
     } else {
-      DLB_TRY(dlb_activation_backward(m->ctx, prev.delta, prev.A, b.IN, nullptr, b.af, TB, (int)b.fan_in, nullptr));
-      DLB_TRY(dlb_split_planes_2d(m->ctx, prev.delta, prev.delta_lo, TB, (int)b.fan_in));
+      DLB_TRY(activation_backward_planes(m->ctx, prev.delta, prev.delta_lo, prev.A, b.IN, b.af, TB, (int)b.fan_in));
     }
   }
   return DLB_OK;
@@ -1971,14 +1968,17 @@ static dlb_status backward_pass_time(dlb_model *m, size_t rows) {
     LayerRT &l = m->layers[i];
     LayerRT *below = pos > 1 ? &m->layers[tops[pos - 1]] : nullptr;  // the error into the input layer is never formed
     if (l.type == DLB_LAYER_RESIDUAL) {
-      DLB_TRY(backward_residual_time(m, i, B, T));
+      // The shortcut's error: where the widths agree it leaves with the block's.
+      const bool same = below && l.fan_in == l.units && m->layers[i + l.depth].units == l.units;
+      DLB_TRY(backward_residual_time(m, i, same ? below->delta : nullptr, B, T));
       if (below) {
         // shortcut error (its window of the residual layer's error) + delta_1 W_1
         LayerRT &first = m->layers[i + 1];
         const size_t first_col = l.fan_in < l.units ? l.pad : 0;
-        DLB_CUDA(cudaMemcpy2DAsync(below->delta, l.fan_in * sizeof(float), l.delta + first_col,
-                                   l.units * sizeof(float), l.fan_in * sizeof(float), (size_t)TB,
-                                   cudaMemcpyDeviceToDevice, m->ctx->stream));
+        if (!same)
+          DLB_CUDA(cudaMemcpy2DAsync(below->delta, l.fan_in * sizeof(float), l.delta + first_col,
+                                     l.units * sizeof(float), l.fan_in * sizeof(float), (size_t)TB,
+                                     cudaMemcpyDeviceToDevice, m->ctx->stream));
         GemmOperand A{first.delta, first.delta_lo, (long long)first.units, 1};
         GemmOperand Bo{m->params + first.first_conn, m->params_lo + first.first_conn, 1, (long long)first.fan_in};
         GemmEpilogue ep;
@@ -2017,8 +2017,7 @@ static dlb_status backward_pass_time(dlb_model *m, size_t rows) {
         DLB_TRY(dlb_split_planes_2d(m->ctx, l.delta, l.delta_lo, TB, H));
       }
     } else {
-      DLB_TRY(dlb_activation_backward(m->ctx, l.delta, l.Z, l.A, nullptr, l.af, TB, H, nullptr));
-      DLB_TRY(dlb_split_planes_2d(m->ctx, l.delta, l.delta_lo, TB, H));
+      DLB_TRY(activation_backward_planes(m->ctx, l.delta, l.delta_lo, l.Z, l.A, l.af, TB, H));
     }
     if (!below) break;
     const size_t I = l.fan_in;
@@ -2043,15 +2042,18 @@ dlb_status dlb_model_backward_pass(dlb_model *m, size_t rows) {
     LayerRT &l = m->layers[i];
     LayerRT *below = pos > 1 ? &m->layers[tops[pos - 1]] : nullptr;
     if (l.type == DLB_LAYER_RESIDUAL) {
-      DLB_TRY(backward_residual(m, i, B));
+      // The shortcut's error: where the widths agree it leaves with the block's.
+      const bool same = below && l.fan_in == l.units && m->layers[i + l.depth].units == l.units;
+      DLB_TRY(backward_residual(m, i, same ? below->delta : nullptr, B));
       if (below) {
         // shortcut error + delta_1 W_1
         LayerRT &first = m->layers[i + 1];
         // (the shortcut's window of the residual layer's error)
         const size_t first_col = l.fan_in < l.units ? l.pad : 0;
-        DLB_CUDA(cudaMemcpy2DAsync(below->delta, l.fan_in * sizeof(float), l.delta + first_col,
-                                   l.units * sizeof(float), l.fan_in * sizeof(float), (size_t)B,
-                                   cudaMemcpyDeviceToDevice, m->ctx->stream));
+        if (!same)
+          DLB_CUDA(cudaMemcpy2DAsync(below->delta, l.fan_in * sizeof(float), l.delta + first_col,
+                                     l.units * sizeof(float), l.fan_in * sizeof(float), (size_t)B,
+                                     cudaMemcpyDeviceToDevice, m->ctx->stream));
         GemmOperand A{first.delta, first.delta_lo, (long long)first.units, 1};
         GemmOperand Bo{m->params + first.first_conn, m->params_lo + first.first_conn, 1,
                        (long long)first.fan_in};
@@ -2067,8 +2069,7 @@ dlb_status dlb_model_backward_pass(dlb_model *m, size_t rows) {
       if (l.norm != DLB_NORM_NONE) {
         DLB_TRY(norm_backward(m, l, l.delta, l.delta_lo, l.Z, l.A, l.af, B));
       } else {
-        DLB_TRY(dlb_activation_backward(m->ctx, l.delta, l.Z, l.A, nullptr, l.af, B, H, nullptr));
-        DLB_TRY(dlb_split_planes_2d(m->ctx, l.delta, l.delta_lo, B, H));
+        DLB_TRY(activation_backward_planes(m->ctx, l.delta, l.delta_lo, l.Z, l.A, l.af, B, H));
       }
     }
     l.error_final = false;
@@ -2648,8 +2649,7 @@ static dlb_status backward_and_derivatives_overlapped(dlb_model *m, size_t rows,
       if (l.norm != DLB_NORM_NONE) {
         DLB_TRY(norm_backward(m, l, l.delta, l.delta_lo, l.Z, l.A, l.af, B));
       } else {
-        DLB_TRY(dlb_activation_backward(m->ctx, l.delta, l.Z, l.A, nullptr, l.af, B, H, nullptr));
-        DLB_TRY(dlb_split_planes_2d(m->ctx, l.delta, l.delta_lo, B, H));
+        DLB_TRY(activation_backward_planes(m->ctx, l.delta, l.delta_lo, l.Z, l.A, l.af, B, H));
       }
     }
     l.error_final = false;
