@@ -430,14 +430,24 @@ struct PlaneJob {
 dlb_status planes_open(dlb_ctx *ctx, const float *x, float *planes, size_t n, int rows, int cols,
                        bool kernel_can_fuse, PlaneJob *job);
 dlb_status planes_close(dlb_ctx *ctx, const PlaneJob &job);
+// Jobs whose kernels wrote their planes, in one launch.
+dlb_status planes_close_all(dlb_ctx *ctx, const PlaneJob *jobs, int count);
 // max |x| of a tensor no kernel of the library produced (inputs, fresh weights).
 dlb_status planes_absmax(dlb_ctx *ctx, const float *x, size_t n, float *slot);
 dlb_status optimizer_step_amax(dlb_ctx *ctx, int rule, const dlb_optimizer_scalars *s, float *p, float *g,
                                float *first, float *second, float *second_hat, const float *wd_mask, size_t n,
                                unsigned *amax);
-dlb_status optimizer_step_sink(dlb_ctx *ctx, int rule, const dlb_optimizer_scalars *s, float *p, float *g,
-                               float *first, float *second, float *second_hat, const float *wd_mask, int rows,
-                               int cols, const PlaneSink &sink);
+// The update of several weight matrices and their planes in one launch.  The arrays
+// start at the whole vector's first parameter.
+struct MatrixUpdate {
+  size_t at;  // first parameter of the matrix
+  int rows, cols;
+  int rows_per_chunk, first_block;  // filled in by the call
+  PlaneSink sink;
+};
+constexpr int UPDATE_BATCH = 32;
+dlb_status optimizer_matrices(dlb_ctx *ctx, int rule, const dlb_optimizer_scalars *s, float *p, float *g, float *first,
+                              float *second, float *second_hat, const float *wd_mask, MatrixUpdate *jobs, int count);
 constexpr int SCALE_SLOTS = 8192;
 constexpr int SLOT_WORDS = 8;    // words of one scale slot (layout: planes.cuh)
 constexpr int MAX_DEVICES = 64;  // device indices a process may hold contexts on

@@ -2361,14 +2361,15 @@ dlb_status dlb_model_update_weights(dlb_model *m, size_t rows, size_t training_s
   const float wd = k.weight_decay;
   if (m->use_clip_gradient)
     DLB_TRY(dlb_clip_gradient(m->ctx, m->grads, m->total_parameters, m->clip_gradient));
-  // One pass per weight matrix where the products run on fp16 planes: the pass
-  // leaves the matrix's largest |w| in the scale slot of its plane buffer and
-  // the split follows at once, while the matrix is still partly in L2; the
-  // next forward pass then finds the planes ready.  Everything between and
-  // after the matrices (recurrent weights, biases, scales, shifts) goes in
-  // passes of its own.
+  // One launch for the weight matrices where the products run on fp16 planes: it writes
+  // their planes too, so that the next forward pass finds them ready.  (A matrix whose
+  // buffer has no scale to predict from gets a pass of its own that leaves its
+  // largest |w| in the scale slot, and the split.)  Everything between and after the
+  // matrices (recurrent weights, biases, scales, shifts) goes in passes of its own.
   const bool planes_form = m->ctx->gemm_kind == DLB_GEMM_F16X3 && m->params_lo != nullptr;
   bool all_split = planes_form;  // every matrix whose planes are read has them after this update
+  std::vector<MatrixUpdate> updates;
+  std::vector<PlaneJob> jobs;
   auto segment = [&](size_t at, size_t n, unsigned *amax) -> dlb_status {
     if (n == 0) return DLB_OK;
     return optimizer_step_amax(m->ctx, m->optimizer, &k, m->params + at, m->grads + at, m->m1 + at, m->m2 + at,
@@ -2387,14 +2388,18 @@ dlb_status dlb_model_update_weights(dlb_model *m, size_t rows, size_t training_s
     PlaneJob job;
     DLB_TRY(planes_open(m->ctx, m->params + o, m->params_lo + o, nw, (int)l.units, (int)l.fan_in, true, &job));
     if (job.fused) {
-      DLB_TRY(optimizer_step_sink(m->ctx, m->optimizer, &k, m->params + o, m->grads + o, m->m1 + o, m->m2 + o,
-                                  m->m2hat ? m->m2hat + o : nullptr, wd != 0.f ? m->wd_mask + o : nullptr,
-                                  (int)l.units, (int)l.fan_in, job.sink));
+      updates.push_back(MatrixUpdate{o, (int)l.units, (int)l.fan_in, 0, 0, job.sink});
+      jobs.push_back(job);
     } else {
       DLB_TRY(segment(o, nw, job.active ? reinterpret_cast<unsigned *>(job.sink.slot) + 2 : nullptr));
+      DLB_TRY(planes_close(m->ctx, job));
     }
-    DLB_TRY(planes_close(m->ctx, job));
     at = o + nw;
+  }
+  if (!updates.empty()) {
+    DLB_TRY(optimizer_matrices(m->ctx, m->optimizer, &k, m->params, m->grads, m->m1, m->m2, m->m2hat,
+                               wd != 0.f ? m->wd_mask : nullptr, updates.data(), (int)updates.size()));
+    DLB_TRY(planes_close_all(m->ctx, jobs.data(), (int)jobs.size()));
   }
   DLB_TRY(segment(at, m->total_parameters - at, nullptr));
   // Recurrent weights of every IndRNN layer back into the layer's bounds

@@ -121,23 +121,43 @@ __global__ void __launch_bounds__(256)
 // matrix again.  Grid (column blocks of 128, row chunks); a thread owns four
 // columns and walks its rows eight apart.
 constexpr int OPT_LANES_Y = 8;
+// All matrices of a step share a launch: a matrix of 1024 x 1024 alone took 10 us (36 MB,
+// 3.6 TB/s, one wave of blocks that each wait once for memory) and a launch for its
+// statistics 2.4; 17 of them together
+// take 98 us (6.2 TB/s) and 4.
+struct MatrixBatch {
+  MatrixUpdate jobs[UPDATE_BATCH];
+  int count;
+};
 template <int RULE, bool WD>
 __global__ void __launch_bounds__(32 * OPT_LANES_Y)
     optimizer_rows_kernel(dlb_optimizer_scalars k, float *__restrict__ p, float *__restrict__ g,
                           float *__restrict__ m, float *__restrict__ v, float *__restrict__ vh,
-                          const float *__restrict__ mask, int rows, int cols, int rows_per_chunk, PlaneSink sink) {
+                          const float *__restrict__ mask, const __grid_constant__ MatrixBatch batch) {
   pdl_enter();
+  int which = 0;
+  while (which + 1 < batch.count && (int)blockIdx.x >= batch.jobs[which + 1].first_block) ++which;
+  const MatrixUpdate &job = batch.jobs[which];
+  const PlaneSink &sink = job.sink;
+  const int rows = job.rows, cols = job.cols, rows_per_chunk = job.rows_per_chunk;
+  const int col_blocks = (cols + 127) / 128, block = (int)blockIdx.x - job.first_block;
+  const int bx = block % col_blocks, by = block / col_blocks;
+  p += job.at, g += job.at;
+  if (RULE != R_GD) m += job.at;
+  if (!(RULE == R_GD || RULE == R_GD_MOMENTUM || RULE == R_GD_NESTEROV)) v += job.at;
+  if (RULE == R_AMSGRAD || RULE == R_AMSBOUND) vh += job.at;
+  if (WD) mask += job.at;
   __shared__ unsigned line_shared[OPT_LANES_Y * 128];
   constexpr bool HAT = (RULE == R_AMSGRAD || RULE == R_AMSBOUND);
   constexpr bool FIRST = RULE != R_GD;
   constexpr bool SECOND = !(RULE == R_GD || RULE == R_GD_MOMENTUM || RULE == R_GD_NESTEROV);
   const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
-  const int col = blockIdx.x * 128 + tx * 4;
+  const int col = bx * 128 + tx * 4;
   const bool live = col < cols;
   const float plane_scale = sink_scale(sink);
   LineTracker track;
   if (live) {
-    const int r0 = blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
+    const int r0 = by * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
     for (int r = r0 + ty; r < r1; r += OPT_LANES_Y) {
       const size_t o = (size_t)r * cols + col;
       float4 P = *reinterpret_cast<const float4 *>(p + o);
@@ -163,7 +183,7 @@ __global__ void __launch_bounds__(32 * OPT_LANES_Y)
       track.row(sink, r, out);
     }
   }
-  track.finish(sink, line_shared, tx, ty, OPT_LANES_Y, blockIdx.x * 128, cols, live);
+  track.finish(sink, line_shared, tx, ty, OPT_LANES_Y, bx * 128, cols, live);
 }
 
 // Calls f(std::integral_constant<int, R>) with the kernel rule of an optimizer
@@ -189,19 +209,26 @@ static dlb_status with_rule(int rule, const dlb_optimizer_scalars &s, F f) {
   }
 }
 
+// Chunks of about two waves of blocks over the chip, at least a row per lane.
 template <int RULE>
 static dlb_status launch_rule_rows(dlb_ctx *ctx, const dlb_optimizer_scalars &k, float *p, float *g, float *m,
-                                   float *v, float *vh, const float *mask, int rows, int cols,
-                                   const PlaneSink &sink) {
-  const int col_blocks = ceil_div(cols, 128);
-  int chunks = max(1, min(ceil_div(ctx->sm_count * 8, col_blocks), ceil_div(rows, OPT_LANES_Y)));
-  const int rpc = ceil_div(ceil_div(rows, chunks), OPT_LANES_Y) * OPT_LANES_Y;
-  chunks = ceil_div(rows, rpc);
-  const dim3 grid(col_blocks, chunks);
+                                   float *v, float *vh, const float *mask, MatrixUpdate *jobs, int count) {
+  long long lines = 0;
+  for (int i = 0; i < count; ++i) lines += (long long)ceil_div(jobs[i].cols, 128) * jobs[i].rows;
+  const int rpc = (int)align_up((size_t)max(1LL, lines / (ctx->sm_count * 16)), OPT_LANES_Y);
+  MatrixBatch batch;
+  batch.count = count;
+  int blocks = 0;
+  for (int i = 0; i < count; ++i) {
+    jobs[i].rows_per_chunk = rpc;
+    jobs[i].first_block = blocks;
+    blocks += ceil_div(jobs[i].cols, 128) * ceil_div(jobs[i].rows, rpc);
+    batch.jobs[i] = jobs[i];
+  }
   if (k.weight_decay != 0.f)
-    DLB_LAUNCH_KERNEL(ctx, (optimizer_rows_kernel<RULE, true>), grid, 32 * OPT_LANES_Y, 0, k, p, g, m, v, vh, mask, rows, cols, rpc, sink);
+    DLB_LAUNCH_KERNEL(ctx, (optimizer_rows_kernel<RULE, true>), blocks, 32 * OPT_LANES_Y, 0, k, p, g, m, v, vh, mask, batch);
   else
-    DLB_LAUNCH_KERNEL(ctx, (optimizer_rows_kernel<RULE, false>), grid, 32 * OPT_LANES_Y, 0, k, p, g, m, v, vh, mask, rows, cols, rpc, sink);
+    DLB_LAUNCH_KERNEL(ctx, (optimizer_rows_kernel<RULE, false>), blocks, 32 * OPT_LANES_Y, 0, k, p, g, m, v, vh, mask, batch);
   DLB_LAUNCHED(ctx);
   return DLB_OK;
 }
@@ -321,15 +348,20 @@ dlb_status dlb::optimizer_step_amax(dlb_ctx *ctx, int rule, const dlb_optimizer_
   });
 }
 
-// The pass over one weight matrix [rows, cols] that also writes the matrix's
-// fp16 planes and range statistics through `sink` (optimizer_rows_kernel).
-dlb_status dlb::optimizer_step_sink(dlb_ctx *ctx, int rule, const dlb_optimizer_scalars *s, float *p, float *g,
-                                    float *first, float *second, float *second_hat, const float *wd_mask,
-                                    int rows, int cols, const PlaneSink &sink) {
-  DLB_REQUIRE(ctx && s && p && g && rows > 0 && cols > 0 && (cols & 3) == 0 && sink.hi && sink.slot,
-              "optimizer_step_sink");
-  return with_rule(rule, *s, [&](auto R) {
-    return launch_rule_rows<decltype(R)::value>(ctx, *s, p, g, first, second, second_hat, wd_mask, rows, cols, sink);
+// The pass over weight matrices that also writes their fp16 planes and range
+// statistics (optimizer_rows_kernel).
+dlb_status dlb::optimizer_matrices(dlb_ctx *ctx, int rule, const dlb_optimizer_scalars *s, float *p, float *g,
+                                   float *first, float *second, float *second_hat, const float *wd_mask,
+                                   MatrixUpdate *jobs, int count) {
+  DLB_REQUIRE(ctx && s && p && g && jobs, "optimizer_matrices");
+  for (int i = 0; i < count; ++i)
+    DLB_REQUIRE(jobs[i].rows > 0 && jobs[i].cols > 0 && (jobs[i].cols & 3) == 0 && jobs[i].sink.hi && jobs[i].sink.slot,
+                "optimizer_matrices: matrix");
+  return with_rule(rule, *s, [&](auto R) -> dlb_status {
+    for (int i = 0; i < count; i += UPDATE_BATCH)
+      DLB_TRY(launch_rule_rows<decltype(R)::value>(ctx, *s, p, g, first, second, second_hat, wd_mask, jobs + i,
+                                                   min(UPDATE_BATCH, count - i)));
+    return DLB_OK;
   });
 }
 

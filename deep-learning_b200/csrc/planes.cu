@@ -252,8 +252,14 @@ __global__ void __launch_bounds__(LS_THREADS) split_lines_kernel(const __grid_co
   else split_contiguous_lines(o, block, flag);
 }
 
-__global__ void __launch_bounds__(1024) planes_finalize_kernel(PlaneSink k) {
+// A block per tensor.
+struct FinalizeBatch {
+  PlaneSink sinks[UPDATE_BATCH];
+};
+__global__ void __launch_bounds__(1024) planes_finalize_kernel(const __grid_constant__ PlaneSink k) {
   pdl_enter(); sink_finalize(k); }
+__global__ void __launch_bounds__(1024) planes_finalize_all_kernel(const __grid_constant__ FinalizeBatch b) {
+  pdl_enter(); sink_finalize(b.sinks[blockIdx.x]); }
 
 int stream_blocks(dlb_ctx *ctx, size_t items) {
   const size_t blocks = (items + 255) / 256;
@@ -535,6 +541,25 @@ dlb_status planes_close(dlb_ctx *ctx, const PlaneJob &job) {
   DLB_LAUNCH_KERNEL(ctx, planes_finalize_kernel, 1, 1024, 0, k);
   DLB_LAUNCHED(ctx);
   e.seen = true;
+  return DLB_OK;
+}
+
+dlb_status planes_close_all(dlb_ctx *ctx, const PlaneJob *jobs, int count) {
+  for (int first = 0; first < count; first += UPDATE_BATCH) {
+    FinalizeBatch b;
+    const int n = min(UPDATE_BATCH, count - first);
+    for (int i = 0; i < n; ++i) {
+      const PlaneJob &job = jobs[first + i];
+      auto it = ctx->planes.find(reinterpret_cast<uintptr_t>(job.planes));
+      DLB_REQUIRE(job.active && job.fused && it != ctx->planes.end(), "plane buffers: closed together");
+      b.sinks[i] = job.sink;
+      sink_lines(b.sinks[i], it->second.lines, it->second.rows, it->second.cols, job.sink.rows_exempt != 0);
+      b.sinks[i].predicted = 1;
+      it->second.seen = true;
+    }
+    DLB_LAUNCH_KERNEL(ctx, planes_finalize_all_kernel, n, 1024, 0, b);
+    DLB_LAUNCHED(ctx);
+  }
   return DLB_OK;
 }
 
