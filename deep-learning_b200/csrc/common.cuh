@@ -468,6 +468,11 @@ dlb_status shakedrop_backward_shortcut(dlb_ctx *ctx, const float *d, int width_d
 dlb_status activation_backward_planes(dlb_ctx *ctx, float *dA, float *dA_lo, const float *Z, const float *A, int af,
                                       int rows, int n_units);
 
+// Flags of ShakeDrop (stream), forward factors from U(-1, 1) (stream + 1) and backward
+// ones from U(0, 1) (stream + 2), the factors of flagged rows only.
+dlb_status noise_shakedrop(dlb_ctx *ctx, uint8_t *mask, float *fwd, float *bwd, size_t rows, size_t width, float p,
+                           uint64_t seed, uint32_t stream, uint32_t step, uint64_t first_row);
+
 // All time steps of an LSTM layer in one launch (lstm_walk.cu).  done: whether this
 // was the faster way and has been enqueued; the step entry points otherwise.
 // Backward: dH [T, rows, C] gets the recurrent part added.

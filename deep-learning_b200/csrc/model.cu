@@ -1719,12 +1719,9 @@ dlb_status dlb_model_draw_noise(dlb_model *m, size_t rows, uint64_t seed, uint32
         // factors from U(-1, 1), backward factors from U(0, 1)
         // (fwp_mp.cpp L:3881-3888, bwp_mp.cpp ShakeDrop backward).
         DLB_TRY(ensure_shakedrop(m, l, rows));
-        DLB_TRY(dlb_noise_bernoulli(m->ctx, l.sd_mask, rows, l.dropout_value, seed, stream, step, first_row));
         // (one factor per element of the block's output, norm_units wide)
-        DLB_TRY(dlb_noise_uniform(m->ctx, l.sd_fwd, rows * l.norm_units, -1.f, 1.f, seed, stream + 1, step,
-                                  first_row * l.norm_units));
-        DLB_TRY(dlb_noise_uniform(m->ctx, l.sd_bwd, rows * l.norm_units, 0.f, 1.f, seed, stream + 2, step,
-                                  first_row * l.norm_units));
+        DLB_TRY(noise_shakedrop(m->ctx, l.sd_mask, l.sd_fwd, l.sd_bwd, rows, l.norm_units, l.dropout_value, seed, stream,
+                                step, first_row));
         break;
       default:
         break;
