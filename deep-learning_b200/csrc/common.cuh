@@ -292,6 +292,10 @@ dlb_status gemm_simt(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, f
 dlb_status gemm_small(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C, long long ldc, int M, int N,
                       int K, const GemmEpilogue &ep);
 double gemm_small_us(const dlb_ctx *ctx, int M, int N, int K);
+// Products of k-contiguous operands in fp32 with every sum in ascending k (gemm_ordered.cu).
+dlb_status gemm_ordered(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C, long long ldc, int M, int N,
+                        int K, const GemmEpilogue &ep);
+double gemm_ordered_us(const dlb_ctx *ctx, int M, int N, int K);
 // Tensor-core product from the fp32 tensors (gemm_direct.cu).
 dlb_status gemm_direct(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, float *C, long long ldc, int M, int N,
                        int K, const GemmEpilogue &ep);

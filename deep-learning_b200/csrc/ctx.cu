@@ -103,16 +103,26 @@ static bool planes_beat_small(const dlb_ctx *ctx, int M, int N, int K, double pl
 }
 // The way of a product whose operands' planes are not both kept: the shortest by the
 // kernels' own estimates, missing planes made for it.
-enum class Way { SMALL, DIRECT, PLANES };
+enum class Way { SMALL, DIRECT, PLANES, ORDERED };
 static Way gemm_way(const dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K,
                     bool accumulate, bool have_a, bool have_b) {
-  const double direct = gemm_direct_us(ctx, M, N, K);
+  const double small = gemm_small_us(ctx, M, N, K), direct = gemm_direct_us(ctx, M, N, K);
+  Way way = small < direct ? Way::SMALL : Way::DIRECT;
+  double best = std::min(small, direct);
   if (plane_size(M, N, K) && gemm_pair_enabled() && !(A.stride_k != 1 && B.stride_k == 1)) {
     const double planes = gemm_planes_us(ctx, A, B, M, N, K, accumulate) +
                           split_us((have_a ? 0 : (long long)M * K) + (have_b ? 0 : (long long)N * K));
-    if (planes <= direct && planes_beat_small(ctx, M, N, K, planes)) return Way::PLANES;
+    if (planes <= direct && planes_beat_small(ctx, M, N, K, planes)) way = Way::PLANES, best = planes;
   }
-  return gemm_small_us(ctx, M, N, K) < direct ? Way::SMALL : Way::DIRECT;
+  // Forward products of a width that TMA cannot address keep their order of summation
+  // as long as the SMs have a tile each and it takes three times the shortest way at
+  // most (333 x 1203 x 1203: 47 us against 21): larger ones have batches in which a unit
+  // more or less on one side of an activation's kink counts less, and would pay more.
+  const bool unaddressable = ((A.stride_mn | B.stride_mn) & 7) != 0;
+  if (A.stride_k == 1 && B.stride_k == 1 && unaddressable && std::min(M, N) >= 64 &&
+      ceil_div(M, 64) * (long long)ceil_div(N, 64) <= ctx->sm_count && gemm_ordered_us(ctx, M, N, K) <= 3.0 * best)
+    way = Way::ORDERED;
+  return way;
 }
 
 // The fused epilogues exist in the medium fp16-plane kernel, for K-major A, with both
@@ -186,6 +196,7 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
     const bool kept = have_a && have_b && gemm_f16_supported(A, B, C, ldc, M, N, K);
     const Way way = kept ? Way::PLANES : gemm_way(ctx, A, B, M, N, K, ep.accumulate, have_a, have_b);
     if (way == Way::SMALL) return gemm_small(ctx, A_in, B_in, C, ldc, M, N, K, ep);
+    if (way == Way::ORDERED) return gemm_ordered(ctx, A_in, B_in, C, ldc, M, N, K, ep);
     if (way == Way::DIRECT) {
       ProfileSpan span;
       DLB_TRY(span.begin(ctx, 0, 2.0 * M * N * K));

@@ -1,0 +1,28 @@
+"""Forward products that keep their order of summation (csrc/gemm_ordered.cu): bit for bit
+the CUDA-core kernel's results, at edges of the 64 x 64 tile and the 32-deep slab and up to
+as many tiles as SMs."""
+import numpy as np
+import pytest
+
+from dlb200 import check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,n_in,n_out", [(64, 129, 64), (70, 133, 65), (333, 617, 1203), (500, 333, 333), (65, 2049, 127)])
+def test_same_bits_as_sums_in_ascending_k(gpu_ctx, rows, n_in, n_out):
+    ctx, rng = gpu_ctx, np.random.default_rng(rows)
+    x, w = rng.standard_normal((rows, n_in), dtype=np.float32), rng.standard_normal((n_out, n_in), dtype=np.float32)
+    b = rng.standard_normal(n_out).astype(np.float32)
+    xd, wd, bd, z = ctx.array(x), ctx.array(w), ctx.array(b), [ctx.empty((rows, n_out)) for _ in range(2)]
+    try:
+        for on in (0, 1):
+            ctx.set_tensor_core(bool(on))
+            check(ctx.L.dlb_fc_forward(ctx.h, xd.ptr, None, wd.ptr, None, bd.ptr, z[on].ptr, rows, n_in, n_out))
+    finally:
+        ctx.set_tensor_core(True)
+    assert ctx.sync() == 0
+    got = z[1].get()
+    assert np.abs(got - (x.astype(np.float64) @ w.T + b)).max() <= 2e-6 * n_in ** 0.5 * 12
+    if rows * n_out >= 128 * 128 and n_in < 2000:
+        assert np.array_equal(got, z[0].get())
