@@ -306,7 +306,7 @@ dlb_status dlb_activation_backward(dlb_ctx *ctx, float *dA, const float *Z, cons
  * normalization, as one call: Z = X W^T + bias, A = dropout(f(Z)) (+ A's plane
  * buffer).  ref: Forward_Pass__FC__OpenMP + Forward_Pass__Bias__OpenMP +
  * Forward_Pass__FC_AF__OpenMP and the dropout forwards (v1/learner/fwp_mp.cpp
- * L:4396-4459, L:4741-4770, L:4809-4985).  Where the product runs on the 2-CTA
+ * L:4396-4459, L:4741-4770, L:4809-4985).  Where the product runs on the medium
  * tensor-core kernel (fp16 planes, at least 256 x 256 outputs, both operands'
  * plane buffers kept by the caller, A's buffer split once before), bias,
  * activation, dropout (Bernoulli flags per unit, inverted Bernoulli, UOut) and
