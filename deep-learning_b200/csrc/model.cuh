@@ -3,6 +3,7 @@
 // reference's text checkpoint format).
 #pragma once
 
+#include <atomic>
 #include <condition_variable>
 #include <functional>
 #include <mutex>
@@ -31,7 +32,10 @@ class HostWorkers {
   std::mutex mu_;
   std::condition_variable work_, done_;
   const std::function<void(size_t)> *fn_ = nullptr;
-  size_t parts_ = 0, next_ = 0, finished_ = 0;
+  size_t parts_ = 0, next_ = 0;
+  // Written under mu_; read without it by threads that look before they sleep.
+  std::atomic<size_t> finished_{0};
+  std::atomic<bool> open_{false};  // parts left to take
   bool stop_ = false;
 };
 
