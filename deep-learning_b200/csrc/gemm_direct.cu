@@ -417,6 +417,10 @@ __global__ void __launch_bounds__(D_THREADS, 1) gemm_direct_kernel(const __grid_
       if (lane == 0) mbar_arrive(parts_bar);
     }
   }
+  // Everything this thread sends is on its way.  The CTAs leave together (at the end):
+  // one whose own wait ran out must not be gone while another still writes its part here.
+  __syncwarp();
+  if (splits > 1) cluster_arrive();
   const bool here = mbar_wait_cluster(parts_bar, 0, abort_flag, a.status);
   if (*reinterpret_cast<volatile int *>(range_flag)) {
     direct_fp32_tile(&a, m0, n0, piece, reinterpret_cast<float *>(smem));
@@ -436,6 +440,9 @@ __global__ void __launch_bounds__(D_THREADS, 1) gemm_direct_kernel(const __grid_
       }
     }
   }
+  __syncwarp();
+  if (splits > 1) cluster_wait();
+  if (*abort_flag) drain_pause();  // MMAs that were issued
   if (warp == D_CONV_WARPS) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(D_STAGES * DN))

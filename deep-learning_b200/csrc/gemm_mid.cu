@@ -355,6 +355,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   }
   __syncthreads();
   cluster_sync_all();  // no CTA leaves while another may still signal it or write its parts
+  if (*abort_flag) drain_pause();  // blocks sent to this CTA that it did not wait for
   if (warp == 1) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * QN))

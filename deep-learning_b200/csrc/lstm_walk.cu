@@ -264,8 +264,13 @@ struct Exchange {
     if (!tc::mbar_wait_cluster(bar + (step & 1) * 8, (uint32_t)(step >> 1) & 1u, abort_flag, status)) return;
     if (threadIdx.x == 0) tc::mbar_expect_tx(bar + (step & 1) * 8, (uint32_t)bytes);
   }
+  // No CTA leaves while another may still send to it; after a wait that ran out the
+  // barrier says nothing about the values in flight.
   __device__ __forceinline__ void finish() const {
-    if (cs > 1) tc::cluster_sync_all();
+    if (cs == 1) return;
+    __syncwarp();
+    tc::cluster_sync_all();
+    if (*static_cast<volatile int *>(abort_flag)) tc::drain_pause();
   }
 };
 

@@ -69,6 +69,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// After a wait that ran out, before a kernel gives up what copies or MMAs in flight
+// may still touch and that no barrier counts any more.
+__device__ __forceinline__ void drain_pause() {
+  const long long t0 = clock64();
+  while (clock64() - t0 < DRAIN_BUDGET_CLOCKS) {
+  }
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar,
                                             int c0, int c1) {
   asm volatile(
