@@ -94,6 +94,7 @@ struct dlb_ctx {
     uint32_t seq = 0;       // exchanges so far, the same on every rank
   } peer;
   uint64_t launches = 0;
+  uint64_t products[DLB_PRODUCT_KINDS] = {};  // by the kernel that formed them
   // Programmatic dependent launch for the library's kernels (DLB_PDL=0 turns it off).
   bool use_pdl = true;
   cudaEvent_t timer_start = nullptr, timer_stop = nullptr;

@@ -447,6 +447,12 @@ dlb_status dlb_ctx_set_tensor_core(dlb_ctx *ctx, int enable) {
 
 uint64_t dlb_ctx_launch_count(dlb_ctx *ctx) { return ctx ? ctx->launches : 0; }
 
+dlb_status dlb_ctx_product_counts(dlb_ctx *ctx, uint64_t counts[DLB_PRODUCT_KINDS]) {
+  DLB_REQUIRE(ctx && counts, "dlb_ctx_product_counts: null");
+  memcpy(counts, ctx->products, sizeof(ctx->products));
+  return DLB_OK;
+}
+
 dlb_status dlb_ctx_timer_start(dlb_ctx *ctx) {
   DLB_REQUIRE(ctx, "dlb_ctx_timer_start: null");
   if (!ctx->timer_start) {

@@ -477,6 +477,7 @@ dlb_status launch_direct(dlb_ctx *ctx, const DirectArgs &args, int tiles) {
   DLB_CUDA(launch_kernel_cluster(ctx, kernel, dim3((unsigned)(tiles << args.split_shift)), dim3(D_THREADS), D_SMEM,
                                  1u << args.split_shift, args));
   DLB_LAUNCHED(ctx);
+  ctx->products[DLB_PRODUCT_DIRECT]++;
   return DLB_OK;
 }
 

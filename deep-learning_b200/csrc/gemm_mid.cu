@@ -396,6 +396,7 @@ dlb_status launch_mid_shift(dlb_ctx *ctx, const GemmOperand &A, const GemmOperan
   DLB_CUDA(launch_kernel_cluster(ctx, kernel, dim3((unsigned)(tiles << (SHIFT + 1))), dim3(NUM_THREADS), Q_SMEM,
                                  2u << SHIFT, ta, tal, tb, tbl, args, FUSED ? *ep.fused : FusedEpilogue{}));
   DLB_LAUNCHED(ctx);
+  ctx->products[DLB_PRODUCT_MID]++;
   return DLB_OK;
 }
 

@@ -144,6 +144,7 @@ dlb_status gemm_ordered(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B
                          quad_target(C, ldc, M, N, ep.bias, ep.accumulate, nullptr), K, ceil_div(N, OT)};
   DLB_LAUNCH_KERNEL(ctx, gemm_ordered_kernel, ceil_div(M, OT) * args.tiles_n, O_THREADS, O_SMEM, args);
   DLB_LAUNCHED(ctx);
+  ctx->products[DLB_PRODUCT_ORDERED]++;
   return DLB_OK;
 }
 

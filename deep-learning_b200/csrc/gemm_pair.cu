@@ -439,6 +439,7 @@ dlb_status launch_pair(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B,
   const int items = whole_tiles + parts * split_tiles;
   DLB_LAUNCH_KERNEL(ctx, kernel, 2 * min(items, lanes), NUM_THREADS, P::TOTAL, ta, tal, tb, tbl, quad_target(C, ldc, M, N, ep.bias, ep.accumulate, B.line_inv), K, tiles_n, band, whole_tiles, parts, items, A.scale, B.scale, ctx->d_status, A.guard, B.guard, A.guard_mask, B.guard_mask, A.line_inv, fp32_operands(A, B), ctx->d_guard ? ctx->d_guard + 1 : nullptr);
   DLB_LAUNCHED(ctx);
+  ctx->products[DLB_PRODUCT_PAIR]++;
   return DLB_OK;
 }
 

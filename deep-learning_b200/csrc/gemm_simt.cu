@@ -20,6 +20,7 @@ dlb_status gemm_simt(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, f
   const int grid = ceil_div(N, ST_N) * ceil_div(M, ST_M);
   DLB_LAUNCH_KERNEL(ctx, gemm_simt_kernel, grid, 256, 0, SimtOperands{A.ptr, A.stride_mn, A.stride_k, B.ptr, B.stride_mn, B.stride_k}, C, ldc, M, N, K, ep.bias, ep.accumulate);
   DLB_LAUNCHED(ctx);
+  ctx->products[DLB_PRODUCT_SIMT]++;
   return DLB_OK;
 }
 

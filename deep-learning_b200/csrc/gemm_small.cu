@@ -167,6 +167,7 @@ dlb_status launch_small(dlb_ctx *ctx, const SmallArgs &args, int tiles) {
   DLB_CUDA(launch_kernel_cluster(ctx, gemm_small_kernel<A_MN, B_MN>, dim3((unsigned)(tiles << args.split_shift)),
                                  dim3(S_THREADS), 0, 1u << args.split_shift, args));
   DLB_LAUNCHED(ctx);
+  ctx->products[DLB_PRODUCT_SMALL]++;
   return DLB_OK;
 }
 

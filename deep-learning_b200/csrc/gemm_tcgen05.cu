@@ -539,6 +539,7 @@ dlb_status launch(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, floa
   const int items = whole_tiles + 2 * split_tiles;
   DLB_LAUNCH_KERNEL(ctx, kernel, min(items, lanes), NUM_THREADS, P::TOTAL, ta, tal, tb, tbl, C, ldc, M, N, K, ep.bias, ep.accumulate, tiles_n, whole_tiles, items, A.scale, B.scale, ctx->d_status, ES == 2 ? A.guard : nullptr, ES == 2 ? B.guard : nullptr, A.guard_mask, B.guard_mask, fp32_operands(A, B), ctx->d_guard ? ctx->d_guard + 1 : nullptr);
   DLB_LAUNCHED(ctx);
+  ctx->products[DLB_PRODUCT_ONE_CTA]++;
   return DLB_OK;
 }
 

@@ -385,6 +385,7 @@ dlb_status planes_split_lines(dlb_ctx *ctx, GemmOperand *A, int M, GemmOperand *
     DLB_LAUNCH_KERNEL(ctx, split_lines_kernel, grid, LS_THREADS, 0, job[0], job[1], flag, next);
   }
   DLB_LAUNCHED(ctx);
+  ctx->products[DLB_PRODUCT_FRESH_PLANES]++;
   return DLB_OK;
 }
 

@@ -45,6 +45,7 @@ SIGNATURES = {
     "dlb_ctx_stream": (_vp, [_vp]),
     "dlb_ctx_set_tensor_core": (_i, [_vp, _i]),
     "dlb_ctx_launch_count": (_u64, [_vp]),
+    "dlb_ctx_product_counts": (_i, [_vp, C.POINTER(_u64)]),
     "dlb_ctx_timer_start": (_i, [_vp]),
     "dlb_ctx_timer_stop": (_i, [_vp, C.POINTER(_f)]),
     "dlb_ctx_gemm_profile": (_i, [_vp, _i]),
@@ -284,6 +285,14 @@ class Context:
 
     def launch_count(self):
         return int(self.L.dlb_ctx_launch_count(self.h))
+
+    PRODUCTS = ("simt", "small", "ordered", "direct", "mid", "pair", "one_cta", "fresh_planes")
+
+    def product_counts(self):
+        """How many products each kernel has formed (DLB_PRODUCT_* of the header)."""
+        n = (_u64 * len(self.PRODUCTS))()
+        check(self.L.dlb_ctx_product_counts(self.h, n), "dlb_ctx_product_counts")
+        return dict(zip(self.PRODUCTS, map(int, n)))
 
     def timer_start(self):
         check(self.L.dlb_ctx_timer_start(self.h), "dlb_ctx_timer_start")

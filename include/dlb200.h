@@ -74,6 +74,20 @@ void *dlb_ctx_stream(dlb_ctx *ctx); /* cudaStream_t */
 dlb_status dlb_ctx_set_tensor_core(dlb_ctx *ctx, int enable);
 /* Number of kernels this context has launched since creation. */
 uint64_t dlb_ctx_launch_count(dlb_ctx *ctx);
+/* Which kernels have formed the context's products, by DLB_PRODUCT_*: the sizes, pitches and
+ * kept planes of a product decide (csrc/ctx.cu), and this shows what they decided. */
+enum {
+  DLB_PRODUCT_SIMT = 0,         /* fp32 on the CUDA cores, any strides */
+  DLB_PRODUCT_SMALL = 1,        /* fp32 on the CUDA cores, small outputs */
+  DLB_PRODUCT_ORDERED = 2,      /* fp32 on the CUDA cores, sums in ascending k */
+  DLB_PRODUCT_DIRECT = 3,       /* tensor cores, operands split in the kernel */
+  DLB_PRODUCT_MID = 4,          /* tensor cores on planes, 256 x 128 tiles */
+  DLB_PRODUCT_PAIR = 5,         /* tensor cores on planes, 256 x 256 tiles */
+  DLB_PRODUCT_ONE_CTA = 6,      /* tensor cores, a tile per CTA (TF32 form) */
+  DLB_PRODUCT_FRESH_PLANES = 7, /* not a product: planes made for one (MID or PAIR) */
+  DLB_PRODUCT_KINDS = 8
+};
+dlb_status dlb_ctx_product_counts(dlb_ctx *ctx, uint64_t counts[DLB_PRODUCT_KINDS]);
 /* Device-side timing on the context's stream (CUDA events): start records an
  * event, stop records another, waits for it and returns the milliseconds
  * between the two. */

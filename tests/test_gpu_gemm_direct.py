@@ -78,3 +78,73 @@ def test_values_the_halves_cannot_hold(gpu_ctx, value):
             assert np.array_equal(np.isnan(got), np.isnan(want))
             assert np.array_equal(np.isfinite(got), finite)
             assert util.rel_l2(got[finite], want[finite]) <= 1e-6
+
+
+B_SEED = 11
+# Sizes at which gemm_direct.cu forms the product (the sizes above it leaves to other
+# kernels): which product of the layer, one CTA and clusters per tile, operands contiguous
+# along k and along the free dimension.
+DIRECT = [((1000, 66, 1001), 0), ((1000, 66, 1001), 1), ((1000, 66, 1001), 2), ((951, 7735, 65), 0), ((951, 65, 7735), 1),
+          ((7735, 65, 951), 2), ((2048, 256, 256), 1)]
+
+
+def _direct_only(ctx, shape, which, x, w, d):
+    """Product `which` of the layer, which must be gemm_direct_kernel's, and the guard's
+    counters that it moved."""
+    before, guard = ctx.product_counts(), ctx.guard_counters()
+    L, (B, I, O) = ctx.L, shape
+    xd, wd, dd = (ctx.array(a) for a in (x, w, d))
+    out = ctx.empty(((B, O), (B, I), (O, I))[which])
+    call = ((L.dlb_fc_forward, xd.ptr, None, wd.ptr, None, None, out.ptr, B, I, O),
+            (L.dlb_fc_backward_input, dd.ptr, None, wd.ptr, None, out.ptr, B, I, O),
+            (L.dlb_fc_weight_gradient, dd.ptr, None, xd.ptr, None, out.ptr, None, B, I, O, 0))[which]
+    check(call[0](ctx.h, *call[1:]))
+    assert ctx.sync() == 0
+    assert {k for k, n in ctx.product_counts().items() if n != before[k]} == {"direct"}
+    assert ctx.guard_counters() == guard
+    return out.get()
+
+
+def _exact(which, x, w, d):
+    """The product and the largest error of an element.  S, the larger of the sum's own size
+    and of sqrt(sum a^2 b^2), that of a sum whose signs are random: 22-bit operands move it
+    by 2^-22 S at most in the mean square (five of that: 2^-20 S); the tensor core cuts
+    off, 12 times in a chunk of 64 k, less than 2^-23 S; fp32 additions one by one move
+    it by 0.3 2^-24 sqrt(k) S in the mean square."""
+    x, w, d = (a.astype(np.float64) for a in (x, w, d))
+    a, b = ((x, w.T), (d, w), (d.T, x))[which]
+    exact = a @ b
+    size = np.maximum(np.sqrt((a * a) @ (b * b)), np.abs(exact))
+    return exact, size * (2.0 ** -20 + 12 * 2.0 ** -23 + 5 * 0.3 * 2.0 ** -24 * np.sqrt(a.shape[1]))
+
+
+@pytest.mark.parametrize("shape,which", DIRECT)
+def test_direct_kernel_lines_of_very_different_size(gpu_ctx, shape, which):
+    """A scale per line and chunk: lines spread over 2^-20 .. 2^20 keep their own accuracy,
+    where every row of the output is fed by one line of an operand."""
+    rng, (B, I, O) = np.random.default_rng(B_SEED + which), shape
+    x, w, d = (rng.standard_normal(s, dtype=np.float32) for s in ((B, I), (O, I), (B, O)))
+    # of the two operands' free lines: rows of x and w; rows of d, columns of w; columns of d and x
+    spread = lambda n: np.exp2(rng.uniform(-20, 20, n)).astype(np.float32)  # noqa: E731
+    if which == 0:
+        x, w = x * spread(B)[:, None], w * spread(O)[:, None]
+    elif which == 1:
+        d, w = d * spread(B)[:, None], w * spread(I)
+    else:
+        d, x = d * spread(O), x * spread(I)
+    got, (want, bound) = _direct_only(gpu_ctx, shape, which, x, w, d), _exact(which, x, w, d)
+    assert np.all(np.abs(got - want) <= bound)
+
+
+@pytest.mark.parametrize("value", [2.0 ** 120, np.inf, np.nan, 1e-40])
+@pytest.mark.parametrize("shape,which", DIRECT)
+def test_direct_kernel_values_the_halves_cannot_hold(gpu_ctx, shape, which, value):
+    """The tile of such a value is formed in fp32, by all CTAs of its cluster."""
+    rng, (B, I, O) = np.random.default_rng(B_SEED + which), shape
+    x, w, d = (rng.standard_normal(s, dtype=np.float32) for s in ((B, I), (O, I), (B, O)))
+    (x, d, d)[which][B - 3, (I, O, O)[which] - 2] = np.float32(value)
+    with np.errstate(all="ignore"):
+        got, (want, bound) = _direct_only(gpu_ctx, shape, which, x, w, d), _exact(which, x, w, d)
+        finite = np.isfinite(want) & (np.abs(want) < 3e38)
+        assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isfinite(got), finite)
+        assert np.all(np.abs(got - want)[finite] <= bound[finite])
