@@ -280,6 +280,9 @@ struct GemmEpilogue {
   const float *bias = nullptr;   // per-n bias added to every row
   float *colsum = nullptr;       // per-n sum over m of C (db), written/accumulated
   int accumulate = 0;            // C += result
+  // No derivative that jumps at 0 is taken of what these sums lead to: gemm() need not
+  // keep their order (gemm_ordered.cu).
+  bool any_order = false;
   // Work of the kernel that would follow the product, done on the tile while the
   // drain warps hold it (the medium fp16-plane kernel only: ask gemm_fused_supported).
   const FusedEpilogue *fused = nullptr;
@@ -404,6 +407,13 @@ struct FusedEpilogue {
   const float *a = nullptr;       //   layer whose error C is
   PlaneSink sink;
 };
+// dlb_fc_forward and dlb_fc_forward_activation with a say on the order of summation
+// (GemmEpilogue::any_order).
+dlb_status fc_forward(dlb_ctx *ctx, const float *X, const float *X_lo, const float *W, const float *W_lo,
+                      const float *bias, float *Z, int rows, int n_in, int n_out, bool any_order);
+dlb_status fc_forward_activation(dlb_ctx *ctx, const float *X, const float *X_lo, const float *W, const float *W_lo,
+                                 const float *bias, float *Z, int af, const dlb_dropout_desc *dropout, float *A_out,
+                                 float *A_lo, int rows, int n_in, int n_out, bool any_order);
 // dlb_fc_weight_gradient with a say on the planes of the error: rescale_lines
 // asks for planes with a scale per unit (per output row of dW), made for this
 // product (gemm() in ctx.cu).

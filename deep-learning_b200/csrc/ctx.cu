@@ -105,21 +105,28 @@ static bool planes_beat_small(const dlb_ctx *ctx, int M, int N, int K, double pl
 // kernels' own estimates, missing planes made for it.
 enum class Way { SMALL, DIRECT, PLANES, ORDERED };
 static Way gemm_way(const dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B, int M, int N, int K,
-                    bool accumulate, bool have_a, bool have_b) {
+                    const GemmEpilogue &ep, bool have_a, bool have_b) {
   const double small = gemm_small_us(ctx, M, N, K), direct = gemm_direct_us(ctx, M, N, K);
   Way way = small < direct ? Way::SMALL : Way::DIRECT;
   double best = std::min(small, direct);
   if (plane_size(M, N, K) && gemm_pair_enabled() && !(A.stride_k != 1 && B.stride_k == 1)) {
-    const double planes = gemm_planes_us(ctx, A, B, M, N, K, accumulate) +
+    const double planes = gemm_planes_us(ctx, A, B, M, N, K, ep.accumulate) +
                           split_us((have_a ? 0 : (long long)M * K) + (have_b ? 0 : (long long)N * K));
     if (planes <= direct && planes_beat_small(ctx, M, N, K, planes)) way = Way::PLANES, best = planes;
   }
-  // Forward products of a width that TMA cannot address keep their order of summation
-  // as long as the SMs have a tile each and it takes three times the shortest way at
-  // most (333 x 1203 x 1203: 47 us against 21): larger ones have batches in which a unit
-  // more or less on one side of an activation's kink counts less, and would pay more.
+  // Forward products whose pitch TMA cannot address have always been summed in ascending
+  // k, and keep that order (gemm_ordered.cu says what for) wherever a derivative that
+  // jumps may follow and it is cheap: a tile of 64 x 64 per SM at most, since a second
+  // round doubles its time (333 rows of 1203 x 1203 47 us against 21, 449 rows 90 against
+  // 22), and three times the shortest way at most (64 rows, 47 against 15).  The line is
+  // one of cost: on its far side, as at the widths TMA can address, which never had that
+  // order, a unit near the jump falls where the rounding of the sums puts it.
+  // Where no such derivative follows, the shortest way is taken unless it is less accurate:
+  // from float64 the ascending sums are 1.8e-8 sqrt(K) away (in norm), sums on planes
+  // 4.8e-7 and the direct kernel's 2.6e-7 whatever K, so up to K = 711 and 208.
   const bool unaddressable = ((A.stride_mn | B.stride_mn) & 7) != 0;
-  if (A.stride_k == 1 && B.stride_k == 1 && unaddressable && std::min(M, N) >= 64 &&
+  const bool keep = !ep.any_order || (way == Way::PLANES && K < 712) || (way == Way::DIRECT && K < 208);
+  if (keep && A.stride_k == 1 && B.stride_k == 1 && unaddressable && std::min(M, N) >= 64 &&
       ceil_div(M, 64) * (long long)ceil_div(N, 64) <= ctx->sm_count && gemm_ordered_us(ctx, M, N, K) <= 3.0 * best)
     way = Way::ORDERED;
   return way;
@@ -160,7 +167,7 @@ PlaneUse gemm_plane_use(dlb_ctx *ctx, const GemmOperand &A, const GemmOperand &B
   // a check launch each: 4 us a product (an epoch of 128-row batches of 784-256-10
   // takes 1430 us where its largest weight gradient has planes, 1340 where not).
   const bool on = a && b ? planes_beat_small(ctx, M, N, K, gemm_planes_us(ctx, A, B, M, N, K, false) + 4.0)
-                         : gemm_way(ctx, A, B, M, N, K, false, a, b) == Way::PLANES;
+                         : gemm_way(ctx, A, B, M, N, K, GemmEpilogue{}, a, b) == Way::PLANES;
   return {on && a, on && b};
 }
 
@@ -182,7 +189,7 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
   // fills a 256 x 256 tile.  Missing ones are made for this product, with a scale per
   // line, where that and the product on planes are estimated to be shorter than the
   // direct kernel, which reads any pitch and width (1024 x 1000 x 2048: 54 us against 6 and
-  // 17; 333 x 1203 x 1203: 24.8 against 21; 333 x 617 x 1203: 18 the direct way).  An operand
+  // 17; 333 x 1203 x 1203: 24.8 against 21; 2048 x 256 x 256: 11.5 the direct way).  An operand
   // whose caller asks for a scale per line (the classes of a softmax error differ by
   // many orders of magnitude: the ones nobody is wrong about have errors 2^-20 and
   // less of the others', and one scale for the tensor would leave their gradient
@@ -194,7 +201,7 @@ dlb_status gemm(dlb_ctx *ctx, const GemmOperand &A_in, const GemmOperand &B_in, 
       have_b = B.h_hi || (planes_serve(B, N, K, false) && planes_lookup(ctx, B.lo, &B));
     }
     const bool kept = have_a && have_b && gemm_f16_supported(A, B, C, ldc, M, N, K);
-    const Way way = kept ? Way::PLANES : gemm_way(ctx, A, B, M, N, K, ep.accumulate, have_a, have_b);
+    const Way way = kept ? Way::PLANES : gemm_way(ctx, A, B, M, N, K, ep, have_a, have_b);
     if (way == Way::SMALL) return gemm_small(ctx, A_in, B_in, C, ldc, M, N, K, ep);
     if (way == Way::ORDERED) return gemm_ordered(ctx, A_in, B_in, C, ldc, M, N, K, ep);
     if (way == Way::DIRECT) {
@@ -587,12 +594,7 @@ dlb_status dlb_host_free(void *host_ptr) {
 dlb_status dlb_fc_forward(dlb_ctx *ctx, const float *X, const float *X_lo, const float *W,
                           const float *W_lo, const float *bias, float *Z, int rows, int n_in,
                           int n_out) {
-  DLB_REQUIRE(ctx && X && W && Z && rows > 0 && n_in > 0 && n_out > 0, "dlb_fc_forward");
-  GemmOperand A{X, X_lo, n_in, 1};   // (m=b, k=i)
-  GemmOperand B{W, W_lo, n_in, 1};   // (n=o, k=i)
-  GemmEpilogue ep;
-  ep.bias = bias;
-  return gemm(ctx, A, B, Z, n_out, rows, n_out, n_in, ep);
+  return fc_forward(ctx, X, X_lo, W, W_lo, bias, Z, rows, n_in, n_out, false);
 }
 
 dlb_status dlb_fc_backward_input(dlb_ctx *ctx, const float *delta, const float *delta_lo,
@@ -632,31 +634,7 @@ dlb_status dlb_fc_forward_activation(dlb_ctx *ctx, const float *X, const float *
                                      const float *W_lo, const float *bias, float *Z, int af,
                                      const dlb_dropout_desc *dropout, float *A_out, float *A_lo, int rows,
                                      int n_in, int n_out) {
-  DLB_REQUIRE(ctx && X && W && Z && A_out && rows > 0 && n_in > 0 && n_out > 0, "dlb_fc_forward_activation");
-  GemmOperand A{X, X_lo, n_in, 1};
-  GemmOperand B{W, W_lo, n_in, 1};
-  FusedEpilogue fe;
-  fe.mode = EPI_ACTIVATION;
-  fe.af = af;
-  fe.out = A_out;
-  const uintptr_t all = reinterpret_cast<uintptr_t>(Z) | reinterpret_cast<uintptr_t>(A_out) |
-                        reinterpret_cast<uintptr_t>(dropout ? dropout->noise : nullptr);
-  // (the epilogue moves quads of a row)
-  if (A_lo && n_out % 4 == 0 && (all & 15) == 0 && epilogue_dropout(dropout, &fe) && gemm_fused_supported(ctx, A, B, Z, n_out, rows, n_out, n_in)) {
-    PlaneJob job;
-    DLB_TRY(planes_open(ctx, A_out, A_lo, (size_t)rows * n_out, rows, n_out, true, &job));
-    if (job.fused || !job.active) {  // (inactive: nobody reads A's planes, the epilogue writes none)
-      fe.sink = job.sink;
-      GemmEpilogue ep;
-      ep.bias = bias;
-      ep.fused = &fe;
-      DLB_TRY(gemm(ctx, A, B, Z, n_out, rows, n_out, n_in, ep));
-      return planes_close(ctx, job);
-    }
-    // No scale to predict from yet (the buffer's first split): the two kernels below.
-  }
-  DLB_TRY(dlb_fc_forward(ctx, X, X_lo, W, W_lo, bias, Z, rows, n_in, n_out));
-  return dlb_activation_forward(ctx, Z, nullptr, af, dropout, A_out, A_lo, rows, n_out);
+  return fc_forward_activation(ctx, X, X_lo, W, W_lo, bias, Z, af, dropout, A_out, A_lo, rows, n_in, n_out, false);
 }
 
 dlb_status dlb_fc_backward_input_derivative(dlb_ctx *ctx, const float *delta, const float *delta_lo,
@@ -696,6 +674,48 @@ dlb_status dlb_fc_weight_gradient(dlb_ctx *ctx, const float *delta, const float 
 }
 
 }  // extern "C"
+
+dlb_status dlb::fc_forward(dlb_ctx *ctx, const float *X, const float *X_lo, const float *W, const float *W_lo,
+                           const float *bias, float *Z, int rows, int n_in, int n_out, bool any_order) {
+  DLB_REQUIRE(ctx && X && W && Z && rows > 0 && n_in > 0 && n_out > 0, "dlb_fc_forward");
+  GemmOperand A{X, X_lo, n_in, 1};   // (m=b, k=i)
+  GemmOperand B{W, W_lo, n_in, 1};   // (n=o, k=i)
+  GemmEpilogue ep;
+  ep.bias = bias;
+  ep.any_order = any_order;
+  return gemm(ctx, A, B, Z, n_out, rows, n_out, n_in, ep);
+}
+
+dlb_status dlb::fc_forward_activation(dlb_ctx *ctx, const float *X, const float *X_lo, const float *W,
+                                      const float *W_lo, const float *bias, float *Z, int af,
+                                      const dlb_dropout_desc *dropout, float *A_out, float *A_lo, int rows, int n_in,
+                                      int n_out, bool any_order) {
+  DLB_REQUIRE(ctx && X && W && Z && A_out && rows > 0 && n_in > 0 && n_out > 0, "dlb_fc_forward_activation");
+  GemmOperand A{X, X_lo, n_in, 1};
+  GemmOperand B{W, W_lo, n_in, 1};
+  FusedEpilogue fe;
+  fe.mode = EPI_ACTIVATION;
+  fe.af = af;
+  fe.out = A_out;
+  const uintptr_t all = reinterpret_cast<uintptr_t>(Z) | reinterpret_cast<uintptr_t>(A_out) |
+                        reinterpret_cast<uintptr_t>(dropout ? dropout->noise : nullptr);
+  // (the epilogue moves quads of a row)
+  if (A_lo && n_out % 4 == 0 && (all & 15) == 0 && epilogue_dropout(dropout, &fe) && gemm_fused_supported(ctx, A, B, Z, n_out, rows, n_out, n_in)) {
+    PlaneJob job;
+    DLB_TRY(planes_open(ctx, A_out, A_lo, (size_t)rows * n_out, rows, n_out, true, &job));
+    if (job.fused || !job.active) {  // (inactive: nobody reads A's planes, the epilogue writes none)
+      fe.sink = job.sink;
+      GemmEpilogue ep;
+      ep.bias = bias;
+      ep.fused = &fe;
+      DLB_TRY(gemm(ctx, A, B, Z, n_out, rows, n_out, n_in, ep));
+      return planes_close(ctx, job);
+    }
+    // No scale to predict from yet (the buffer's first split): the two kernels below.
+  }
+  DLB_TRY(fc_forward(ctx, X, X_lo, W, W_lo, bias, Z, rows, n_in, n_out, any_order));
+  return dlb_activation_forward(ctx, Z, nullptr, af, dropout, A_out, A_lo, rows, n_out);
+}
 
 dlb_status dlb::fc_weight_gradient_lines(dlb_ctx *ctx, const float *delta, const float *delta_lo, const float *X,
                                          const float *X_lo, float *dW, float *dbias, int rows, int n_in, int n_out,

@@ -1,12 +1,14 @@
 // Forward products in fp32 with every sum in ascending k, bit for bit what
 // gemm_simt.cuh gives, for widths that TMA cannot address and moderate sizes.
 //
-// Why the order matters: a derivative that jumps at 0 (ELU' from 1 to 0, SELU', the
-// leaky ReLU's) makes a unit's error depend on which side of 0 its pre-activation
-// falls, and sums in another order, however accurate, put a few in a million on the
-// other side.  In a batch of a few hundred rows one such unit of an upper layer moves
-// every weight's first Adam steps by some 5 %.  So the products that have always run
-// in this order keep it where that costs little.
+// What the order is for: a derivative that jumps at 0 (ReLU', the leaky ReLU's, ELU' from
+// 1 to 0, SELU') makes a unit's error depend on which side of 0 its pre-activation falls,
+// and sums in another order, however accurate, put a few in a million on the other side;
+// in a batch of 333 rows one such unit moved the weights after four Adam steps by up to
+// 3e-4.  Neither side is the better one.  But these products ran in this order before they
+// had another way (as the reference's own loops do), and training on such widths keeps
+// giving what it gave where that is cheap (gemm_way in ctx.cu has the line).  Evaluation
+// and models without such a derivative take the shortest way that is as accurate.
 //
 // A CTA forms 64 x 64: four warps of 8 x 4 sums per lane read and multiply, four others
 // bring 32 k of both operands at a time, k-major, two slabs ahead (with the loads done by

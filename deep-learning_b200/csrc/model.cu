@@ -60,6 +60,14 @@ bool is_lstm(const LayerRT &l) { return l.type == DLB_LAYER_LSTM; }
 bool class_error(const dlb_model *m, size_t i) {
   return i + 1 == m->layers.size() && m->layers[i].af == DLB_AF_SOFTMAX;
 }
+// Whether the order in which a forward product sums is free: no backward pass follows, or
+// no layer's derivative jumps at 0 (a lower layer's rounding decides an upper layer's side).
+bool any_order(const dlb_model *m) {
+  if (m->propagation == DLB_PROPAGATION_INFERENCE) return true;
+  for (const LayerRT &l : m->layers)
+    if (l.af == DLB_AF_RELU || l.af == DLB_AF_LEAKY_RELU || l.af == DLB_AF_ELU || l.af == DLB_AF_SELU) return false;
+  return true;
+}
 size_t lstm_gates(const LayerRT &l) { return l.units + 3 * l.blocks; }
 
 // Bounds the recurrent weights of an IndRNN layer are clamped to after an
@@ -694,8 +702,8 @@ dlb_status forward_residual(dlb_model *m, size_t i, const float *X, const float 
       in_lo = b.IN_lo;
     }
     const float *bias = norm ? nullptr : m->params + b.first_bias;
-    DLB_TRY(dlb_fc_forward(m->ctx, in, in_lo, m->params + b.first_conn, m->params_lo + b.first_conn,
-                           bias, b.A, B, (int)b.fan_in, (int)b.units));
+    DLB_TRY(fc_forward(m->ctx, in, in_lo, m->params + b.first_conn, m->params_lo + b.first_conn, bias, b.A, B,
+                       (int)b.fan_in, (int)b.units, any_order(m)));
     prev_sums = b.A;
   }
   LayerRT &last = m->layers[i + res.depth];
@@ -797,8 +805,8 @@ dlb_status forward_residual_time(dlb_model *m, size_t i, const float *X, const f
       in_lo = b.IN_lo;
     }
     const float *bias = norm ? nullptr : m->params + b.first_bias;
-    DLB_TRY(dlb_fc_forward(m->ctx, in, in_lo, m->params + b.first_conn, m->params_lo + b.first_conn, bias, b.A, TB,
-                           (int)b.fan_in, (int)b.units));
+    DLB_TRY(fc_forward(m->ctx, in, in_lo, m->params + b.first_conn, m->params_lo + b.first_conn, bias, b.A, TB,
+                       (int)b.fan_in, (int)b.units, any_order(m)));
     prev_sums = b.A;
   }
   LayerRT &last = m->layers[i + res.depth];
@@ -836,14 +844,15 @@ dlb_status forward_lstm(dlb_model *m, LayerRT &l, const float *X, const float *X
   DLB_TRY(dlb_gather_rows(m->ctx, m->params, l.lstm_map_rec, l.lstm_wrec, (size_t)G, C));
   DLB_TRY(dlb_gather_rows(m->ctx, m->params, l.lstm_map_bias, l.lstm_bias, (size_t)G, 1));
   DLB_TRY(dlb_gather_rows(m->ctx, m->params, l.lstm_map_peep, l.lstm_peep, (size_t)3 * C, 1));
-  DLB_TRY(dlb_fc_forward(m->ctx, X, X_lo, l.lstm_wff, nullptr, nullptr, l.lstm_gin, T * B, I, G));
+  DLB_TRY(fc_forward(m->ctx, X, X_lo, l.lstm_wff, nullptr, nullptr, l.lstm_gin, T * B, I, G, any_order(m)));
   const size_t sc = (size_t)B * C, sb = (size_t)B * l.blocks, sg = (size_t)B * G;
   bool walked = false;
   DLB_TRY(lstm_forward_walk(m->ctx, l.lstm_gin, l.lstm_wrec, l.lstm_bias, l.lstm_peep, l.lstm_z, l.lstm_c, l.lstm_ca,
                             l.A, l.lstm_gi, l.lstm_gf, l.lstm_go, B, T, (int)l.blocks, (int)l.cells, &walked));
   for (int t = 0; t < T && !walked; ++t) {
     if (t > 0)
-      DLB_TRY(dlb_fc_forward(m->ctx, l.A + (t - 1) * sc, nullptr, l.lstm_wrec, nullptr, nullptr, l.lstm_grec, B, C, G));
+      DLB_TRY(fc_forward(m->ctx, l.A + (t - 1) * sc, nullptr, l.lstm_wrec, nullptr, nullptr, l.lstm_grec, B, C, G,
+                         any_order(m)));
     DLB_TRY(dlb_lstm_forward_step(m->ctx, l.lstm_gin + t * sg, t ? l.lstm_grec : nullptr, l.lstm_bias, l.lstm_peep,
                                   t ? l.lstm_c + (t - 1) * sc : nullptr, l.lstm_z + t * sc, l.lstm_c + t * sc,
                                   l.lstm_ca + t * sc, l.A + t * sc, l.lstm_gi + t * sb, l.lstm_gf + t * sb,
@@ -935,8 +944,8 @@ dlb_status forward_layers_time(dlb_model *m, size_t rows) {
     const bool norm = l.norm != DLB_NORM_NONE;
     const bool last = i + 1 == m->layers.size();
     const float *bias = norm ? nullptr : m->params + l.first_bias;
-    DLB_TRY(dlb_fc_forward(m->ctx, X, X_lo, m->params + l.first_conn, m->params_lo + l.first_conn,
-                           bias, l.Z, TB, I, H));
+    DLB_TRY(fc_forward(m->ctx, X, X_lo, m->params + l.first_conn, m->params_lo + l.first_conn, bias, l.Z, TB, I, H,
+                       any_order(m)));
     if (l.af == DLB_AF_SOFTMAX) {
       DLB_TRY(dlb_softmax_forward(m->ctx, l.Z, l.A, TB, H));
     } else if (norm || is_indrnn(l) || l.dropout != DLB_DROPOUT_NONE) {
@@ -1012,15 +1021,15 @@ dlb_status forward_layers(dlb_model *m, size_t rows) {
       // in the product's epilogue (where the kernel that runs has one).
       DLB_TRY(uout_ready(m, l, i, B));
       dlb_dropout_desc dp{l.dropout, l.dropout_value, l.mask, l.uout};
-      DLB_TRY(dlb_fc_forward_activation(m->ctx, X, X_lo, m->params + l.first_conn, m->params_lo + l.first_conn,
-                                        bias, l.Z, l.af, l.dropout != DLB_DROPOUT_NONE ? &dp : nullptr, l.A,
-                                        l.A_lo, B, I, H));
+      DLB_TRY(fc_forward_activation(m->ctx, X, X_lo, m->params + l.first_conn, m->params_lo + l.first_conn, bias,
+                                    l.Z, l.af, l.dropout != DLB_DROPOUT_NONE ? &dp : nullptr, l.A, l.A_lo, B, I, H,
+                                    any_order(m)));
       X = l.A;
       X_lo = l.A_lo;
       continue;
     }
-    DLB_TRY(dlb_fc_forward(m->ctx, X, X_lo, m->params + l.first_conn, m->params_lo + l.first_conn,
-                           bias, l.Z, B, I, H));
+    DLB_TRY(fc_forward(m->ctx, X, X_lo, m->params + l.first_conn, m->params_lo + l.first_conn, bias, l.Z, B, I, H,
+                       any_order(m)));
     dlb_brn_unit_arrays u;
     if (norm) DLB_TRY(norm_statistics(m, l, l.Z, B, &u));
     if (l.af == DLB_AF_SOFTMAX) {
