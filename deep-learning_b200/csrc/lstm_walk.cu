@@ -15,9 +15,10 @@
 // The exchange is by st.async onto an mbarrier that counts the bytes of a step, not
 // by stores and a cluster barrier: the barrier's release waits until this step's
 // stores to global memory are visible too, 6 us a step in all where this form takes
-// 2.9 forward and 3.3 backward (64 examples, 128 blocks of 2 cells; of the 5000 cycles
-// 1600 are the sums, 1600 the cells' chain of five squashing functions, 700 the loads
-// and stores of the step, 1000 the exchange).  The copies and their barriers alternate: a
+// 2.5 forward and 2.9 backward (64 examples, 128 blocks of 2 cells).  What bounds a step
+// is one chain: inputs, the sums (about 115 cycles per example and 128 k), five squashing
+// functions in a row, the exchange; all but the sums take 2800 cycles of the 4700 (the
+// fit in plan_walk).  The copies and their barriers alternate: a
 // CTA sends its part of step t + 2 only after it has all of step t + 1, so every
 // other CTA has read step t by then.
 //
@@ -267,10 +268,10 @@ struct Exchange {
   // No CTA leaves while another may still send to it; after a wait that ran out the
   // barrier says nothing about the values in flight.
   __device__ __forceinline__ void finish() const {
-    if (cs == 1) return;
-    __syncwarp();
-    tc::cluster_sync_all();
-    if (*static_cast<volatile int *>(abort_flag)) tc::drain_pause();
+    if (cs > 1) {
+      tc::cluster_sync_all();
+      if (*static_cast<volatile int *>(abort_flag)) tc::drain_pause();
+    }
   }
 };
 
@@ -512,14 +513,21 @@ struct WalkPlan {
 constexpr size_t W_SMEM_MAX = 226 * 1024;  // beside the barriers
 
 // Rows of a warp, and up to how many chunks of k its registers hold of them (0: the
-// weights lie in shared memory): as many as 128 registers have room for beside the sums
-// of EX examples.
+// weights lie in shared memory).  A lane keeps ROWS x CHUNKS quads of weights beside the
+// sums of ROWS x EX examples: about 10 quads, 40 of its 128 registers, leave room for 32
+// sums, about 20 for 10, so those take more rows or a longer k but fewer examples.  Either
+// number is divided between rows and chunks in the ways that some layer measured fastest
+// with: 63 layers of 8 - 300 blocks of 1 - 3 cells at 8, 64 and 200 examples, every plan
+// of both directions.  (4 x 5, 5 x 4, 1 x 10, 10 x 1 and 20 x 1 never won by more than 2 %.)
 struct WarpRows {
   int rows, chunks;
 };
-constexpr WarpRows W_FORMS[] = {{5, 2}, {2, 5}, {10, 2}, {4, 5}, {4, 0}};
-constexpr int W_NUM_FORMS = 5;
-constexpr bool form_exists(int form, int ex) { return W_FORMS[form].rows * ex <= (W_FORMS[form].chunks * W_FORMS[form].rows > 10 ? 20 : 32); }
+constexpr WarpRows W_FORMS[] = {{5, 2}, {3, 3}, {2, 5}, {10, 2}, {6, 3}, {3, 6}, {2, 10}, {4, 0}};
+constexpr int W_NUM_FORMS = sizeof(W_FORMS) / sizeof(W_FORMS[0]);
+constexpr bool form_dense(int form) { return W_FORMS[form].rows * W_FORMS[form].chunks > 10; }
+constexpr bool form_exists(int form, int ex) {
+  return W_FORMS[form].rows * ex <= (form_dense(form) ? 10 : 32);
+}
 
 template <int EX, int FORM>
 constexpr auto walk_kernel(const ForwardWalk &) {
@@ -539,10 +547,13 @@ int walk_clusters(const dlb_ctx *ctx, int cs) {
   return n;
 }
 
-// The fastest layout by the cost of a step: a fixed part (cells, exchange), the
-// fused multiply-adds, 128 a cycle, the shared-memory reads of the sums, 128 bytes
-// a cycle, and the sums over lanes, times the rounds that the examples need.  None if
-// the weights do not fit.
+// The fastest layout by the cost of a step in cycles, fitted to the plans of the layers
+// above within 2 x of their fastest (the plan it picks takes 1.8 % longer than the fastest
+// on average, 32 % at worst): cells and exchange; a chain of loads and multiply-adds per
+// example and 128 k, times the rounds of rows per warp; the sums over lanes; the
+// weights read from shared memory; and what the dense forms lose to spills.  Times the
+// rounds that the examples need of the CTAs that run at once.  None if the weights do
+// not fit.
 WalkPlan plan_walk(const dlb_ctx *ctx, const WalkShape &s, int rows_per_block, int pitch) {
   WalkPlan best;
   if (s.kp > 32) return best;
@@ -553,18 +564,23 @@ WalkPlan plan_walk(const dlb_ctx *ctx, const WalkShape &s, int rows_per_block, i
         WalkPlan p;
         p.ex = ex, p.cs = cs, p.form = form;
         const int per_warp = W_FORMS[form].rows, chunks = W_FORMS[form].chunks;
-        const int nb = ceil_div(s.B, cs), rows = nb * rows_per_block;
-        const int sum_threads = ceil_div(rows, per_warp) * 32, cell_threads = ceil_div(ex * nb * s.kp, 32) * 32;
-        p.threads = std::min(W_THREADS, std::max(sum_threads, cell_threads));
-        if (chunks && (sum_threads > W_THREADS || pitch > chunks * 128)) continue;
+        const int nb = ceil_div(s.B, cs), rows = nb * rows_per_block, warps = ceil_div(rows, per_warp);
+        const int cell_threads = ceil_div(ex * nb * s.kp, 32) * 32;
+        p.threads = std::min(W_THREADS, std::max(warps * 32, cell_threads));
+        if (chunks && (warps * 32 > W_THREADS || pitch > chunks * 128)) continue;
         p.smem = walk_floats(ex, chunks > 0, rows, pitch) * sizeof(float);
         if (p.smem > W_SMEM_MAX || cell_threads > W_THREADS) continue;
-        const long long groups = ((long long)s.rows + ex - 1) / ex, at_once = walk_clusters(ctx, cs);
-        const long long rounds = (groups + at_once - 1) / at_once;
-        const double fma = (double)rows * pitch * ex / 128;
-        const double reads = (double)pitch / 32 * (ceil_div(rows, per_warp) * ex + (chunks ? 0 : rows));
-        const double cycles = 2700.0 + (cs > 1 ? 600.0 : 0.0) + fma + reads + 2.0 * rows * ex;
-        p.us = 3.0 + (double)rounds * (3.0 + s.T * cycles / 1900.0);
+        // CTAs of an SM: by the registers (128 a thread) and the shared memory.
+        const int per_sm = std::max(1, std::min(W_THREADS / (ceil_div(p.threads, 128) * 128), (int)(W_SMEM_MAX / (p.smem + 1024))));
+        const long long groups = ((long long)s.rows + ex - 1) / ex, one_each = walk_clusters(ctx, cs);
+        const long long rounds = (groups + one_each * per_sm - 1) / (one_each * per_sm);
+        const double share = (double)std::min<long long>(per_sm, (groups + one_each - 1) / one_each);
+        const int pieces = pitch / 128, passes = ceil_div(warps, p.threads / 32);
+        double cycles = 2500.0 + (cs > 1 ? 310.0 : 0.0) + 115.0 * passes * pieces * ex +
+                        5.6 * share * ceil_div(warps, 4) * per_warp * ex;
+        if (!chunks) cycles += 10.6 * share * rows * pieces + ((ex >= 4 ? 80.0 : 0.0) + (ex == 8 ? 325.0 : 0.0)) * passes * pieces;
+        if (form_dense(form)) cycles += 385.0 + (135.0 + 70.0 * ex) * pieces;
+        p.us = 3.0 + (double)rounds * s.T * cycles / 1900.0;
         if (p.us < best.us) best = p;
       }
   return best;
@@ -599,16 +615,16 @@ dlb_status launch_walk(dlb_ctx *ctx, const Walk &walk, const WalkPlan &p) {
   }
   return launch_walk<8, FORM>(ctx, walk, p);
 }
+template <int FORM, class Walk>
+dlb_status launch_form(dlb_ctx *ctx, const Walk &walk, const WalkPlan &p) {
+  if constexpr (FORM + 1 < W_NUM_FORMS)
+    if (p.form != FORM) return launch_form<FORM + 1>(ctx, walk, p);
+  return launch_walk<FORM>(ctx, walk, p);
+}
 template <class Walk>
 dlb_status run_walk(dlb_ctx *ctx, Walk walk, const WalkPlan &p) {
   walk.s.cs = p.cs, walk.s.status = ctx->d_status;
-  switch (p.form) {
-    case 0: return launch_walk<0>(ctx, walk, p);
-    case 1: return launch_walk<1>(ctx, walk, p);
-    case 2: return launch_walk<2>(ctx, walk, p);
-    case 3: return launch_walk<3>(ctx, walk, p);
-  }
-  return launch_walk<4>(ctx, walk, p);
+  return launch_form<0>(ctx, walk, p);
 }
 
 WalkShape walk_shape(int rows, int T, int blocks, int cells) {
@@ -619,7 +635,7 @@ WalkShape walk_shape(int rows, int T, int blocks, int cells) {
 
 // A step on its own: its product, and a launch of the cells' kernel.
 double step_by_step_us(const dlb_ctx *ctx, const WalkShape &s, int N, int K) {
-  return (double)s.T * (gemm_direct_us(ctx, s.rows, N, K) + 5.0);
+  return (double)s.T * (std::min(gemm_small_us(ctx, s.rows, N, K), gemm_direct_us(ctx, s.rows, N, K)) + 5.0);
 }
 
 }  // namespace

@@ -25,3 +25,37 @@ def test_walk_matches_restatement(gpu_ctx, rows, seq_w, blocks, cells):
     got = util.trace(util.build(dlb200.Model(gpu_ctx), cfg, params=p0), cfg, 1, X, Y)
     assert gpu_ctx.sync() == 0
     _check(got, want, cfg)
+
+
+# Sizes at which the plan takes each form (rows per warp x chunks of 128 k in registers, or
+# weights in shared memory) with few and with many examples per cluster: forward / backward.
+@pytest.mark.parametrize("rows,blocks,cells", [
+    (5, 150, 2),   # 6 x 3 / 3 x 6
+    (5, 200, 1),   # 10 x 2 / 2 x 10
+    (16, 250, 1),  # shared memory / 2 x 10, two examples
+    (16, 150, 2),  # shared memory / 3 x 6, two examples
+    (40, 60, 3),   # 3 x 3, four examples / 3 x 3, two
+    (200, 30, 3),  # 3 x 3, eight examples / 3 x 3, four
+    (200, 99, 1),  # shared memory, eight examples / 2 x 5, eight
+    (64, 128, 1),  # 5 x 2, five examples / 2 x 5
+    (40, 150, 1),  # 5 x 2 / 2 x 5, four examples
+    (150, 99, 1),  # shared memory, five examples / 2 x 5, five
+])
+def test_forms_of_the_walk(gpu_ctx, rows, blocks, cells):
+    launches = []
+    for seq_w in (2, 4):
+        cfg = configs.lstm_stack(n_in=24, blocks=blocks, cells=cells, depth=1, n_out=blocks * cells + 3, seq_w=seq_w,
+                                 batch=rows)
+        X, Y = configs.synthetic_batch(cfg)
+        p0 = _random_parameters(cfg)
+        want = util.trace(util.build(fc_lstm.LstmOracleModel(), cfg, params=p0), cfg, 1, X, Y)
+        model = util.build(dlb200.Model(gpu_ctx), cfg, params=p0)
+        _check(util.trace(model, cfg, 1, X, Y), want, cfg)
+        before = gpu_ctx.launch_count()
+        model.forward_pass(rows, X)
+        model.compute_error(rows, Y)
+        model.backward_pass(rows)
+        assert gpu_ctx.sync() == 0
+        launches.append(gpu_ctx.launch_count() - before)
+    # one launch per direction walks over all time steps
+    assert launches[1] - launches[0] <= 1
