@@ -43,6 +43,7 @@ struct dlb_ctx {
     float *scale;
     int rows = 0, cols = 0;
     unsigned *lines = nullptr;  // [rows] row maxima, then [cols] column maxima (raw bits of |x|)
+    size_t line_words = 0;      // words allocated for them
     bool seen = false;          // a split has completed: the slot holds a scale predicted for the next one
   };
   std::map<uintptr_t, PlaneEntry> planes;

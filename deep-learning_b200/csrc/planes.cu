@@ -452,10 +452,28 @@ static void sink_lines(PlaneSink &k, unsigned *lines, int rows, int cols, bool e
   k.rows_exempt = exempt ? 1 : 0;
 }
 
+// Room for the line maxima of a [rows, cols] tensor; they are zero between splits.
+static dlb_status entry_lines(dlb_ctx *ctx, dlb_ctx::PlaneEntry &e) {
+  const size_t need = (size_t)e.rows + e.cols;
+  if (e.rows == 0 || need <= e.line_words) return DLB_OK;
+  if (e.lines) {
+    DLB_CUDA(cudaStreamSynchronize(ctx->stream));  // a check kernel may still read the array
+    DLB_CUDA(cudaFree(e.lines));
+    e.lines = nullptr;
+    e.line_words = 0;
+  }
+  DLB_CUDA(cudaMalloc(&e.lines, need * sizeof(unsigned)));
+  e.line_words = need;
+  DLB_CUDA(cudaMemsetAsync(e.lines, 0, need * sizeof(unsigned), ctx->stream));
+  return DLB_OK;
+}
+
 // Registers `planes` as the plane buffer of x[0..n) with the given shape (0, 0:
-// none) and fills the job.  A registration of the same tensor, size and shape
-// is kept, with its predicted scale; anything else this buffer overlaps is
-// stale and dropped.
+// none) and fills the job.  A registration of the same tensor and width is kept, with
+// its predicted scale, also where the number of rows differs (a longer last batch of an
+// epoch: dropped, it cost a cudaFree, a cudaMalloc and the fused form of the producing
+// kernel, twice an epoch for every tensor); anything else this buffer overlaps is stale
+// and dropped.
 dlb_status planes_open(dlb_ctx *ctx, const float *x, float *planes, size_t n, int rows, int cols,
                        bool kernel_can_fuse, PlaneJob *job) {
   DLB_REQUIRE(x && planes && n > 0 && n < ((size_t)1 << 40), "plane buffer: tensor, buffer and size");
@@ -472,10 +490,17 @@ dlb_status planes_open(dlb_ctx *ctx, const float *x, float *planes, size_t n, in
     if (before->first + before->second.n * sizeof(float) > key) planes_forget(ctx, before->first, 1);
   }
   auto it = ctx->planes.find(key);
-  if (it != ctx->planes.end() &&
-      (it->second.x != x || it->second.n != n || it->second.rows != rows || it->second.cols != cols)) {
-    planes_forget(ctx, key, 1);
-    it = ctx->planes.end();
+  if (it != ctx->planes.end()) {
+    dlb_ctx::PlaneEntry &e = it->second;
+    const bool same = e.x == x && e.n == n && e.rows == rows && e.cols == cols;
+    if (!same && e.x == x && e.cols == cols && e.rows > 0 && rows > 0) {
+      e.n = n;
+      e.rows = rows;
+      DLB_TRY(entry_lines(ctx, e));
+    } else if (!same) {
+      planes_forget(ctx, key, 1);
+      it = ctx->planes.end();
+    }
   }
   if (it == ctx->planes.end()) {
     dlb_ctx::PlaneEntry e;
@@ -485,10 +510,7 @@ dlb_status planes_open(dlb_ctx *ctx, const float *x, float *planes, size_t n, in
     e.cols = cols;
     DLB_TRY(scale_slot(ctx, &e.scale));
     DLB_CUDA(cudaMemsetAsync(e.scale, 0, SLOT_WORDS * sizeof(float), ctx->stream));
-    if (rows > 0) {
-      DLB_CUDA(cudaMalloc(&e.lines, (size_t)(rows + cols) * sizeof(unsigned)));
-      DLB_CUDA(cudaMemsetAsync(e.lines, 0, (size_t)(rows + cols) * sizeof(unsigned), ctx->stream));
-    }
+    DLB_TRY(entry_lines(ctx, e));
     it = ctx->planes.emplace(key, e).first;
   }
   dlb_ctx::PlaneEntry &e = it->second;

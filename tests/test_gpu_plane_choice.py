@@ -37,3 +37,29 @@ def test_batches_that_do_and_do_not_keep_planes(gpu_ctx, norm):
         assert abs(losses[0] - losses[1]) <= 2e-5 * abs(losses[1]), rows
     assert gpu_ctx.sync() == 0
     assert util.rel_l2(mod.get_array("parameters"), ora.get_array("parameters")) <= 1e-4
+
+
+@pytest.mark.parametrize("norm", [True, False], ids=["normalised", "plain"])
+def test_a_change_of_rows_keeps_the_registrations(gpu_ctx, norm):
+    """Batches of two sizes, both of which keep planes: after the first step at either, a
+    step launches the same kernels whether the rows changed before it or not (a producer
+    whose registration is dropped cannot write the planes itself), and the weights
+    follow the restatement's."""
+    cfg = configs.deep_brn_mlp(256, 512, 2, 256, 640, af=ACTIVATION.ISRLU, optimizer=OPTIMIZER.ADAM, dropout=None,
+                               norm=norm)
+    X, Y = configs.synthetic_batch(cfg)
+    mod = util.build(dlb200.Model(gpu_ctx), cfg, seed=0)
+    ora = util.build(fc_step.OracleModel(), cfg, params=mod.get_array("parameters"))
+    sizes = (640, 640, 640, 512, 512, 512, 640, 512, 640, 512)
+    launches = []
+    for m in (mod, ora):
+        m.train_begin(cfg["batch"])
+        for rows in sizes:
+            before = gpu_ctx.launch_count()
+            m.train_step(rows, X[:rows], Y[:rows])
+            launches.append(gpu_ctx.launch_count() - before)
+    assert gpu_ctx.sync() == 0
+    for rows in (640, 512):
+        steps = [n for r, n in zip(sizes, launches) if r == rows]
+        assert set(steps[1:]) == {steps[2]}
+    assert util.rel_l2(mod.get_array("parameters"), ora.get_array("parameters")) <= 1e-4
