@@ -1071,9 +1071,11 @@ HostWorkers::~HostWorkers() {
 
 // A thread that sleeps takes 30 - 60 us to wake, as long as 1 MB takes to gather, and a
 // step gathers its inputs and, a hundred microseconds later, its targets.  So both
-// sides look for 200 us before they sleep: the workers for the next gather, the caller
-// for the end of this one.  With 1024 rows of 1 KB the device waited 60 - 135 us for the
-// inputs and 34 - 93 for the targets, now 60 - 70 and 17 - 39.
+// sides look for 200 us before they sleep: one worker for the next gather (it and the
+// caller begin; the others wake meanwhile), the caller for the end of this one.  1024-wide
+// stack on 1024 rows by row pointers, four steps: 2072 us with nobody looking, 2053 with one
+// worker, 2034 with all seven, which would be 56 busy threads beside the program's own where
+// eight ranks share a host.
 template <class Ready>
 static void spin_until(Ready ready) {
   constexpr auto SPIN = std::chrono::microseconds(200);
@@ -1089,10 +1091,12 @@ void HostWorkers::loop() {
   std::unique_lock<std::mutex> lock(mu_);
   bool worked = false;
   for (;;) {
-    if (worked && !stop_ && !(fn_ && next_ < parts_)) {
+    if (worked && !polled_ && !stop_ && !(fn_ && next_ < parts_)) {
+      polled_ = true;
       lock.unlock();
       spin_until([this] { return open_.load(std::memory_order_acquire); });
       lock.lock();
+      polled_ = false;
     }
     work_.wait(lock, [this] { return stop_ || (fn_ && next_ < parts_); });
     if (stop_) return;

@@ -36,6 +36,7 @@ class HostWorkers {
   // Written under mu_; read without it by threads that look before they sleep.
   std::atomic<size_t> finished_{0};
   std::atomic<bool> open_{false};  // parts left to take
+  bool polled_ = false;            // a thread looks at open_
   bool stop_ = false;
 };
 
