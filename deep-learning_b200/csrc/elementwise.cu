@@ -44,6 +44,10 @@ constexpr size_t column_reduce_shared_bytes() {
   return ring > fold ? ring : fold;
 }
 
+// Whether an operation's tensors allow 16-byte loads where n is a multiple of 4.
+template <class Op>
+constexpr bool reads_quads = true;
+
 // ONE: all rows in one chunk by plain loads, folded into double every Op::IN_FLIGHT rows.
 template <int NSUM, class Op, class Fin, bool ONE>
 __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, Op::MIN_BLOCKS)
@@ -62,7 +66,7 @@ __global__ void __launch_bounds__(CR_LANES_X *CR_LANES_Y, Op::MIN_BLOCKS)
   double whole[ONE ? NSUM : 1][4] = {};
 
   if (col < n) {
-    if ((n & 3) == 0) {
+    if (reads_quads<Op> && (n & 3) == 0) {
       typename Op::Cols4 c;
       op.load_cols4(col, c);
       // The rows come through the thread's copy ring (Op::DEPTH - 1 rows of
@@ -230,7 +234,7 @@ static int column_reduce_per_sm() {
 // Whether the kernel folds into double as it goes when all rows are one chunk.
 template <class Op>
 static bool column_one_chunk(int n) {
-  return Op::DEPTH == 0 && (n & 3) == 0;
+  return reads_quads<Op> && Op::DEPTH == 0 && (n & 3) == 0;
 }
 
 // fin(column, n, sums) runs once per column, in the last kernel of the reduction.  The
@@ -321,6 +325,11 @@ struct SumOp {
     acc[0] += X[(size_t)r * n + col];
   }
 };
+
+// The same of a tensor that is not 16-byte aligned: column by column.
+struct UnalignedSumOp : SumOp {};
+template <>
+constexpr bool reads_quads<UnalignedSumOp> = false;
 
 // Per-column constants of a batch-renormalised unit.
 struct BrnCol {
@@ -1388,6 +1397,8 @@ namespace dlb {
 // Column sum of delta into the bias gradient (used by dlb_fc_weight_gradient).
 dlb_status bias_gradient(dlb_ctx *ctx, const float *delta, int rows, int n, float *dbias,
                          int accumulate) {
+  if (reinterpret_cast<uintptr_t>(delta) & 15)
+    return column_reduce<1>(ctx, UnalignedSumOp{{delta, n}}, rows, n, BiasGrad{dbias, accumulate});
   return column_reduce<1>(ctx, SumOp{delta, n}, rows, n, BiasGrad{dbias, accumulate});
 }
 }  // namespace dlb
