@@ -517,7 +517,7 @@ constexpr size_t W_SMEM_MAX = 226 * 1024;  // beside the barriers
 // sums of ROWS x EX examples: about 10 quads, 40 of its 128 registers, leave room for 32
 // sums, about 20 for 10, so those take more rows or a longer k but fewer examples.  Either
 // number is divided between rows and chunks in the ways that some layer measured fastest
-// with: 63 layers of 8 - 300 blocks of 1 - 3 cells at 8, 64 and 200 examples, every plan
+// with: 79 layers of 8 - 300 blocks of 1 - 3 cells at 8, 64 and 200 examples, every plan
 // of both directions.  (4 x 5, 5 x 4, 1 x 10, 10 x 1 and 20 x 1 never won by more than 2 %.)
 struct WarpRows {
   int rows, chunks;
