@@ -118,7 +118,8 @@ static Way gemm_way(const dlb_ctx *ctx, const GemmOperand &A, const GemmOperand 
   // k, and keep that order (gemm_ordered.cu says what for) wherever a derivative that
   // jumps may follow and it is cheap: a tile of 64 x 64 per SM at most, since a second
   // round doubles its time (333 rows of 1203 x 1203 47 us against 21, 449 rows 90 against
-  // 22), and three times the shortest way at most (64 rows, 47 against 15).  The line is
+  // 22), and three times the shortest way at most (64 rows, 47 against 15); an output
+  // narrower than its tile is the small kernel's.  The line is
   // one of cost: on its far side, as at the widths TMA can address, which never had that
   // order, a unit near the jump falls where the rounding of the sums puts it.
   // Where no such derivative follows, the shortest way is taken unless it is less accurate:
