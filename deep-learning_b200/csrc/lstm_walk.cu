@@ -518,7 +518,7 @@ constexpr size_t W_SMEM_MAX = 226 * 1024;  // beside the barriers
 // sums, about 20 for 10, so those take more rows or a longer k but fewer examples.  Either
 // number is divided between rows and chunks in the ways that some layer measured fastest
 // with: 79 layers of 8 - 300 blocks of 1 - 3 cells at 8, 64 and 200 examples, every plan
-// of both directions.  (4 x 5, 5 x 4, 1 x 10, 10 x 1 and 20 x 1 never won by more than 2 %.)
+// of both directions.  (4 x 5, 5 x 4, 1 x 10, 10 x 1 and 20 x 1 never won by more than 4 %.)
 struct WarpRows {
   int rows, chunks;
 };
@@ -548,8 +548,8 @@ int walk_clusters(const dlb_ctx *ctx, int cs) {
 }
 
 // The fastest layout by the cost of a step in cycles, fitted to the plans of the layers
-// above within 2 x of their fastest (the plan it picks takes 1.8 % longer than the fastest
-// on average, 32 % at worst): cells and exchange; a chain of loads and multiply-adds per
+// above near their fastest (the plan it picks takes 1.5 % longer than the fastest on
+// average, 43 % at worst, 14 % next to it): cells and exchange; a chain of loads and multiply-adds per
 // example and 128 k, times the rounds of rows per warp; the sums over lanes; the
 // weights read from shared memory; and what the dense forms lose to spills.  Times the
 // rounds that the examples need of the CTAs that run at once.  None if the weights do
